@@ -1,7 +1,7 @@
 // capi.cu -- status handling and the generic C entry points of libvsmc_cuda:
 // RNG word streams, the device WeightSet update, the device resampler and
 // the particle gather.  The CV filter's entry points are in cv_filter.cu.
-#include "resample.cuh"
+#include "resample_cluster.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -437,8 +437,8 @@ int vsmc_cuda_resample(int scheme, uint64_t N, const double *weight,
     }
     WeightsGiven w;
     w.w = weight;
-    launch_resample_core(scheme, w, (long long)N, eng, ws, uniforms,
-                         (long long)n_uniforms, false, replication, cf, s);
+    launch_resample(scheme, w, (long long)N, eng, ws, uniforms,
+                    (long long)n_uniforms, false, replication, cf, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample: launch");
@@ -523,9 +523,9 @@ int vsmc_cuda_resample_mn(int scheme, uint64_t M, uint64_t N,
     }
     WeightsGiven w;
     w.w = weight;
-    launch_resample_core(scheme, w, (long long)M, eng, ws, uniforms,
-                         (long long)n_uniforms, false, rep, cf_scratch, s,
-                         false, /*cfrp=*/false, (long long)N);
+    launch_resample(scheme, w, (long long)M, eng, ws, uniforms,
+                    (long long)n_uniforms, false, rep, cf_scratch, s,
+                    /*cfrp=*/false, (long long)N);
     if (copy_from != nullptr)
         launch_expand(rep, (long long)M, (long long)N, ws, copy_from, s);
     e = cudaGetLastError();

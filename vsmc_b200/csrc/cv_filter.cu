@@ -14,6 +14,7 @@
 // kernels of resample.cuh, which return at once when the step does not
 // resample.  No host round trip happens inside a step.
 #include "cv_kernels.cuh"
+#include "resample_cluster.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -217,12 +218,12 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
         if (compare) {
             // the step's own resampling of its own weights, into the
             // record row; the engine advances by the words it drew
-            launch_resample_core(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
-                                 /*spine_done=*/true, nullptr,
-                                 f->rec_cf + (size_t)f->iter * c.N, s);
-            f->launches += resample_launches(c.scheme, false,
-                                           WeightsFromLog<Real>::kExactNorm,
-                                           WeightsFromLog<Real>::kApprox);
+            launch_resample(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
+                            /*spine_done=*/true, nullptr,
+                            f->rec_cf + (size_t)f->iter * c.N, s);
+            f->launches += resample_launch_count(
+                N, c.scheme, WeightsFromLog<Real>::kExactNorm,
+                WeightsFromLog<Real>::kApprox);
         }
         // replay: the recorded ancestry of this step (used only if the
         // recorded decision was to resample)
@@ -236,17 +237,17 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
         f->launches -= 5; // the sequence's launches are counted on the side
         enqueue_sequence(f); // for the next resampling
     } else {
-        launch_resample_core(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
-                             /*spine_done=*/true, nullptr, f->copy_from, s);
+        launch_resample(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
+                        /*spine_done=*/true, nullptr, f->copy_from, s);
     }
     if (f->rec_cf != nullptr && !compare)
         cudaMemcpyAsync(f->rec_cf + (size_t)f->iter * c.N, f->copy_from,
                         c.N * 4, cudaMemcpyDeviceToDevice, s);
     if (ev)
         cudaEventRecord(ev[2], s);
-    f->launches += 2 + resample_launches(c.scheme, false,
-                                           WeightsFromLog<Real>::kExactNorm,
-                                           WeightsFromLog<Real>::kApprox);
+    f->launches += 2 + resample_launch_count(
+                           N, c.scheme, WeightsFromLog<Real>::kExactNorm,
+                           WeightsFromLog<Real>::kApprox);
     ++f->iter;
 }
 
@@ -419,7 +420,9 @@ int vsmc_cuda_cv_create(const vsmc_cuda_cv_config *cfg, void *stream,
     // persistent grid striding over tiles (measured 5% faster at 2^24)
     f->move_grid = (int)f->ntiles;
     e = cudaMemsetAsync(f->mem, 0, f->bytes, f->stream);
-    if (e == cudaSuccess && cfg->scheme == VSMC_CUDA_MULTINOMIAL) {
+    // (a filter that resamples in one cluster draws its sequence there)
+    if (e == cudaSuccess && cfg->scheme == VSMC_CUDA_MULTINOMIAL &&
+        !rc_fits((long long)N, 0)) {
         // the lowest priority: the sequence fills SMs the step's own
         // kernels leave idle (the one-CTA finalize and spines) instead of
         // competing with the move

@@ -156,9 +156,19 @@ struct SmemExactThread {
     int elast[kThreads];
 };
 
+// A thread's own part of the classification: e and special as in
+// ExactThread, kloc[j] the clean k of its elements through j, nsp its
+// specials.
+struct ExactLocal {
+    unsigned long long kloc[kItems];
+    int e[kItems];
+    unsigned special;
+    int nsp;
+};
+
 __device__ __forceinline__ void
-exact_thread(long long i0, long long N, const double (&w)[kItems], double a,
-             double pre, double rel, ExactThread &x, SmemExactThread &sm)
+exact_classify(long long i0, long long N, const double (&w)[kItems], double a,
+               double pre, double rel, ExactLocal &x)
 {
     // one error bound for the thread's elements
     double p = pre, wmax = 0.0;
@@ -181,7 +191,7 @@ exact_thread(long long i0, long long N, const double (&w)[kItems], double a,
     double gp = __dadd_rn(a, pre);
     unsigned long long kr = 0;
     int nsp = 0;
-    unsigned long long kloc[kItems];
+    unsigned long long (&kloc)[kItems] = x.kloc;
     x.special = 0;
     // the common case: the windows of the thread's first and last prefix
     // lie in one binade, so every window between them does and each of
@@ -257,6 +267,22 @@ exact_thread(long long i0, long long N, const double (&w)[kItems], double a,
             ep = ec;
         }
     }
+    x.nsp = nsp;
+}
+
+__device__ __forceinline__ void
+exact_thread(long long i0, long long N, const double (&w)[kItems], double a,
+             double pre, double rel, ExactThread &x, SmemExactThread &sm)
+{
+    ExactLocal l;
+    exact_classify(i0, N, w, a, pre, rel, l);
+#pragma unroll
+    for (int j = 0; j < kItems; ++j)
+        x.e[j] = l.e[j];
+    x.special = l.special;
+    const unsigned long long kr = l.kloc[kItems - 1];
+    const unsigned long long (&kloc)[kItems] = l.kloc;
+    const int nsp = l.nsp;
     int nspec;
     x.rank0 = block_excl_scan(nsp, sm.shi, nspec);
     x.nspec = nspec;

@@ -32,6 +32,7 @@
 // special-function units, one log2 per pair of points) and accumulates the
 // log terms of a particle in double.  Everything else is double in both.
 #include "cv_kernels.cuh"
+#include "resample_cluster.cuh"
 
 #include <cmath>
 #include <cstring>
@@ -1234,8 +1235,8 @@ int vsmc_cuda_gmm_iterate(vsmc_cuda_gmm *g, uint64_t num)
         WeightsFromLog<double> w;
         w.lw = g->lw;
         w.stats = &g->ctl->lw_max;
-        launch_resample_core(scheme, w, N, g->eng, g->rws, nullptr, 0,
-                             /*spine_done=*/true, nullptr, g->copy_from, s);
+        launch_resample(scheme, w, N, g->eng, g->rws, nullptr, 0,
+                        /*spine_done=*/true, nullptr, g->copy_from, s);
         cudaEvent_t *ev = nullptr;
         if (g->timing) {
             if (g->ev_used + 2 > g->ev.size())
@@ -1261,7 +1262,7 @@ int vsmc_cuda_gmm_iterate(vsmc_cuda_gmm *g, uint64_t num)
             g->buf[1 - g->cur].base + 13 * N, g->lw, g->ctl, N, (long long)t,
             a, g->gctl, g->hist_accept, g->hist_integrand, g->hist_grid);
         g->cur = 1 - g->cur;
-        g->launches += 4 + resample_launches(scheme, false, true);
+        g->launches += 4 + resample_launch_count(N, scheme, true, false);
         ++g->iter;
     }
     cudaError_t e = cudaGetLastError();

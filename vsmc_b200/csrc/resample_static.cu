@@ -17,7 +17,7 @@
 // so nothing stale is used, but two calls that overlap on the GPU (for
 // example on two streams) race on the same memory and must be serialised by
 // the caller.
-#include "resample.cuh"
+#include "resample_cluster.cuh"
 
 #include <cstring>
 #include <mutex>
@@ -159,8 +159,8 @@ extern "C" int vsmc_cuda_resample_noalloc(int scheme, uint64_t N,
     }
     WeightsGiven w;
     w.w = weight;
-    launch_resample_core(scheme, w, (long long)N, eng, ws, uniforms,
-                         (long long)n_uniforms, false, replication, cf, s);
+    launch_resample(scheme, w, (long long)N, eng, ws, uniforms,
+                    (long long)n_uniforms, false, replication, cf, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_noalloc: launch");

@@ -14,6 +14,7 @@
 // copy_from when the previous step resampled; vsmc_cuda_smc_finish_step then
 // runs the same finalize and resampling kernels as the built-in filter.
 #include "cv_kernels.cuh"
+#include "resample_cluster.cuh"
 
 #include <cstring>
 #include <new>
@@ -273,10 +274,9 @@ int vsmc_cuda_smc_finish_step(vsmc_cuda_smc *s)
     WeightsFromLog<double> w;
     w.lw = s->lw;
     w.stats = &s->ctl->lw_max;
-    launch_resample_core(sch, w, N, s->eng, s->rws, nullptr, 0,
-                         /*spine_done=*/true, nullptr, s->copy_from,
-                         s->stream);
-    s->launches += 1 + resample_launches(sch, false, true);
+    launch_resample(sch, w, N, s->eng, s->rws, nullptr, 0,
+                    /*spine_done=*/true, nullptr, s->copy_from, s->stream);
+    s->launches += 1 + resample_launch_count(N, sch, true, false);
     ++s->iter;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VSMC_CUDA_OK
