@@ -156,25 +156,27 @@ struct SmemExactThread {
     int elast[kThreads];
 };
 
-// A thread's own part of the classification: e and special as in
-// ExactThread, kloc[j] the clean k of its elements through j, nsp its
-// specials.
+// A thread's own part of the classification of its R elements: e and
+// special as in ExactThread, kloc[j] the clean k of its elements through j,
+// nsp its specials.
+template <int R>
 struct ExactLocal {
-    unsigned long long kloc[kItems];
-    int e[kItems];
+    unsigned long long kloc[R];
+    int e[R];
     unsigned special;
     int nsp;
 };
 
+template <int R>
 __device__ __forceinline__ void
-exact_classify(long long i0, long long N, const double (&w)[kItems], double a,
-               double pre, double rel, ExactLocal &x)
+exact_classify(long long i0, long long N, const double (&w)[R], double a,
+               double pre, double rel, ExactLocal<R> &x)
 {
     // one error bound for the thread's elements
     double p = pre, wmax = 0.0;
     bool bad = false;
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
+    for (int j = 0; j < R; ++j) {
         p += w[j];
         wmax = fmax(wmax, w[j]);
         bad |= !(w[j] >= 0.0);
@@ -184,26 +186,26 @@ exact_classify(long long i0, long long N, const double (&w)[kItems], double a,
     double d = 0.0;
     if (ok) {
         const double ulp2 = exact_pow2(exact_binade(m) + 1 - 52);
-        const double il = (double)(i0 + kItems - 1);
+        const double il = (double)(i0 + R - 1);
         d = __dadd_rn(__dmul_rn(__dadd_rn(8.0 * il, 256.0), ulp2),
                       __dmul_rn(rel, m));
     }
     double gp = __dadd_rn(a, pre);
     unsigned long long kr = 0;
     int nsp = 0;
-    unsigned long long (&kloc)[kItems] = x.kloc;
+    unsigned long long (&kloc)[R] = x.kloc;
     x.special = 0;
     // the common case: the windows of the thread's first and last prefix
     // lie in one binade, so every window between them does and each of
     // the thread's elements is clean (unless a tie)
     bool fast = false;
-    if (ok && i0 > 0 && i0 + kItems <= N) {
+    if (ok && i0 > 0 && i0 + R <= N) {
         const int e0 = exact_window(gp, d);
         if (e0 != kNoBinade && e0 == exact_window(__dadd_rn(a, p), d)) {
             const double sc = exact_pow2(52 - e0);
             bool slow = false;
 #pragma unroll
-            for (int j = 0; j < kItems; ++j) {
+            for (int j = 0; j < R; ++j) {
                 const double kf = __dmul_rn(w[j], sc);
                 const double t = __dadd_rn(kf, 0x1p52);
                 slow |= !(kf < 0x1p52) ||
@@ -222,7 +224,7 @@ exact_classify(long long i0, long long N, const double (&w)[kItems], double a,
     if (!fast) {
         kr = 0;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             const long long i = i0 + j;
             p += w[j];
             const double g = __dadd_rn(a, p);
@@ -274,7 +276,7 @@ __device__ __forceinline__ void
 exact_thread(long long i0, long long N, const double (&w)[kItems], double a,
              double pre, double rel, ExactThread &x, SmemExactThread &sm)
 {
-    ExactLocal l;
+    ExactLocal<kItems> l;
     exact_classify(i0, N, w, a, pre, rel, l);
 #pragma unroll
     for (int j = 0; j < kItems; ++j)

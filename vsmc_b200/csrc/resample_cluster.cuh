@@ -4,7 +4,7 @@
 // few tiles each of them holds one or a few CTAs' work and costs 4 to 15 us
 // of latency: kernel boundary, control block, global-memory round trips
 // between producer and consumer.  Here one thread-block cluster runs the
-// whole resampling: each group of kThreads threads owns one tile and keeps
+// whole resampling: each group of kTile / R threads owns one tile and keeps
 // its weights, records and counts in registers; what tiles exchange (tile
 // sums, exact-scan records and specials, zero counts, surplus prefixes)
 // goes through distributed shared memory between cluster barriers; every
@@ -16,11 +16,10 @@
 // The results are those of the launch sequence: the exact scans reproduce
 // the reference's sequential sums bit for bit whatever the split, and the
 // mixed form's plain scan and residual sums keep the same association
-// (the same block scans over the same 256 threads).
+// (the same block scans over the same 256 runs of 8 particles).
 //
-// Bound: latency (barriers, dependent shared-memory and L2 reads).
-// Measured on one B200, us a step of a filter, launch sequence -> cluster:
-// see launch_resample below.
+// Bound: latency (FP64 chains, barriers, dependent shared-memory and L2
+// reads); see rc_shape for the split and its measurements.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -40,11 +39,18 @@ constexpr int kRcStage = 256;   // specials of a scan staged per CTA
 // How a resampling draws its U01 sequence.
 enum { kRcSorted = 0, kRcStrat = 1, kRcSys = 2 };
 
-// Barrier of one group (named barriers 1, 2; 0 is __syncthreads).
-__device__ __forceinline__ void rc_gsync(int grp)
-{
-    asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(kThreads) : "memory");
-}
+// A group: the threads of one tile, R consecutive particles each, with a
+// named barrier of its own (barriers 1, 2; 0 is __syncthreads).
+template <int R>
+struct RcThread {
+    static constexpr int TT = kTile / R; // threads of the group
+    static constexpr int NW = TT / 32;   // its warps
+    int grp, tid, lane, wid;
+    __device__ __forceinline__ void sync() const
+    {
+        asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TT) : "memory");
+    }
+};
 
 struct RcScan {
     ExactTile tile;
@@ -65,27 +71,34 @@ struct alignas(16) RcGroup {
     int zeros, sinc_last;
     alignas(16) int32_t sinc[kTile]; // surplus counts (sinc_local)
     // the group's own
-    double sv_w[kExactCap], sv_u[kExactCap]; // exact S at the specials
-    double red_d[kThreads / 32];
-    unsigned long long red_k[kThreads / 32], red_s[kThreads / 32];
-    int red_n[kThreads / 32], red_e[kThreads / 32];
+    double sv_w[kExactCap], sv_u[kExactCap]; // (rc_walk_slow) exact S at
+                                             // the tile's specials
+    double red_d[32];
+    unsigned long long red_k[32], red_s[32];
+    int red_n[32], red_e[32];
     long long bound[2];
-    alignas(16) double buf[kUStage]; // uniforms; overflow tiles' S; ranks
+    // engine words, overflow tiles' S, uniforms, rank table in turn
+    alignas(16) double buf[kUStage];
 };
 
-// The gathered records of one exact scan and its walk.
+// The gathered records of one exact scan and its walk: the additions in
+// order, first the clean run `seg` before a special (or the end of the
+// tile), then the special's weight (0 at the end of a tile).
+struct RcStep {
+    double seg, w;
+};
 struct RcWalk {
     ExactTile t[kRcMaxTiles];
-    int off[kRcMaxTiles + 1];
-    double start[kRcMaxTiles + 1];
-    ExactSpecial st[kRcStage];
-    int overflow;
+    int off[kRcMaxTiles + 1]; // specials before tile t
+    RcStep step[kRcStage + kRcMaxTiles + 8];
+    double S[kRcStage + kRcMaxTiles + 8]; // after each step
+    double start[kRcMaxTiles + 1];        // before each tile
+    int slow; // overflow tiles, or more specials than staged
 };
 
 struct RcShared {
     RcWalk w, u;
     double sums[kRcMaxTiles], usums[kRcMaxTiles];
-    double sh[kThreads / 32];
     double total; // the residuals' approximate sum
     long long NN;
     long long kexcl[kRcMaxTiles + 1];
@@ -116,171 +129,215 @@ struct RcArgs {
     int32_t *copy_from;
 };
 
-// Exclusive scan over a group: block_excl_scan's association.
-__device__ __forceinline__ double rc_excl_scan(double v, double *sh, int gtid,
-                                               int grp, double &total)
+// Exclusive scan over a group (any association: FP64 sums here feed only
+// the exact scan's classification, or are integers).
+template <typename T, int R>
+__device__ __forceinline__ T rc_excl_scan(T v, T *sh, const RcThread<R> &th,
+                                          T &total)
 {
-    constexpr int NW = kThreads / 32;
-    const int lane = gtid & 31, wid = gtid >> 5;
-    const double inc = warp_incl_scan(v);
-    if (lane == 31)
-        sh[wid] = inc;
-    rc_gsync(grp);
-    if (wid == 0) {
-        double s = lane < NW ? sh[lane] : 0.0;
-        s = warp_incl_scan(s);
-        if (lane < NW)
-            sh[lane] = s;
-    }
-    rc_gsync(grp);
-    const double wexcl = wid > 0 ? sh[wid - 1] : 0.0;
-    total = sh[NW - 1];
-    rc_gsync(grp);
-    return wexcl + inc - v;
+    constexpr int NW = RcThread<R>::NW;
+    const T inc = warp_incl_scan(v);
+    if (th.lane == 31)
+        sh[th.wid] = inc;
+    th.sync();
+    const T x = th.lane < NW ? sh[th.lane] : T(0);
+    const T xi = warp_incl_scan(x);
+    total = __shfl_sync(0xffffffffu, xi, 31);
+    const T before = __shfl_sync(0xffffffffu, xi - x, th.wid);
+    th.sync();
+    return before + inc - v;
 }
 
-// ... of integers (any association).
-template <typename T>
-__device__ __forceinline__ T rc_excl_scan_int(T v, T *sh, int gtid, int grp,
-                                              T &total)
+// The plain scan's prefixes of a tile in the launch sequence's association:
+// each run of kItems values in order, block_excl_scan over the 256 runs,
+// then each run's prefixes in order from its offset.  rec: inclusive.
+template <int R>
+__device__ __forceinline__ void rc_plain_scan(const double (&w)[R],
+                                              const RcThread<R> &th,
+                                              RcGroup &g, double (&rec)[R],
+                                              double &total)
 {
-    constexpr int NW = kThreads / 32;
-    const int lane = gtid & 31, wid = gtid >> 5;
-    const T inc = warp_incl_scan(v);
-    if (lane == 31)
-        sh[wid] = inc;
-    rc_gsync(grp);
-    T before = 0, all = 0;
+    constexpr int Q = kItems / R; // threads of a run
+    const int q = th.tid % Q;
+    double run = 0.0;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-        const T x = sh[w];
-        before += w < wid ? x : T(0);
-        all += x;
+    for (int k = 0; k < Q; ++k) {
+        const double in = __shfl_up_sync(0xffffffffu, run, 1);
+        if (q == k) {
+            if (k > 0)
+                run = in;
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                run += w[j];
+        }
     }
-    total = all;
-    rc_gsync(grp);
-    return before + inc - v;
+    double *vr = g.buf; // the runs' sums, then their offsets
+    if (q == Q - 1)
+        vr[th.tid / Q] = run;
+    th.sync();
+    double inc = 0.0, v = 0.0;
+    if (th.tid < kThreads) {
+        v = vr[th.tid];
+        inc = warp_incl_scan(v);
+        if (th.lane == 31)
+            g.red_d[th.wid] = inc;
+    }
+    th.sync();
+    if (th.wid == 0) {
+        double s = th.lane < kThreads / 32 ? g.red_d[th.lane] : 0.0;
+        s = warp_incl_scan(s);
+        if (th.lane < kThreads / 32)
+            g.red_d[th.lane] = s;
+    }
+    th.sync();
+    if (th.tid < kThreads) {
+        const double wexcl = th.wid > 0 ? g.red_d[th.wid - 1] : 0.0;
+        vr[th.tid] = wexcl + inc - v;
+    }
+    total = g.red_d[kThreads / 32 - 1];
+    th.sync();
+    double s = vr[th.tid / Q];
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+        const double in = __shfl_up_sync(0xffffffffu, s, 1);
+        if (q == k) {
+            if (k > 0)
+                s = in;
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                s += w[j];
+                rec[j] = s;
+            }
+        }
+    }
+    th.sync(); // vr and red_d are free again
 }
 
 // A thread's share of an exact scan: its element records (exact_scan.cuh)
 // and the specials of the tile before them.
+template <int R>
 struct RcRec {
-    double rec[kItems];
+    double rec[R];
     int rank0;
 };
 
 // Classification of the group's tile (weights w, approximate start a and
 // exclusive prefix pre): the tile's record and specials into `out`, the
-// thread's records into r.  One segmented scan gives the clean k, the
-// number of specials and the clean k since the last special before the
-// thread's elements.
+// thread's records into r.  The clean k is scanned over the group; the last
+// special before a thread is found by ballots, so the usual warp without
+// specials pays nothing for them.
+template <int R>
 __device__ __forceinline__ void
-rc_classify(long long base, long long N, const double (&w)[kItems], double a,
-            double pre, double rel, int gtid, int grp, RcGroup &g,
-            RcScan &out, double *dump, RcRec &r)
+rc_classify(long long base, long long N, const double (&w)[R], double a,
+            double pre, double rel, const RcThread<R> &th, RcGroup &g,
+            RcScan &out, double *dump, RcRec<R> &r)
 {
-    constexpr int NW = kThreads / 32;
-    const int lane = gtid & 31, wid = gtid >> 5;
-    const long long i0 = base + (long long)gtid * kItems;
-    ExactLocal x;
+    constexpr int NW = RcThread<R>::NW;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = th.lane;
+    const long long i0 = base + (long long)th.tid * R;
+    ExactLocal<R> x;
     exact_classify(i0, N, w, a, pre, rel, x);
-    const unsigned long long kr = x.kloc[kItems - 1];
+    const unsigned long long kr = x.kloc[R - 1];
     unsigned long long kat = 0; // kloc at the thread's last special
 #pragma unroll
-    for (int j = 0; j < kItems; ++j)
+    for (int j = 0; j < R; ++j)
         if ((x.special >> j) & 1u)
             kat = x.kloc[j];
-    unsigned long long k = kr, s = x.nsp ? kr - kat : kr;
-    int n = x.nsp;
-    const int elast =
-        (x.special >> (kItems - 1)) & 1u ? kNoBinade : x.e[kItems - 1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long pk = __shfl_up_sync(0xffffffffu, k, o);
-        const unsigned long long ps = __shfl_up_sync(0xffffffffu, s, o);
-        const int pn = __shfl_up_sync(0xffffffffu, n, o);
-        if (lane >= o) {
-            k += pk;
-            s = n ? s : ps + s;
-            n += pn;
+    const unsigned long long ki = warp_incl_scan(kr);
+    const unsigned long long ke = ki - kr;
+    const int elast = (x.special >> (R - 1)) & 1u ? kNoBinade : x.e[R - 1];
+    int e_before = __shfl_up_sync(kAll, elast, 1);
+    // specials of the warp: their count before the thread and the warp's
+    // clean k at the last of them
+    const unsigned any = __ballot_sync(kAll, x.nsp != 0);
+    int ne = 0;
+    bool has = false;
+    unsigned long long kb = 0;
+    if (any != 0) {
+        const int ni = warp_incl_scan(x.nsp);
+        const unsigned before = any & ((1u << lane) - 1u);
+        const int src = 31 - __clz(before | 1u);
+        const unsigned long long q = __shfl_sync(kAll, ke + kat, src);
+        has = before != 0;
+        kb = has ? q : 0ull;
+        ne = ni - x.nsp;
+        if (lane == 31) {
+            g.red_n[th.wid] = ni;
+            g.red_s[th.wid] = x.nsp ? ke + kat : q;
         }
+    } else if (lane == 31) {
+        g.red_n[th.wid] = 0;
     }
     if (lane == 31) {
-        g.red_k[wid] = k;
-        g.red_s[wid] = s;
-        g.red_n[wid] = n;
-        g.red_e[wid] = elast;
+        g.red_k[th.wid] = ki;
+        g.red_e[th.wid] = elast;
     }
-    // exclusive within the warp
-    unsigned long long ke = __shfl_up_sync(0xffffffffu, k, 1);
-    unsigned long long se = __shfl_up_sync(0xffffffffu, s, 1);
-    int ne = __shfl_up_sync(0xffffffffu, n, 1);
-    int e_before = __shfl_up_sync(0xffffffffu, elast, 1);
-    if (lane == 0) {
-        ke = se = 0;
-        ne = 0;
-    }
-    rc_gsync(grp);
-    unsigned long long kp = 0, sp = 0, ktile = 0;
-    int np = 0, nspec = 0;
-#pragma unroll
-    for (int q = 0; q < NW; ++q) {
-        const unsigned long long qk = g.red_k[q];
-        const int qn = g.red_n[q];
-        if (q < wid) {
-            kp += qk;
-            sp = qn ? g.red_s[q] : sp + g.red_s[q];
-            np += qn;
-        }
-        ktile += qk;
-        nspec += qn;
+    th.sync();
+    const unsigned long long wk = lane < NW ? g.red_k[lane] : 0ull;
+    const int wn = lane < NW ? g.red_n[lane] : 0;
+    const unsigned long long wki = warp_incl_scan(wk);
+    const unsigned long long ktile = __shfl_sync(kAll, wki, 31);
+    const unsigned long long kp = __shfl_sync(kAll, wki - wk, th.wid);
+    const unsigned wany = __ballot_sync(kAll, wn != 0);
+    int nspec = 0, np = 0;
+    unsigned long long kbw = 0; // the tile's clean k at the last special
+                                // of the earlier warps
+    if (wany != 0) {
+        const int wni = warp_incl_scan(wn);
+        nspec = __shfl_sync(kAll, wni, 31);
+        np = __shfl_sync(kAll, wni - wn, th.wid);
+        const unsigned before = wany & ((1u << th.wid) - 1u);
+        const unsigned long long at =
+            wki - wk + (wn != 0 ? g.red_s[lane] : 0ull);
+        const unsigned long long q =
+            __shfl_sync(kAll, at, 31 - __clz(before | 1u));
+        kbw = before != 0 ? q : 0ull;
     }
     if (lane == 0)
-        e_before = wid > 0 ? g.red_e[wid - 1] : kNoBinade;
-    ke += kp;
-    se = ne ? se : sp + se;
+        e_before = th.wid > 0 ? g.red_e[th.wid - 1] : kNoBinade;
+    const unsigned long long k0 = kp + ke; // clean k before the thread
+    unsigned long long kl = has ? kp + kb : kbw; // ... at the last special
     r.rank0 = np + ne;
     const long long last = min(base + (long long)kTile, N) - 1;
     int rank = r.rank0;
-    unsigned long long kb = 0; // kloc at the last special, se before it
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
+    for (int j = 0; j < R; ++j) {
         if ((x.special >> j) & 1u) {
             if (rank < kExactCap) {
                 ExactSpecial q;
                 q.w = w[j];
-                q.k_before = ke + x.kloc[j];
+                q.k_before = k0 + x.kloc[j];
                 q.idx = (int)(i0 + j - base);
                 q.e_seg = j == 0 ? e_before
-                                 : ((x.special >> (j - 1)) & 1u
+                                 : ((x.special >> (j > 0 ? j - 1 : 0)) & 1u
                                         ? kNoBinade
-                                        : x.e[j - 1]);
+                                        : x.e[j > 0 ? j - 1 : 0]);
                 out.spec[rank] = q;
             }
             ++rank;
-            se = 0;
-            kb = x.kloc[j];
+            kl = k0 + x.kloc[j];
             r.rec[j] = -1.0;
         } else {
-            const unsigned long long K = se + (x.kloc[j] - kb);
+            const unsigned long long K = k0 + x.kloc[j] - kl;
             r.rec[j] = K == 0 ? 0.0
                               : __dmul_rn((double)K, exact_pow2(x.e[j] - 52));
         }
         if (i0 + j == last)
             out.tile.e_last = (x.special >> j) & 1u ? kNoBinade : x.e[j];
     }
-    if (gtid == 0) {
+    if (th.tid == 0) {
         out.tile.k_total = ktile;
         out.tile.nspec = nspec;
     }
     // a tile with more specials than kept: its values for the walk
     if (nspec > kExactCap) {
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             if (i0 + j < N)
                 dump[i0 + j] = w[j];
     }
-    rc_gsync(grp); // the red_* arrays are free again
+    th.sync(); // the red_* arrays are free again
 }
 
 // The records of every tile's scan into the CTA's shared memory (after the
@@ -308,41 +365,73 @@ __device__ __forceinline__ void rc_gather_tiles(cg::cluster_group &cl,
         if (lane == 31)
             k.off[32] = in;
         const unsigned ov = __ballot_sync(0xffffffffu, et.nspec > kExactCap);
-        if (lane == 0)
-            k.overflow = ov != 0;
+        if (lane == 31)
+            k.slow = ov != 0 || in > kRcStage;
     }
 }
 
+__device__ __forceinline__ double rc_clean(unsigned long long K, int e)
+{
+    return K == 0 ? 0.0 : __dmul_rn((double)K, exact_pow2(e - 52));
+}
+
+// The walk's additions: a warp per tile.
 template <int B>
 __device__ __forceinline__ void rc_gather_specials(cg::cluster_group &cl,
                                                    RcShared &sm, RcWalk &k,
-                                                   int nt, int G)
+                                                   int nt, int G, int w0)
 {
-    if (k.off[32] > kRcStage)
+    if (k.slow)
         return;
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int t = threadIdx.x >> 5; t < nt; t += nw) {
+    const int wq = (threadIdx.x >> 5) - w0;
+    for (int t = wq < 0 ? wq + nw : wq; t < nt; t += nw) {
         const int b = k.off[t], n = k.off[t + 1] - b;
-        if (n == 0)
-            continue;
+        const ExactTile et = k.t[t];
         const RcGroup *rg = cl.map_shared_rank(&sm.g[t % G], t / G);
         const ExactSpecial *sp = rg->scan[B].spec;
-        for (int r = lane; r < n; r += 32)
-            k.st[b + r] = sp[r];
+        for (int r = lane; r <= n; r += 32) {
+            const unsigned long long kb = r > 0 ? sp[r - 1].k_before : 0ull;
+            RcStep st;
+            if (r < n) {
+                st.seg = rc_clean(sp[r].k_before - kb, sp[r].e_seg);
+                st.w = sp[r].w;
+            } else {
+                st.seg = rc_clean(et.k_total - kb, et.e_last);
+                st.w = 0.0;
+            }
+            k.step[b + t + r] = st;
+        }
     }
 }
 
-// Phase B of the exact scan (one thread): the exact S before every tile
-// and, for the CTA's own tiles [own, own + G), at their specials.
-// Overflow tiles are summed element by element from `vals`; their S goes
-// into the group's buffer.
+// Phase B of the exact scan (one thread): the additions in order.
+__device__ __forceinline__ void rc_walk(RcWalk &k, int nt)
+{
+    const int n = k.off[nt] + nt;
+    double S = 0.0;
+    for (int i = 0; i < n; i += 4) { // (reads past n stay in the array)
+        RcStep q[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            q[m] = k.step[i + m];
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            if (i + m < n) {
+                S = __dadd_rn(__dadd_rn(S, q[m].seg), q[m].w);
+                k.S[i + m] = S;
+            }
+    }
+}
+
+// ... with overflow tiles, summed element by element from `vals` (their S
+// goes into the group's buffer), or more specials than staged.
 template <int B>
-__device__ __forceinline__ void rc_walk(cg::cluster_group &cl, RcShared &sm,
-                                        RcWalk &k, int nt, int G, int own,
-                                        const double *vals, long long N)
+__device__ __noinline__ void rc_walk_slow(cg::cluster_group cl, RcShared &sm,
+                                          RcWalk &k, int nt, int G, int own,
+                                          const double *vals, long long N)
 {
     constexpr bool U = B == kRcU;
-    const bool fits = k.off[32] <= kRcStage;
     double S = 0.0;
     for (int t = 0; t < nt; ++t) {
         k.start[t] = S;
@@ -350,20 +439,11 @@ __device__ __forceinline__ void rc_walk(cg::cluster_group &cl, RcShared &sm,
         const int mine = t - own;
         const bool keep = mine >= 0 && mine < G;
         if (et.nspec <= kExactCap) {
+            const RcGroup *rg = cl.map_shared_rank(&sm.g[t % G], t / G);
             unsigned long long kb = 0;
             for (int r = 0; r < et.nspec; ++r) {
-                ExactSpecial sp;
-                if (fits) {
-                    sp = k.st[k.off[t] + r];
-                } else {
-                    const RcGroup *rg =
-                        cl.map_shared_rank(&sm.g[t % G], t / G);
-                    sp = rg->scan[B].spec[r];
-                }
-                const unsigned long long seg = sp.k_before - kb;
-                if (seg != 0)
-                    S = __dadd_rn(S, __dmul_rn((double)seg,
-                                               exact_pow2(sp.e_seg - 52)));
+                const ExactSpecial sp = rg->scan[B].spec[r];
+                S = __dadd_rn(S, rc_clean(sp.k_before - kb, sp.e_seg));
                 S = __dadd_rn(S, sp.w);
                 if (keep) {
                     if (U)
@@ -373,10 +453,7 @@ __device__ __forceinline__ void rc_walk(cg::cluster_group &cl, RcShared &sm,
                 }
                 kb = sp.k_before;
             }
-            const unsigned long long tail = et.k_total - kb;
-            if (tail != 0)
-                S = __dadd_rn(S, __dmul_rn((double)tail,
-                                           exact_pow2(et.e_last - 52)));
+            S = __dadd_rn(S, rc_clean(et.k_total - kb, et.e_last));
         } else {
             const long long b0 = (long long)t * kTile;
             const int n = (int)(min(b0 + (long long)kTile, N) - b0);
@@ -391,22 +468,64 @@ __device__ __forceinline__ void rc_walk(cg::cluster_group &cl, RcShared &sm,
     k.start[nt] = S;
 }
 
+// The exact S before tile t (t <= the tiles walked).
+__device__ __forceinline__ double rc_start(const RcWalk &k, int t)
+{
+    if (k.slow)
+        return k.start[t];
+    return t == 0 ? 0.0 : k.S[k.off[t] + t - 1];
+}
+
 // The exact S of a thread's elements after the walk.
-template <bool U>
-__device__ __forceinline__ void rc_values(const RcShared &sm, const RcWalk &k,
-                                          const RcGroup &g, int tile,
-                                          int gtid, const RcRec &r,
-                                          double (&S)[kItems])
+template <bool U, int R>
+__device__ __forceinline__ void rc_values(const RcWalk &k, const RcGroup &g,
+                                          int tile, const RcThread<R> &th,
+                                          const RcRec<R> &r, double (&S)[R])
 {
     if (k.t[tile].nspec > kExactCap) {
-        const double *o = g.buf + (U ? kTile : 0) + gtid * kItems;
+        const double *o = g.buf + (U ? kTile : 0) + th.tid * R;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             S[j] = o[j];
         return;
     }
-    exact_values(r.rec, r.rank0, k.start[tile], U ? g.sv_u : g.sv_w, false,
-                 S);
+    const double *sv =
+        k.slow ? (U ? g.sv_u : g.sv_w) : &k.S[k.off[tile] + tile];
+    const double start = rc_start(k, tile);
+    int q = r.rank0 - 1; // rank of the last special before element j
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        if (r.rec[j] < 0.0) {
+            ++q;
+            S[j] = sv[min(q, kExactCap - 1)];
+        } else {
+            S[j] = __dadd_rn(q < 0 ? start : sv[min(q, kExactCap - 1)],
+                             r.rec[j]);
+        }
+    }
+}
+
+// Engine words [first, first + count) of the group's tile into its buffer
+// (count <= kTile + 2): a Threefry block per thread, shared by the threads
+// whose words it holds.  Returns the first word's place; barriers inside.
+template <int R>
+__device__ __forceinline__ const uint64_t *
+rc_words(const EngineRef &eng, unsigned long long first, int count,
+         const RcThread<R> &th, RcGroup &g)
+{
+    uint64_t *q = reinterpret_cast<uint64_t *>(g.buf);
+    const unsigned long long b0 = first / 4;
+    const int s = (int)(first % 4), nb = (s + count + 3) / 4;
+    th.sync(); // (earlier reads of the buffer)
+    for (int b = th.tid; b < nb; b += RcThread<R>::TT) {
+        const u64x4 x =
+            threefry4x64_20(ctr64_add(eng.ctr, b0 + b + 1), eng.key);
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            q[4 * b + l] = x.v[l];
+    }
+    th.sync();
+    return q + s;
 }
 
 // Sum of the tile sums before tile t (for the classification).
@@ -418,18 +537,18 @@ __device__ __forceinline__ double rc_before(const double *sums, int t)
     return a;
 }
 
-// Eight consecutive values of a thread (zero past N).
-template <typename T>
-__device__ __forceinline__ void rc_load8(const T *src, long long i0,
-                                         long long N, T (&v)[kItems])
+// R consecutive values of a thread (zero past N).
+template <typename T, int R>
+__device__ __forceinline__ void rc_load(const T *src, long long i0,
+                                        long long N, T (&v)[R])
 {
-    if (i0 + kItems <= N &&
-        (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-        constexpr int P = 16 / sizeof(T);
+    constexpr int B = R * (int)sizeof(T) < 16 ? R * (int)sizeof(T) : 16;
+    typedef typename std::conditional<B == 16, int4, int2>::type V;
+    if (i0 + R <= N && (reinterpret_cast<uintptr_t>(src) & (B - 1)) == 0) {
+        constexpr int P = B / sizeof(T);
 #pragma unroll
-        for (int j = 0; j < kItems / P; ++j) {
-            const int4 q =
-                *reinterpret_cast<const int4 *>(src + i0 + j * P);
+        for (int j = 0; j < R / P; ++j) {
+            const V q = *reinterpret_cast<const V *>(src + i0 + j * P);
             const T *t = reinterpret_cast<const T *>(&q);
 #pragma unroll
             for (int m = 0; m < P; ++m)
@@ -437,43 +556,63 @@ __device__ __forceinline__ void rc_load8(const T *src, long long i0,
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             v[j] = i0 + j < N ? src[i0 + j] : T(0);
     }
 }
 
-// Eight consecutive ints to a caller's array of any alignment.
-__device__ __forceinline__ void rc_store8(int32_t *dst, long long i0,
-                                          long long N,
-                                          const int (&v)[kItems])
+// R consecutive ints to and from shared memory (R a multiple of 2).
+template <int R>
+__device__ __forceinline__ void rc_put(int *dst, const int (&v)[R])
 {
-    if (i0 + kItems <= N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        int4 *d = reinterpret_cast<int4 *>(dst + i0);
-        d[0] = make_int4(v[0], v[1], v[2], v[3]);
-        d[1] = make_int4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+    for (int j = 0; j < R; j += 2)
+        *reinterpret_cast<int2 *>(dst + j) = make_int2(v[j], v[j + 1]);
+}
+template <int R>
+__device__ __forceinline__ void rc_get(const int *src, int (&v)[R])
+{
+#pragma unroll
+    for (int j = 0; j < R; j += 2) {
+        const int2 q = *reinterpret_cast<const int2 *>(src + j);
+        v[j] = q.x;
+        v[j + 1] = q.y;
+    }
+}
+
+// R consecutive ints to a caller's array of any alignment.
+template <int R>
+__device__ __forceinline__ void rc_store(int32_t *dst, long long i0,
+                                         long long N, const int (&v)[R])
+{
+    if (i0 + R <= N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+        rc_put<R>(dst + i0, v);
     } else {
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             if (i0 + j < N)
                 dst[i0 + j] = v[j];
     }
 }
 
 // One resampling; every thread of the cluster calls it.
-template <typename W, bool Residual, int U>
+template <typename W, bool Residual, int U, int R>
 __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                                             RcShared &sm)
 {
     constexpr bool Sys = U == kRcSys;
-    constexpr int NW = kThreads / 32;
+    constexpr int TT = RcThread<R>::TT;
     if (!a.ctl->active)
         return; // (the whole cluster)
     cg::cluster_group cl = cg::this_cluster();
-    const int G = (int)blockDim.x / kThreads;
+    const int G = (int)blockDim.x / TT;
     const int rank = (int)cl.block_rank();
-    const int grp = (int)threadIdx.x / kThreads;
-    const int gtid = (int)threadIdx.x % kThreads;
-    const int lane = gtid & 31, wid = gtid >> 5;
+    RcThread<R> th;
+    th.grp = (int)threadIdx.x / TT;
+    th.tid = (int)threadIdx.x % TT;
+    th.lane = th.tid & 31;
+    th.wid = th.tid >> 5;
+    const int grp = th.grp, gtid = th.tid, lane = th.lane, wid = th.wid;
     const int own = rank * G;
     const int tile = own + grp;
     const int nt = a.nt;
@@ -481,7 +620,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     RcGroup &g = sm.g[grp];
     const bool act = tile < nt;
     const long long base = (long long)tile * kTile;
-    const long long i0 = base + (long long)gtid * kItems;
+    const long long i0 = base + (long long)gtid * R;
     const long long Nout = resample_children(a.ctl, N);
     const double Nd = (double)Nout;
     wsrc.prepare();
@@ -508,20 +647,20 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     __syncthreads();
 
     // ---- the weights --------------------------------------------------
-    double w[kItems]; // as scanned
-    int kk[kItems];   // floor(N w) (residual)
-    RcRec rw;
+    double w[R]; // as scanned
+    int kk[R];   // floor(N w) (residual)
+    RcRec<R> rw;
     double pre = 0.0, coeff_r = 1.0;
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
+    for (int j = 0; j < R; ++j) {
         w[j] = 0.0;
         kk[j] = 0;
     }
     if (act) {
-        typename W::stage_t x[kItems];
-        rc_load8(wsrc.stage_src(), i0, N, x);
+        typename W::stage_t x[R];
+        rc_load(wsrc.stage_src(), i0, N, x);
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             if (i0 + j < N)
                 w[j] = W::kExactNorm ? wsrc.unnorm_stage(x[j])
                                      : wsrc.from_stage(x[j]);
@@ -531,38 +670,44 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         if (act) {
             double run = 0.0, total;
 #pragma unroll
-            for (int j = 0; j < kItems; ++j)
+            for (int j = 0; j < R; ++j)
                 run += w[j];
-            pre = rc_excl_scan(run, g.red_d, gtid, grp, total);
+            pre = rc_excl_scan(run, g.red_d, th, total);
             rc_classify(base, N, w,
                         __dmul_rn(a.tile_excl[tile], wsrc.spine_unnorm()),
-                        pre, ExactMargin<W>::rel, gtid, grp, g, g.scan[kRcA], a.rec,
+                        pre, ExactMargin<W>::rel, th, g, g.scan[kRcA], a.rec,
                         rw);
         }
     }
     // the drawn sequence's first stage, beside the weights' (its length is
     // known unless the scheme is residual)
-    double tv[kItems]; // negated terms
-    RcRec ru;
+    double tv[R]; // negated terms
+    RcRec<R> ru;
     double pre_u = 0.0;
     const auto terms = [&]() {
         // log(1 - U_n) / (NN - n), negated, and the tile's sum
         const long long NN = sm.NN;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             tv[j] = 0.0;
         if (base < NN) {
-            if (i0 < NN) {
-                sorted_terms8(a.eng, sm.offset, i0, NN, tv);
+            const uint64_t *q = rc_words(
+                a.eng, sm.offset + (unsigned long long)base,
+                (int)min((long long)kTile, NN - base), th, g);
 #pragma unroll
-                for (int j = 0; j < kItems; ++j)
-                    tv[j] = -tv[j];
+            for (int j = 0; j < R; ++j) {
+                const long long n = i0 + j;
+                if (n < NN) {
+                    const double U1 = canonical_u64(q[gtid * R + j]);
+                    tv[j] = -__ddiv_rn(fm::fm_log(__dadd_rn(1.0, -U1)),
+                                       (double)(NN - n));
+                }
             }
             double run = 0.0, total;
 #pragma unroll
-            for (int j = 0; j < kItems; ++j)
+            for (int j = 0; j < R; ++j)
                 run += tv[j];
-            pre_u = rc_excl_scan(run, g.red_d, gtid, grp, total);
+            pre_u = rc_excl_scan(run, g.red_d, th, total);
             if (gtid == 0)
                 g.sum_u = total;
         }
@@ -574,12 +719,12 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         // (the terms' tile sums are in sm.usums)
         if (base < sm.NN)
             rc_classify(base, sm.NN, tv, rc_before(sm.usums, tile), pre_u,
-                        ExactMargin<TermsNeg>::rel, gtid, grp, g,
+                        ExactMargin<TermsNeg>::rel, th, g,
                         g.scan[kRcU], a.u,
                         ru);
     };
     const auto gather_usums = [&](int nu) {
-        if ((int)(threadIdx.x >> 5) == NW - 1 && lane < nu)
+        if ((int)(threadIdx.x >> 5) == 7 && lane < nu)
             sm.usums[lane] =
                 cl.map_shared_rank(&sm.g[lane % G], lane / G)->sum_u;
     };
@@ -588,15 +733,15 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         const long long NN = sm.NN;
         if (base >= NN)
             return;
-        double S[kItems];
-        rc_values<true>(sm, sm.u, g, tile, gtid, ru, S);
-        const double s0 = sm.u.start[tile];
+        double S[R];
+        rc_values<true>(sm.u, g, tile, th, ru, S);
+        const double s0 = rc_start(sm.u, tile);
         const double umax =
             tile > 0 ? __dadd_rn(1.0, -fm::fm_exp(-s0)) : -INFINITY;
-        double uv[kItems];
+        double uv[R];
         double tmax = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             uv[j] = __dadd_rn(1.0, -fm::fm_exp(-S[j]));
             tmax = fmax(tmax, uv[j]);
         }
@@ -612,15 +757,15 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         double exc = __shfl_up_sync(0xffffffffu, inc, 1);
         if (lane == 0)
             exc = -INFINITY;
-        rc_gsync(grp);
-        for (int q = 0; q < wid; ++q)
-            exc = fmax(exc, g.red_d[q]);
-        rc_gsync(grp);
+        th.sync();
+        const double wm = warp_max(lane < wid ? g.red_d[lane] : -INFINITY);
+        th.sync();
+        exc = fmax(exc, wm);
         double m = fmax(umax, exc);
         const int kb = sm.kbits;
         long long kprev = bin_floor(m, kb);
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             m = fmax(m, uv[j]);
             const long long n = i0 + j;
             if (n < NN) {
@@ -639,44 +784,25 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         const double delta = sm.delta;
         const int kb = sm.kbits;
         const unsigned long long off = sm.offset;
-        double raw[kItems];
+        // (two words more in front: a thread's first value needs the two
+        // before it)
+        const int lead = base > 0 ? 2 : 0;
+        const uint64_t *q = rc_words(
+            a.eng, off + (unsigned long long)(base - lead),
+            (int)min((long long)kTile, NN - base) + lead, th, g);
+        const auto at = [&](long long n) {
+            return n >= 0 && n < NN ? strat_u(q[n - base + lead], n, delta)
+                                    : -INFINITY;
+        };
+        double raw[R];
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
-            raw[j] = -INFINITY;
-        if (i0 < NN) {
-            uint64_t q[8];
-            threefry_words8(a.eng, off + (unsigned long long)i0, q);
-#pragma unroll
-            for (int j = 0; j < kItems; ++j)
-                if (i0 + j < NN)
-                    raw[j] = strat_u(q[j], i0 + j, delta);
-        }
-        double p1 = __shfl_up_sync(0xffffffffu, raw[7], 1);
-        double p2 = __shfl_up_sync(0xffffffffu, raw[6], 1);
-        if (lane == 31) {
-            g.red_d[wid] = raw[7];
-            g.sv_u[wid] = raw[6];
-        }
-        rc_gsync(grp);
-        if (lane == 0) {
-            p1 = p2 = -INFINITY;
-            if (wid > 0) {
-                p1 = g.red_d[wid - 1];
-                p2 = g.sv_u[wid - 1];
-            } else if (base > 0) {
-                p1 = strat_u(threefry_word(a.eng.key, a.eng.ctr,
-                                           off + i0 - 1),
-                             i0 - 1, delta);
-                p2 = strat_u(threefry_word(a.eng.key, a.eng.ctr,
-                                           off + i0 - 2),
-                             i0 - 2, delta);
-            }
-        }
-        rc_gsync(grp);
+        for (int j = 0; j < R; ++j)
+            raw[j] = at(i0 + j);
+        const double p1 = at(i0 - 1), p2 = at(i0 - 2);
         long long kprev = bin_floor(fmax(p1, p2), kb);
         double rprev = p1;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             const long long n = i0 + j;
             if (n < NN) {
                 const double v = fmax(raw[j], rprev);
@@ -687,6 +813,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             }
             rprev = raw[j];
         }
+        th.sync(); // the words' buffer is free again
     };
     // the walks of the weights' and / or the terms' scans (after a cluster
     // barrier); a walk over an overflow tile reads its values in global
@@ -701,17 +828,25 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             rc_gather_tiles<kRcU>(cl, sm, sm.u, nu, G, 1);
         __syncthreads();
         if (ww)
-            rc_gather_specials<B>(cl, sm, sm.w, nt, G);
+            rc_gather_specials<B>(cl, sm, sm.w, nt, G, 0);
         if (wu)
-            rc_gather_specials<kRcU>(cl, sm, sm.u, nu, G);
+            rc_gather_specials<kRcU>(cl, sm, sm.u, nu, G,
+                                     nt % (int)(blockDim.x >> 5));
         __syncthreads();
-        if (ww && threadIdx.x == 0)
-            rc_walk<B>(cl, sm, sm.w, nt, G, own, a.rec, N);
-        if (wu && threadIdx.x == 32)
-            rc_walk<kRcU>(cl, sm, sm.u, nu, G, own, a.u, sm.NN);
+        if (ww && threadIdx.x == 0) {
+            if (sm.w.slow)
+                rc_walk_slow<B>(cl, sm, sm.w, nt, G, own, a.rec, N);
+            else
+                rc_walk(sm.w, nt);
+        }
+        if (wu && threadIdx.x == 32) {
+            if (sm.u.slow)
+                rc_walk_slow<kRcU>(cl, sm, sm.u, nu, G, own, a.u, sm.NN);
+            else
+                rc_walk(sm.u, nu);
+        }
         __syncthreads();
-        if ((ww && (sm.w.overflow || sm.w.off[32] > kRcStage)) ||
-            (wu && (sm.u.overflow || sm.u.off[32] > kRcStage)))
+        if ((ww && sm.w.slow) || (wu && sm.u.slow))
             cl.sync();
     };
 
@@ -727,19 +862,19 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             gather_usums(utiles());
         walks(std::integral_constant<int, kRcA>(), true, false);
         // w = exp(lw - M) * (1 / sum)
-        const double coeff = __ddiv_rn(1.0, sm.w.start[nt]);
+        const double coeff = __ddiv_rn(1.0, rc_start(sm.w, nt));
         pre *= coeff;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             w[j] = __dmul_rn(w[j], coeff);
     }
     bool exact = true;
     if (Residual) {
         // r = modf(N w, &k); the tile's sums
-        double r[kItems];
+        double r[R];
         long long ks = 0;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             double k = 0.0;
             r[j] = i0 + j < N ? residual_split(w[j], Nd, k) : 0.0;
             kk[j] = (int32_t)k;
@@ -748,46 +883,47 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         if (act) {
             double run = 0.0, total;
 #pragma unroll
-            for (int j = 0; j < kItems; ++j)
+            for (int j = 0; j < R; ++j)
                 run += fabs(r[j]);
             if (W::kApprox) {
-                // the launch sequence's sum: strided elements per thread,
-                // warp trees, the warps in order
-                double s = 0.0;
+                // the launch sequence's sum: eight strided elements per
+                // thread of 256, warp trees, the warps in order
 #pragma unroll
-                for (int j = 0; j < kItems; ++j)
-                    g.buf[pad8(gtid * kItems + j)] = fabs(r[j]);
-                rc_gsync(grp);
+                for (int j = 0; j < R; ++j)
+                    g.buf[pad8(gtid * R + j)] = fabs(r[j]);
+                th.sync();
+                if (gtid < kThreads) {
+                    double s = 0.0;
 #pragma unroll
-                for (int j = 0; j < kItems; ++j) {
-                    const int l = j * kThreads + gtid;
-                    if (base + l < N)
-                        s += g.buf[pad8(l)];
+                    for (int j = 0; j < kItems; ++j) {
+                        const int l = j * kThreads + gtid;
+                        if (base + l < N)
+                            s += g.buf[pad8(l)];
+                    }
+                    s = warp_sum(s);
+                    if (lane == 0)
+                        g.red_d[wid] = s;
                 }
-                s = warp_sum(s);
-                if (lane == 0)
-                    g.red_d[wid] = s;
-                rc_gsync(grp);
+                th.sync();
                 if (gtid == 0) {
                     double t = 0.0;
-                    for (int q = 0; q < NW; ++q)
+                    for (int q = 0; q < kThreads / 32; ++q)
                         t += g.red_d[q];
                     g.sum_w = t;
                 }
-                rc_gsync(grp);
+                th.sync();
             } else {
-                pre = rc_excl_scan(run, g.red_d, gtid, grp, total);
+                pre = rc_excl_scan(run, g.red_d, th, total);
                 if (gtid == 0)
                     g.sum_w = total;
             }
             long long kt;
-            rc_excl_scan_int(ks, reinterpret_cast<long long *>(g.red_k), gtid,
-                             grp, kt);
+            rc_excl_scan(ks, reinterpret_cast<long long *>(g.red_k), th, kt);
             if (gtid == 0)
                 g.ksum = kt;
         }
 #pragma unroll
-        for (int j = 0; j < kItems; ++j)
+        for (int j = 0; j < R; ++j)
             w[j] = r[j];
         cl.sync();
         // NN = children - sum floor(N w); the residuals' approximate sum
@@ -834,28 +970,27 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             // the residuals' sequential sum
             const double a0 = act ? rc_before(sm.sums, tile) : 0.0;
             if (act)
-                rc_classify(base, N, w, a0, pre, ExactMargin<W>::rel, gtid,
-                            grp, g, g.scan[kRcB], a.rec, rw);
+                rc_classify(base, N, w, a0, pre, ExactMargin<W>::rel, th, g, g.scan[kRcB], a.rec, rw);
             cl.sync();
             if (U == kRcSorted) {
                 gather_usums(utiles());
                 __syncthreads();
             }
             walks(std::integral_constant<int, kRcB>(), true, false);
-            coeff_r = __ddiv_rn(1.0, sm.w.start[nt]);
+            coeff_r = __ddiv_rn(1.0, rc_start(sm.w, nt));
             if (act) {
                 pre *= coeff_r;
 #pragma unroll
-                for (int j = 0; j < kItems; ++j)
+                for (int j = 0; j < R; ++j)
                     w[j] = __dmul_rn(w[j], coeff_r);
                 rc_classify(base, N, w, a0 * coeff_r, pre,
-                            ExactMargin<W>::rel, gtid, grp, g, g.scan[kRcA], a.rec,
+                            ExactMargin<W>::rel, th, g, g.scan[kRcA], a.rec,
                             rw);
             }
         } else if (W::kApprox) {
             coeff_r = __ddiv_rn(1.0, sm.total);
 #pragma unroll
-            for (int j = 0; j < kItems; ++j)
+            for (int j = 0; j < R; ++j)
                 w[j] = __dmul_rn(w[j], coeff_r);
         }
     } else if (W::kExactNorm) {
@@ -863,17 +998,17 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             rc_classify(base, N, w,
                         __dmul_rn(a.tile_excl[tile],
                                   __ddiv_rn(wsrc.spine_unnorm(),
-                                            sm.w.start[nt])),
-                        pre, ExactMargin<W>::rel, gtid, grp, g, g.scan[kRcB], a.rec,
+                                            rc_start(sm.w, nt))),
+                        pre, ExactMargin<W>::rel, th, g, g.scan[kRcB], a.rec,
                         rw);
     } else if (!W::kApprox) {
         // given weights: tile sums first
         if (act) {
             double run = 0.0, total;
 #pragma unroll
-            for (int j = 0; j < kItems; ++j)
+            for (int j = 0; j < R; ++j)
                 run += w[j];
-            pre = rc_excl_scan(run, g.red_d, gtid, grp, total);
+            pre = rc_excl_scan(run, g.red_d, th, total);
             if (gtid == 0)
                 g.sum_w = total;
         }
@@ -886,21 +1021,13 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         __syncthreads();
         if (act)
             rc_classify(base, N, w, rc_before(sm.sums, tile), pre,
-                        ExactMargin<W>::rel, gtid, grp, g, g.scan[kRcA], a.rec, rw);
+                        ExactMargin<W>::rel, th, g, g.scan[kRcA], a.rec, rw);
     }
     if (W::kApprox && exact && act) {
         // the plain scan: inclusive prefixes within the tile, the tile's
         // total in fixed point
-        double run = 0.0, total;
-#pragma unroll
-        for (int j = 0; j < kItems; ++j)
-            run += w[j];
-        double s = rc_excl_scan(run, g.red_d, gtid, grp, total);
-#pragma unroll
-        for (int j = 0; j < kItems; ++j) {
-            s += w[j];
-            rw.rec[j] = s;
-        }
+        double total;
+        rc_plain_scan(w, th, g, rw.rec, total);
         if (gtid == 0)
             g.fixed = approx_fixed(total);
     }
@@ -914,9 +1041,9 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     cl.sync();
 
     // ---- the cumulative weights ------------------------------------------
-    double Cx[kItems];
+    double Cx[R];
 #pragma unroll
-    for (int j = 0; j < kItems; ++j)
+    for (int j = 0; j < R; ++j)
         Cx[j] = 0.0;
     if (exact) {
         // the weights' scan: kRcB after the normalisation's, else kRcA
@@ -939,11 +1066,11 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             if (act) {
                 const double s0 = sm.w.start[tile];
 #pragma unroll
-                for (int j = 0; j < kItems; ++j)
+                for (int j = 0; j < R; ++j)
                     Cx[j] = __dadd_rn(s0, rw.rec[j]);
             }
         } else if (act) {
-            rc_values<false>(sm, sm.w, g, tile, gtid, rw, Cx);
+            rc_values<false>(sm.w, g, tile, th, rw, Cx);
         }
         if (U == kRcSorted) {
             sorted_values();
@@ -957,11 +1084,14 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     const long long nu = NN;
     const double *u = a.u;
     double *sw = g.buf;
-    int rep[kItems];
-    int zl[kItems]; // rank among the tile's slots without offspring, or -1
+    int rep[R];
+    int zl[R]; // rank among the tile's slots without offspring, or -1
     if (act) {
-        const double sa = exact ? sm.w.start[tile] : 0.0;
-        const double sb = exact ? sm.w.start[tile + 1] : 0.0;
+        const auto start = [&](int t) {
+            return W::kApprox ? sm.w.start[t] : rc_start(sm.w, t);
+        };
+        const double sa = exact ? start(tile) : 0.0;
+        const double sb = exact ? start(tile + 1) : 0.0;
         if (wid < 2) {
             const double C = wid == 0 ? sa : sb;
             long long r;
@@ -980,25 +1110,25 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             if (lane == 0)
                 g.bound[wid] = r;
         }
-        rc_gsync(grp);
+        th.sync();
         const long long lo = g.bound[0];
         const long long hi = max(g.bound[1], lo);
         const bool staged = !Sys && (hi - lo) <= kUStage;
         if (staged) {
-            for (int k = gtid; k < (int)(hi - lo); k += kThreads)
+            for (int k = gtid; k < (int)(hi - lo); k += TT)
                 cp_async8(&sw[k], &u[lo + k]);
             cp_async_commit();
             cp_async_wait_all();
         }
-        rc_gsync(grp);
+        th.sync();
         const int ilo = (int)lo, ihi = (int)hi, iNN = (int)NN, iN = (int)N;
         const int p0 = (int)i0;
         const int tile_last = (int)min(base + (long long)kTile, N) - 1;
-        int cnt[kItems];
+        int cnt[R];
         int pos = -1;
         long long gpos = -1;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             const int i = p0 + j;
             const double C = Cx[j];
             int c;
@@ -1020,17 +1150,17 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             cnt[j] = min(max(c, ilo), i >= iN - 1 ? iNN : ihi);
         }
 #pragma unroll
-        for (int j = 1; j < kItems; ++j)
+        for (int j = 1; j < R; ++j)
             cnt[j] = max(cnt[j], cnt[j - 1]);
-        int prev = __shfl_up_sync(0xffffffffu, cnt[kItems - 1], 1);
+        int prev = __shfl_up_sync(0xffffffffu, cnt[R - 1], 1);
         if (lane == 31)
-            g.red_e[wid] = cnt[kItems - 1];
-        rc_gsync(grp);
+            g.red_e[wid] = cnt[R - 1];
+        th.sync();
         if (lane == 0)
             prev = wid == 0 ? (tile > 0 ? ilo : 0) : g.red_e[wid - 1];
         int zeros = 0, ksum = 0;
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             const int i = p0 + j;
             const int c = max(cnt[j], prev);
             rep[j] = (i < iN) ? (c - prev) + kk[j] : 0;
@@ -1046,33 +1176,32 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                 a.ctl->n_final = c;
         }
         int ztot, ktot;
-        int zloc = rc_excl_scan_int(zeros, g.red_n, gtid, grp, ztot);
+        int zloc = rc_excl_scan(zeros, g.red_n, th, ztot);
         int kprefix = 0;
         if (Residual)
             kprefix = (int)sm.kexcl[tile] +
-                      rc_excl_scan_int(ksum, g.red_n, gtid, grp, ktot);
+                      rc_excl_scan(ksum, g.red_n, th, ktot);
         if (gtid == 0)
             g.zeros = ztot;
-        int sc[kItems];
+        int sc[R];
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+        for (int j = 0; j < R; ++j) {
             const int i = p0 + j;
             kprefix += kk[j];
-            const int R = (i >= iN - 1) ? (int)Nout : cnt[j] + kprefix;
+            const int upto =
+                (i >= iN - 1) ? (int)Nout : cnt[j] + kprefix;
             zl[j] = -1;
             if (rep[j] == 0) {
                 zl[j] = zloc;
                 ++zloc;
             }
-            sc[j] = R - (i + 1) + zloc;
+            sc[j] = upto - (i + 1) + zloc;
             if (i == tile_last)
                 g.sinc_last = sc[j];
         }
-        int4 *sd = reinterpret_cast<int4 *>(g.sinc + gtid * kItems);
-        sd[0] = make_int4(sc[0], sc[1], sc[2], sc[3]);
-        sd[1] = make_int4(sc[4], sc[5], sc[6], sc[7]);
+        rc_put<R>(g.sinc + gtid * R, sc);
         if (a.rep_out != nullptr)
-            rc_store8(a.rep_out, i0, N, rep);
+            rc_store(a.rep_out, i0, N, rep);
     }
     cl.sync();
     if (rank == 0 && threadIdx.x == 0)
@@ -1108,11 +1237,12 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                 __ballot_sync(0xffffffffu, e > Z0 + z - 1);
             const int tf = min(__ffs(above0) - 1, nt - 1);
             const int tl = min(__ffs(above1) - 1, nt - 1);
-            const int4 none = make_int4(-1, -1, -1, -1);
-            int4 *t4 = reinterpret_cast<int4 *>(tab + gtid * kItems);
-            t4[0] = none;
-            t4[1] = none;
-            rc_gsync(grp);
+            int m[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                m[j] = -1;
+            rc_put<R>(tab + gtid * R, m);
+            th.sync();
             // parent p owns the ranks [sinc(p - 1), sinc(p)): it marks the
             // first of them that falls in the window
             int prev_top = INT_MIN;
@@ -1121,16 +1251,13 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                 const int len = (int)min((long long)kTile, N - pb);
                 const int zoff = sm.zexcl[pt];
                 const RcGroup *rg = cl.map_shared_rank(&sm.g[pt % G], pt / G);
-                const int4 *s4 =
-                    reinterpret_cast<const int4 *>(rg->sinc + gtid * kItems);
-                const int4 q0 = s4[0], q1 = s4[1];
-                const int v[kItems] = {q0.x, q0.y, q0.z, q0.w,
-                                       q1.x, q1.y, q1.z, q1.w};
-                int before = gtid > 0 ? rg->sinc[gtid * kItems - 1] + zoff
-                                      : prev_top;
+                int v[R];
+                rc_get<R>(rg->sinc + gtid * R, v);
+                int before =
+                    gtid > 0 ? rg->sinc[gtid * R - 1] + zoff : prev_top;
 #pragma unroll
-                for (int j = 0; j < kItems; ++j) {
-                    const int l = gtid * kItems + j;
+                for (int j = 0; j < R; ++j) {
+                    const int l = gtid * R + j;
                     if (l < len) {
                         const int cur = v[j] + zoff;
                         const int rl = max(before, Z0);
@@ -1142,15 +1269,14 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                 prev_top = max(prev_top, rg->sinc[len - 1] + zoff);
             }
             top = prev_top - Z0;
-            rc_gsync(grp);
+            th.sync();
             // parents increase with the rank: the running maximum of the
             // marks is each rank's parent
-            const int4 m0 = t4[0], m1 = t4[1];
-            int m[kItems] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            rc_get<R>(tab + gtid * R, m);
 #pragma unroll
-            for (int j = 1; j < kItems; ++j)
+            for (int j = 1; j < R; ++j)
                 m[j] = max(m[j], m[j - 1]);
-            int in = m[kItems - 1];
+            int in = m[R - 1];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int q = __shfl_up_sync(0xffffffffu, in, o);
@@ -1162,18 +1288,18 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             int ex = __shfl_up_sync(0xffffffffu, in, 1);
             if (lane == 0)
                 ex = -1;
-            rc_gsync(grp);
-            for (int q = 0; q < wid; ++q)
-                ex = max(ex, g.red_n[q]);
-            t4[0] = make_int4(max(m[0], ex), max(m[1], ex), max(m[2], ex),
-                              max(m[3], ex));
-            t4[1] = make_int4(max(m[4], ex), max(m[5], ex), max(m[6], ex),
-                              max(m[7], ex));
-            rc_gsync(grp);
-        }
-        int cf[kItems];
+            th.sync();
+            ex = max(ex, __reduce_max_sync(0xffffffffu,
+                                           lane < wid ? g.red_n[lane] : -1));
 #pragma unroll
-        for (int j = 0; j < kItems; ++j) {
+            for (int j = 0; j < R; ++j)
+                m[j] = max(m[j], ex);
+            rc_put<R>(tab + gtid * R, m);
+            th.sync();
+        }
+        int cf[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
             cf[j] = (int)i0 + j;
             if (i0 + j < N && zl[j] >= 0) {
                 const int p = zl[j] < min(z, top) ? tab[zl[j]] : -1;
@@ -1183,29 +1309,31 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                     atomicExch(&a.ctl->error, (int)VSMC_CUDA_EDEGENERATE);
             }
         }
-        rc_store8(a.copy_from, i0, N, cf);
+        rc_store(a.copy_from, i0, N, cf);
     }
     cl.sync(); // no CTA leaves while another reads its shared memory
 }
 
-template <typename W, bool Residual, int U>
-__global__ void __launch_bounds__(kThreads *kRcGroups, 1)
+template <typename W, bool Residual, int U, int R>
+__global__ void __launch_bounds__(R == 8 ? 512 : kTile / R, 1)
 k_resample_cluster(W wsrc, RcArgs a)
 {
     extern __shared__ __align__(16) unsigned char rc_smem[];
-    rc_resample<W, Residual, U>(wsrc, a,
-                                *reinterpret_cast<RcShared *>(rc_smem));
+    rc_resample<W, Residual, U, R>(wsrc, a,
+                                   *reinterpret_cast<RcShared *>(rc_smem));
 }
 
-// CTAs and groups for nt tiles: a tile a CTA up to 16 tiles, then two.
+// The cluster of nt tiles: up to 16 a CTA of 1024 threads each (two
+// particles a thread), above two tiles a CTA of 512 threads (eight).
 struct RcShape {
-    int ctas, groups;
+    int ctas, groups, r;
 };
 
 inline RcShape rc_shape(int nt)
 {
     RcShape s;
     s.groups = nt > kRcMaxCtas ? kRcGroups : 1;
+    s.r = nt > kRcMaxCtas ? 8 : 2;
     s.ctas = 1;
     while (s.ctas * s.groups < nt)
         s.ctas *= 2;
@@ -1227,7 +1355,7 @@ inline cudaError_t rc_launch(K k, RcShape shape, int clusters,
         return e;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((unsigned)(shape.ctas * clusters));
-    c.blockDim = dim3((unsigned)(kThreads * shape.groups));
+    c.blockDim = dim3((unsigned)(kTile / shape.r * shape.groups));
     c.dynamicSmemBytes = smem;
     c.stream = s;
     cudaLaunchAttribute at[1];
@@ -1246,6 +1374,16 @@ inline bool rc_fits(long long N, long long Nout)
 {
     const long long n = Nout > N ? Nout : N;
     return resample_ntiles(n) <= kRcMaxTiles;
+}
+
+template <typename W, bool Residual, int U>
+inline void rc_launch_shape(const RcShape &sh, const W &w, const RcArgs &a,
+                            cudaStream_t s)
+{
+    if (sh.r == 8)
+        rc_launch(k_resample_cluster<W, Residual, U, 8>, sh, 1, s, w, a);
+    else
+        rc_launch(k_resample_cluster<W, Residual, U, 2>, sh, 1, s, w, a);
 }
 
 // A resampling: one cluster where it fits, the launch sequence of
@@ -1281,22 +1419,22 @@ inline void launch_resample(int scheme, W wsrc, long long N,
     const RcShape sh = rc_shape(resample_ntiles(Nout > N ? Nout : N));
     switch (scheme) {
     case VSMC_CUDA_MULTINOMIAL:
-        rc_launch(k_resample_cluster<W, false, kRcSorted>, sh, 1, s, wsrc, a);
+        rc_launch_shape<W, false, kRcSorted>(sh, wsrc, a, s);
         break;
     case VSMC_CUDA_RESIDUAL:
-        rc_launch(k_resample_cluster<W, true, kRcSorted>, sh, 1, s, wsrc, a);
+        rc_launch_shape<W, true, kRcSorted>(sh, wsrc, a, s);
         break;
     case VSMC_CUDA_STRATIFIED:
-        rc_launch(k_resample_cluster<W, false, kRcStrat>, sh, 1, s, wsrc, a);
+        rc_launch_shape<W, false, kRcStrat>(sh, wsrc, a, s);
         break;
     case VSMC_CUDA_SYSTEMATIC:
-        rc_launch(k_resample_cluster<W, false, kRcSys>, sh, 1, s, wsrc, a);
+        rc_launch_shape<W, false, kRcSys>(sh, wsrc, a, s);
         break;
     case VSMC_CUDA_RESIDUAL_STRATIFIED:
-        rc_launch(k_resample_cluster<W, true, kRcStrat>, sh, 1, s, wsrc, a);
+        rc_launch_shape<W, true, kRcStrat>(sh, wsrc, a, s);
         break;
     default:
-        rc_launch(k_resample_cluster<W, true, kRcSys>, sh, 1, s, wsrc, a);
+        rc_launch_shape<W, true, kRcSys>(sh, wsrc, a, s);
         break;
     }
 }
