@@ -253,6 +253,18 @@ struct LazyBound<float> {
     static constexpr double v = 40.0;
 };
 
+// One particle's exponential e and position into the sums: explicit fused
+// multiply-adds, so that every kernel that folds the same particles in the
+// same order rounds alike.
+__device__ __forceinline__ void lse_sum(LseRef &a, double e, double x,
+                                        double y)
+{
+    a.s1 = __dadd_rn(a.s1, e);
+    a.s2 = __fma_rn(e, e, a.s2);
+    a.sx = __fma_rn(e, x, a.sx);
+    a.sy = __fma_rn(e, y, a.sy);
+}
+
 template <typename Real>
 __device__ __forceinline__ void lse_add(LseRef &a, Real lw, Real x, Real y)
 {
@@ -275,10 +287,7 @@ __device__ __forceinline__ void lse_add(LseRef &a, Real lw, Real x, Real y)
         a.ref = l;
     }
     const double e = lse_exp((Real)(lw - (Real)a.ref));
-    a.s1 += e;
-    a.s2 += e * e;
-    a.sx += e * (double)x;
-    a.sy += e * (double)y;
+    lse_sum(a, e, (double)x, (double)y);
 }
 
 // Rescale a thread's sums to the common maximum M: exp(ref - M) <= 1.
@@ -314,22 +323,18 @@ __device__ __forceinline__ void warp_sum_stats(LseRef &a, double &gx,
 }
 
 
-// The tile's statistics from every thread's accumulator (acc, plus the sums
-// gx, gy of gathered positions, 0 where unused): per warp a common maximum,
-// one rescale per lane and plain sums in a fixed shuffle tree; then warp 0
-// joins the NW warps in the same way and writes *out.  `sh_w` holds
-// 7 x NW doubles; one barrier (callers that run several tiles alternate two
-// such buffers).  Every thread of the CTA calls it.
+// One warp's share of a tile's statistics (a common maximum, one rescale per
+// lane, plain sums in a fixed shuffle tree) into column `wid` of sh_w, which
+// holds 7 x NW doubles.
 template <int NW>
-__device__ __forceinline__ void tile_stats_reduce(LseRef acc, double gx,
-                                                  double gy, double *sh_w,
-                                                  TileStats *out)
+__device__ __forceinline__ void tile_stats_warp(LseRef acc, double gx,
+                                                double gy, double *sh_w,
+                                                int wid)
 {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double wm = warp_max_nan(acc.mx, 32);
     lse_rescale(acc, wm);
     warp_sum_stats(acc, gx, gy, 32);
-    if (lane == 0) {
+    if ((threadIdx.x & 31) == 0) {
         double *w = sh_w;
         w[0 * NW + wid] = wm;
         w[1 * NW + wid] = acc.s1;
@@ -339,38 +344,58 @@ __device__ __forceinline__ void tile_stats_reduce(LseRef acc, double gx,
         w[5 * NW + wid] = gx;
         w[6 * NW + wid] = gy;
     }
-    __syncthreads();
-    if (wid == 0) {
-        const double *w = sh_w;
-        LseRef r;
-        double tx = 0.0, ty = 0.0;
-        r.init();
-        if (lane < NW) {
-            r.ref = w[0 * NW + lane];
-            r.mx = r.ref;
-            r.s1 = w[1 * NW + lane];
-            r.s2 = w[2 * NW + lane];
-            r.sx = w[3 * NW + lane];
-            r.sy = w[4 * NW + lane];
-            tx = w[5 * NW + lane];
-            ty = w[6 * NW + lane];
-        }
-        const double tm = warp_max_nan(r.mx, NW);
-        lse_rescale(r, tm);
-        warp_sum_stats(r, tx, ty, NW);
-        if (lane == 0) {
-            TileStats ts;
-            ts.m = tm;
-            ts.s1 = r.s1;
-            ts.s2 = r.s2;
-            ts.sx = r.sx;
-            ts.sy = r.sy;
-            ts.gx = tx;
-            ts.gy = ty;
-            ts.pad = 0.0;
-            *out = ts;
-        }
+}
+
+// The NW warps of sh_w joined in the same way by one warp into *out.
+template <int NW>
+__device__ __forceinline__ void tile_stats_join(const double *w,
+                                                TileStats *out)
+{
+    const int lane = threadIdx.x & 31;
+    LseRef r;
+    double tx = 0.0, ty = 0.0;
+    r.init();
+    if (lane < NW) {
+        r.ref = w[0 * NW + lane];
+        r.mx = r.ref;
+        r.s1 = w[1 * NW + lane];
+        r.s2 = w[2 * NW + lane];
+        r.sx = w[3 * NW + lane];
+        r.sy = w[4 * NW + lane];
+        tx = w[5 * NW + lane];
+        ty = w[6 * NW + lane];
     }
+    const double tm = warp_max_nan(r.mx, NW);
+    lse_rescale(r, tm);
+    warp_sum_stats(r, tx, ty, NW);
+    if (lane == 0) {
+        TileStats ts;
+        ts.m = tm;
+        ts.s1 = r.s1;
+        ts.s2 = r.s2;
+        ts.sx = r.sx;
+        ts.sy = r.sy;
+        ts.gx = tx;
+        ts.gy = ty;
+        ts.pad = 0.0;
+        *out = ts;
+    }
+}
+
+// The tile's statistics from every thread's accumulator (acc, plus the sums
+// gx, gy of gathered positions, 0 where unused): tile_stats_warp, then
+// warp 0 joins the NW warps and writes *out.  `sh_w` holds 7 x NW doubles;
+// one barrier (callers that run several tiles alternate two such buffers).
+// Every thread of the CTA calls it.
+template <int NW>
+__device__ __forceinline__ void tile_stats_reduce(LseRef acc, double gx,
+                                                  double gy, double *sh_w,
+                                                  TileStats *out)
+{
+    tile_stats_warp<NW>(acc, gx, gy, sh_w, (int)(threadIdx.x >> 5));
+    __syncthreads();
+    if (threadIdx.x < 32)
+        tile_stats_join<NW>(sh_w, out);
 }
 
 } // namespace vsmc_b200

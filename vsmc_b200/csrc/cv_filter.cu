@@ -48,7 +48,6 @@ struct vsmc_cuda_cv_filter {
     double *mon_part;
     ResampleWorkspace rws;
     long long ntiles;
-    int move_grid;
     uint64_t iter;   // steps launched so far
     uint64_t T_obs;
     EngineRef eng;
@@ -127,6 +126,45 @@ void join_sequence(vsmc_cuda_cv_filter *f)
         cudaStreamWaitEvent(f->stream, f->ev_seq, 0);
 }
 
+template <typename Real, bool Init, int S>
+void launch_move_split(const MoveArgs<Real> &a, cudaStream_t s)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)(a.ntiles * S));
+    c.blockDim = dim3(kMoveThreads);
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = S;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k_cv_move_split<Real, Init, S>, a);
+}
+
+// The largest split of a tile whose CTAs are at most two per SM, else one
+// CTA per tile.  Measured (FP64 move with its events, us; whole tile, 2, 4
+// and 8 CTAs a tile): 65536 particles 29.0, 20.8, 16.8, 16.7; 131072 29.2,
+// 21.0, 18.9, 26.9; 262144 30.3, 25.0, 33.7, 37.5; 524288 36.7, 45.1, 48.1,
+// 66.4.
+template <typename Real, bool Init>
+void launch_move(const MoveArgs<Real> &a, cudaStream_t s)
+{
+    const int room = 2 * device_sms() / a.ntiles;
+    if (room >= 8)
+        launch_move_split<Real, Init, 8>(a, s);
+    else if (room >= 4)
+        launch_move_split<Real, Init, 4>(a, s);
+    else if (room >= 2)
+        launch_move_split<Real, Init, 2>(a, s);
+    else
+        // the block scheduler hands tiles to SMs as they free, which
+        // balances the rejection loops' uneven cost better than a
+        // persistent grid striding over tiles (measured 5% faster at 2^24)
+        k_cv_move<Real, Init><<<a.ntiles, kMoveThreads, 0, s>>>(a);
+}
+
 template <typename Real>
 void launch_step(vsmc_cuda_cv_filter *f, bool init)
 {
@@ -170,9 +208,9 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
         cudaEventRecord(ev[0], s);
     }
     if (init)
-        k_cv_move<Real, true><<<f->move_grid, kMoveThreads, 0, s>>>(a);
+        launch_move<Real, true>(a, s);
     else
-        k_cv_move<Real, false><<<f->move_grid, kMoveThreads, 0, s>>>(a);
+        launch_move<Real, false>(a, s);
     if (ev)
         cudaEventRecord(ev[1], s);
     f->cur = dst;
@@ -415,10 +453,6 @@ int vsmc_cuda_cv_create(const vsmc_cuda_cv_config *cfg, void *stream,
     cudaFuncSetAttribute(k_cv_finalize,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kFinalSmemTiles * (int)sizeof(double));
-    // one CTA per tile: the block scheduler hands tiles to SMs as they
-    // free, which balances the rejection loops' uneven cost better than a
-    // persistent grid striding over tiles (measured 5% faster at 2^24)
-    f->move_grid = (int)f->ntiles;
     e = cudaMemsetAsync(f->mem, 0, f->bytes, f->stream);
     // (a filter that resamples in one cluster draws its sequence there)
     if (e == cudaSuccess && cfg->scheme == VSMC_CUDA_MULTINOMIAL &&

@@ -13,6 +13,8 @@
 // 274-302 with integrate/is_integrate.hpp:56-80 (posterior mean).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "resample.cuh"
 
 namespace vsmc_b200 {
@@ -358,6 +360,166 @@ k_cv_move(MoveArgs<Real> a)
         cv_move_tile<Real, Init>(a, ms, tile, sh_w[buf]);
         buf ^= 1;
     }
+}
+
+// ---- the move of a small filter -------------------------------------
+// A tile's CTA takes its 8 particles per thread one after another (about
+// 4 us each: the FP64 chains and Philox blocks of one warp), and a filter of
+// nt tiles keeps nt SMs busy.  Here a cluster of S CTAs shares a tile, each
+// thread moving kMoveItems / S particles.  The tile's statistics keep the
+// one-CTA association: they are sums over 256 lanes of 8 particles each in
+// order, so every particle's log-weight and position go to the CTA that
+// folds its lane (distributed shared memory), whose warps fold and reduce
+// exactly as tile_stats_reduce's; the warps' results meet in CTA 0.
+template <typename Real, int S>
+struct MoveSplitShared {
+    static constexpr int kLanes = kMoveThreads / S; // folded by one CTA
+    Real lw[kMoveItems][kLanes], x[kMoveItems][kLanes], y[kMoveItems][kLanes];
+    Real gx[kMoveItems][kLanes], gy[kMoveItems][kLanes];
+    double sh_w[7 * kMoveWarps];
+};
+
+// Particle k (0..7) of lane `tid` of a tile.
+template <typename Real>
+__device__ __forceinline__ int move_item(int k, int tid)
+{
+    constexpr int V = Vec<Real>::n;
+    return (k / V * kMoveThreads + tid) * V + k % V;
+}
+
+// A lane's statistics: lse_add over its particles in order.  The usual lane
+// (finite log-weights, none far above the first) evaluates the exponentials
+// independently.
+template <typename Real>
+__device__ __forceinline__ void move_fold(LseRef &acc, const Real (&l)[8],
+                                          const Real (&x)[8],
+                                          const Real (&y)[8], int n)
+{
+    bool plain = n == kMoveItems;
+#pragma unroll
+    for (int k = 0; k < kMoveItems; ++k)
+        plain = plain && l[k] > -INFINITY && l[k] < INFINITY &&
+                (double)l[k] - (double)l[0] <= LazyBound<Real>::v;
+    if (plain) {
+        acc.ref = (double)l[0];
+        double e[kMoveItems];
+#pragma unroll
+        for (int k = 0; k < kMoveItems; ++k)
+            e[k] = lse_exp((Real)(l[k] - l[0]));
+#pragma unroll
+        for (int k = 0; k < kMoveItems; ++k) {
+            acc.mx = fmax(acc.mx, (double)l[k]);
+            lse_sum(acc, e[k], (double)x[k], (double)y[k]);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kMoveItems; ++k)
+            if (k < n)
+                lse_add<Real>(acc, l[k], x[k], y[k]);
+    }
+}
+
+template <typename Real, bool Init, int S>
+__device__ __forceinline__ void cv_move_split(const MoveArgs<Real> &a,
+                                              const MoveStep<Real> &ms,
+                                              int tile,
+                                              MoveSplitShared<Real, S> &sm)
+{
+    typedef MoveSplitShared<Real, S> Sh;
+    constexpr int I = kMoveItems / S;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const long long base = (long long)tile * kTile;
+    const int tid = (int)threadIdx.x;
+    Sh &home = *cl.map_shared_rank(&sm, tid / Sh::kLanes);
+    const int lane = tid % Sh::kLanes;
+    // (no store into another CTA before it has started)
+    cl.barrier_arrive();
+#pragma unroll
+    for (int q = 0; q < I; ++q) {
+        const int k = rank * I + q;
+        const long long i = base + move_item<Real>(k, tid);
+        const bool in = i < a.N;
+        Real s[4], lwn = Real(0), gx = Real(0), gy = Real(0);
+        if (in) {
+            Real lw = Real(0);
+            if (!Init) {
+                long long src = i;
+                if (ms.gather) { // clamped: never leaves [0, N)
+                    src = a.copy_from[i];
+                    src = src < 0 ? 0 : (src >= a.N ? a.N - 1 : src);
+                } else {
+                    lw = a.lw[i];
+                }
+#pragma unroll
+                for (int d = 0; d < 4; ++d)
+                    s[d] = a.in[d][src];
+                gx = s[0];
+                gy = s[1];
+            }
+            cv_particle<Init>(a.p,
+                              polar_pair_draw(a.iter, (uint32_t)i, a.stream,
+                                              a.k0, a.k1),
+                              s[0], s[1], s[2], s[3], ms.shx, ms.shy);
+            const Real inc = cv_loglik(a.p, s[0], s[1], ms.ox, ms.oy);
+            lwn = Init ? inc : (lw - ms.mprev) + inc;
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+                a.out[d][i] = s[d];
+            a.lw[i] = lwn;
+        }
+        if (q == 0)
+            cl.barrier_wait();
+        if (in) {
+            home.lw[k][lane] = lwn;
+            home.x[k][lane] = s[0];
+            home.y[k][lane] = s[1];
+            if (ms.gather) {
+                home.gx[k][lane] = gx;
+                home.gy[k][lane] = gy;
+            }
+        }
+    }
+    cl.sync();
+    if (tid < Sh::kLanes) {
+        const int v = rank * Sh::kLanes + tid; // the lane folded here
+        Real l[kMoveItems], x[kMoveItems], y[kMoveItems];
+        double gx = 0.0, gy = 0.0;
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < kMoveItems; ++k) {
+            const bool in = base + move_item<Real>(k, v) < a.N;
+            l[k] = x[k] = y[k] = Real(0);
+            if (in) {
+                l[k] = sm.lw[k][tid];
+                x[k] = sm.x[k][tid];
+                y[k] = sm.y[k][tid];
+                if (ms.gather) {
+                    gx += (double)sm.gx[k][tid];
+                    gy += (double)sm.gy[k][tid];
+                }
+                ++n; // (a lane's particles past N are its last)
+            }
+        }
+        LseRef acc;
+        acc.init();
+        move_fold<Real>(acc, l, x, y, n);
+        tile_stats_warp<kMoveWarps>(acc, gx, gy,
+                                    cl.map_shared_rank(&sm, 0)->sh_w, v >> 5);
+    }
+    cl.sync();
+    if (rank == 0 && tid < 32)
+        tile_stats_join<kMoveWarps>(sm.sh_w, a.tile_stats + tile);
+}
+
+template <typename Real, bool Init, int S>
+__global__ void __launch_bounds__(kMoveThreads, 3)
+k_cv_move_split(MoveArgs<Real> a)
+{
+    __shared__ MoveSplitShared<Real, S> sm;
+    const MoveStep<Real> ms = move_step<Real, Init>(a);
+    cv_move_split<Real, Init, S>(a, ms, (int)(blockIdx.x / S), sm);
 }
 
 struct FinalizeArgs {

@@ -1367,9 +1367,8 @@ __device__ __forceinline__ void cp_async_wait_one()
 #define VSMC_EXACT_STAGE_MIN_BLOCKS 3
 #endif
 
-// The persistent grid of k_exact_tiles for nt tiles: the SMs times the
-// CTAs that fit on one, or fewer for small filters.
-inline int exact_grid(int nt)
+// Multiprocessors of the current device (148 when it cannot be asked).
+inline int device_sms()
 {
     static int sms = 0;
     if (sms == 0) {
@@ -1382,7 +1381,14 @@ inline int exact_grid(int nt)
         else
             sms = 148;
     }
-    const int g = sms * VSMC_EXACT_STAGE_MIN_BLOCKS;
+    return sms;
+}
+
+// The persistent grid of k_exact_tiles for nt tiles: the SMs times the
+// CTAs that fit on one, or fewer for small filters.
+inline int exact_grid(int nt)
+{
+    const int g = device_sms() * VSMC_EXACT_STAGE_MIN_BLOCKS;
     return nt < 1 ? 1 : (nt < g ? nt : g);
 }
 
