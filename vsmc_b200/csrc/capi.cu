@@ -438,7 +438,7 @@ int vsmc_cuda_resample(int scheme, uint64_t N, const double *weight,
     WeightsGiven w;
     w.w = weight;
     launch_resample(scheme, w, (long long)N, eng, ws, uniforms,
-                    (long long)n_uniforms, false, replication, cf, s);
+                    (long long)n_uniforms, replication, cf, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample: launch");
@@ -524,7 +524,7 @@ int vsmc_cuda_resample_mn(int scheme, uint64_t M, uint64_t N,
     WeightsGiven w;
     w.w = weight;
     launch_resample(scheme, w, (long long)M, eng, ws, uniforms,
-                    (long long)n_uniforms, false, rep, cf_scratch, s,
+                    (long long)n_uniforms, rep, cf_scratch, s,
                     /*cfrp=*/false, (long long)N);
     if (copy_from != nullptr)
         launch_expand(rep, (long long)M, (long long)N, ws, copy_from, s);

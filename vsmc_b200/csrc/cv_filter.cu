@@ -244,48 +244,34 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
     fa.replay_flags = f->rep_flags;
     const bool compare = f->rep_cf != nullptr && f->rec_cf != nullptr;
     fa.compare = compare ? 1 : 0;
-    const size_t fin_smem = f->ntiles <= kFinalSmemTiles
-                                ? (size_t)f->ntiles * sizeof(double)
-                                : 0;
-    k_cv_finalize<<<1, kFinalThreads, fin_smem, s>>>(fa);
-
     WeightsFromLog<Real> w;
     w.lw = static_cast<const Real *>(f->lw);
     w.stats = &f->ctl->lw_max;
+    const auto wait = [&] { cudaStreamWaitEvent(s, f->ev_seq, 0); };
     if (f->rep_cf != nullptr) {
-        if (compare) {
-            // the step's own resampling of its own weights, into the
-            // record row; the engine advances by the words it drew
-            launch_resample(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
-                            /*spine_done=*/true, nullptr,
-                            f->rec_cf + (size_t)f->iter * c.N, s);
-            f->launches += resample_launch_count(
-                N, c.scheme, WeightsFromLog<Real>::kExactNorm,
-                WeightsFromLog<Real>::kApprox);
-        }
+        // comparing: the step's own resampling of its own weights goes into
+        // the record row; the engine advances by the words it drew
+        f->launches += launch_finish(
+            c.scheme, fa, w, f->rws,
+            compare ? f->rec_cf + (size_t)f->iter * c.N : f->copy_from,
+            compare, false, [] {}, s);
         // replay: the recorded ancestry of this step (used only if the
         // recorded decision was to resample)
         cudaMemcpyAsync(f->copy_from, f->rep_cf + (size_t)f->iter * c.N,
                         c.N * 4, cudaMemcpyDeviceToDevice, s);
-    } else if (speculate) {
-        cudaStreamWaitEvent(s, f->ev_seq, 0);
-        launch_resample_core(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
-                             /*spine_done=*/true, nullptr, f->copy_from, s,
-                             /*sorted_ready=*/true);
-        f->launches -= 5; // the sequence's launches are counted on the side
-        enqueue_sequence(f); // for the next resampling
     } else {
-        launch_resample(c.scheme, w, N, f->eng, f->rws, nullptr, 0,
-                        /*spine_done=*/true, nullptr, f->copy_from, s);
+        // (a speculative sequence's launches are counted on the side)
+        f->launches += launch_finish(c.scheme, fa, w, f->rws, f->copy_from,
+                                     true, speculate, wait, s);
+        if (speculate)
+            enqueue_sequence(f); // for the next resampling
     }
     if (f->rec_cf != nullptr && !compare)
         cudaMemcpyAsync(f->rec_cf + (size_t)f->iter * c.N, f->copy_from,
                         c.N * 4, cudaMemcpyDeviceToDevice, s);
     if (ev)
         cudaEventRecord(ev[2], s);
-    f->launches += 2 + resample_launch_count(
-                           N, c.scheme, WeightsFromLog<Real>::kExactNorm,
-                           WeightsFromLog<Real>::kApprox);
+    f->launches += 1;
     ++f->iter;
 }
 

@@ -1228,15 +1228,11 @@ int vsmc_cuda_gmm_iterate(vsmc_cuda_gmm *g, uint64_t num)
         fa.eng = g->eng;
         fa.replay_flags = nullptr;
         fa.compare = 0;
-        const size_t fin_smem = g->ntiles <= kFinalSmemTiles
-                                    ? (size_t)g->ntiles * sizeof(double)
-                                    : 0;
-        k_cv_finalize<<<1, kFinalThreads, fin_smem, s>>>(fa);
         WeightsFromLog<double> w;
         w.lw = g->lw;
         w.stats = &g->ctl->lw_max;
-        launch_resample(scheme, w, N, g->eng, g->rws, nullptr, 0,
-                        /*spine_done=*/true, nullptr, g->copy_from, s);
+        g->launches += launch_finish(scheme, fa, w, g->rws, g->copy_from,
+                                     true, false, [] {}, s);
         cudaEvent_t *ev = nullptr;
         if (g->timing) {
             if (g->ev_used + 2 > g->ev.size())
@@ -1262,7 +1258,7 @@ int vsmc_cuda_gmm_iterate(vsmc_cuda_gmm *g, uint64_t num)
             g->buf[1 - g->cur].base + 13 * N, g->lw, g->ctl, N, (long long)t,
             a, g->gctl, g->hist_accept, g->hist_integrand, g->hist_grid);
         g->cur = 1 - g->cur;
-        g->launches += 4 + resample_launch_count(N, scheme, true, false);
+        g->launches += 3;
         ++g->iter;
     }
     cudaError_t e = cudaGetLastError();

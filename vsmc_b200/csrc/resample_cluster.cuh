@@ -25,7 +25,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 
-#include "resample.cuh"
+#include "cv_kernels.cuh"
 
 namespace vsmc_b200 {
 
@@ -106,6 +106,9 @@ struct RcShared {
     double u0, delta;
     int kbits;
     unsigned long long offset;
+    double excl[kRcMaxTiles]; // the weights' approximate spine (filters)
+    double stats[2];          // M, S1
+    int run;                  // the step resamples
     RcGroup g[1]; // as many as the CTA has groups
 };
 
@@ -118,10 +121,8 @@ struct RcArgs {
     long long N;      // weights
     int nt;           // their tiles
     int cfrp;         // copy_from too (0: the counts only)
-    int spine_done;   // tile_excl, NN, delta, kbits and u0 are set (filters)
     ResampleCtl *ctl;
     EngineRef eng;
-    const double *tile_excl;
     double *u;        // the U01 sequence and its bins
     int32_t *bins;
     double *rec;      // an overflow tile's weights
@@ -595,15 +596,14 @@ __device__ __forceinline__ void rc_store(int32_t *dst, long long i0,
     }
 }
 
-// One resampling; every thread of the cluster calls it.
+// One resampling; every thread of the cluster calls it.  A filter's
+// weights (kExactNorm, kApprox) read M, S1 and the spine in sm.
 template <typename W, bool Residual, int U, int R>
 __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                                             RcShared &sm)
 {
     constexpr bool Sys = U == kRcSys;
     constexpr int TT = RcThread<R>::TT;
-    if (!a.ctl->active)
-        return; // (the whole cluster)
     cg::cluster_group cl = cg::this_cluster();
     const int G = (int)blockDim.x / TT;
     const int rank = (int)cl.block_rank();
@@ -627,12 +627,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     if (threadIdx.x == 0) {
         const ResampleCtl *c = a.ctl;
         sm.offset = c->offset;
-        if (a.spine_done && !Residual) {
-            sm.NN = c->NN;
-            sm.delta = c->delta;
-            sm.kbits = c->kbits;
-            sm.u0 = Sys ? c->u0 : 0.0;
-        } else if (!Residual) {
+        if (!Residual) {
             sm.NN = Nout;
             sm.delta = __ddiv_rn(1.0, Nd);
             sm.kbits = bin_kbits(Nout);
@@ -674,7 +669,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
                 run += w[j];
             pre = rc_excl_scan(run, g.red_d, th, total);
             rc_classify(base, N, w,
-                        __dmul_rn(a.tile_excl[tile], wsrc.spine_unnorm()),
+                        __dmul_rn(sm.excl[tile], wsrc.spine_unnorm()),
                         pre, ExactMargin<W>::rel, th, g, g.scan[kRcA], a.rec,
                         rw);
         }
@@ -996,7 +991,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     } else if (W::kExactNorm) {
         if (act)
             rc_classify(base, N, w,
-                        __dmul_rn(a.tile_excl[tile],
+                        __dmul_rn(sm.excl[tile],
                                   __ddiv_rn(wsrc.spine_unnorm(),
                                             rc_start(sm.w, nt))),
                         pre, ExactMargin<W>::rel, th, g, g.scan[kRcB], a.rec,
@@ -1323,6 +1318,114 @@ k_resample_cluster(W wsrc, RcArgs a)
                                    *reinterpret_cast<RcShared *>(rc_smem));
 }
 
+// k_cv_finalize_body for at most 32 tiles, by one warp (lane t holds tile
+// t, as thread t does there): every CTA of a cluster computes the step's
+// maximum, sums and decision, CTA 0 writes them.  Leaves M, S1, the spine
+// and the decision in sm.
+__device__ __forceinline__ void rc_finalize(const FinalizeArgs &a,
+                                            RcShared &sm, bool writer)
+{
+    const int lane = threadIdx.x & 31;
+    FilterCtl *c = a.ctl;
+    int c_res = 0;
+    long long c_mdone = 0;
+    double c_s1 = 0.0, c_logz = 0.0;
+    double ax0 = 0.0, ay0 = 0.0, ax1 = 0.0, ay1 = 0.0;
+    if (writer && lane == 0) {
+        c_res = c->resampled;
+        c_mdone = c->monitor_done;
+        c_s1 = c->s1;
+        c_logz = c->logz;
+        if (a.anchored) {
+            if (!a.init) {
+                ax0 = a.obs_x[a.t - 1];
+                ay0 = a.obs_y[a.t - 1];
+            }
+            ax1 = a.obs_x[a.t];
+            ay1 = a.obs_y[a.t];
+        }
+    }
+    const int rflag =
+        a.replay_flags != nullptr ? a.replay_flags[a.t] : 0;
+    TileStats ts;
+    ts.m = -INFINITY;
+    ts.s1 = ts.s2 = ts.sx = ts.sy = ts.gx = ts.gy = 0.0;
+    if (lane < a.ntiles)
+        ts = a.ts[lane];
+    double M = (ts.m != ts.m || ts.s1 != ts.s1) ? NAN : ts.m;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double q = __shfl_xor_sync(0xffffffffu, M, o);
+        M = (q != q || M != M) ? NAN : fmax(M, q);
+    }
+    const double f = ts.m == -INFINITY ? 0.0 : fm::fm_exp(ts.m - M);
+    const double share = __dmul_rn(ts.s1, f);
+    const double S1 = warp_sum(share);
+    const double S2 = warp_sum(__dmul_rn(__dmul_rn(ts.s2, f), f));
+    const double sx = warp_sum(__dmul_rn(ts.sx, f));
+    const double sy = warp_sum(__dmul_rn(ts.sy, f));
+    const double gx = warp_sum(ts.gx), gy = warp_sum(ts.gy);
+    const double Nd = (double)a.N;
+    const bool bad = !(M > -INFINITY && M < INFINITY && S1 > 0.0 &&
+                       S1 < INFINITY && S2 > 0.0 && S2 < INFINITY);
+    const double ess = bad ? NAN : S1 * S1 / S2;
+    const int own = bad ? 0 : ess < a.threshold * Nd;
+    // the step's own decision resamples unless the step follows a recorded
+    // ancestry without comparing
+    const int run = a.replay_flags == nullptr || a.compare ? own : 0;
+    const int res = a.replay_flags != nullptr ? rflag != 0 : own;
+    // the spine of the normalised shares, for the classification
+    const double sh = share * __ddiv_rn(1.0, S1);
+    const double excl = warp_incl_scan(sh) - sh;
+    sm.excl[lane] = excl;
+    if (lane != 0)
+        return;
+    sm.stats[0] = M;
+    sm.stats[1] = S1;
+    sm.run = run;
+    if (!writer)
+        return;
+    // monitor of the previous step, gathered by this move
+    if (!a.init && c_res && c_mdone != a.t - 1) {
+        a.hist_mean_x[a.t - 1] = ax0 + gx / Nd;
+        a.hist_mean_y[a.t - 1] = ay0 + gy / Nd;
+        c->monitor_done = a.t - 1;
+    }
+    const double s1prev = (a.init || c_res) ? Nd : c_s1;
+    const double dz = bad ? NAN : M + log(S1) - log(s1prev);
+    if (bad)
+        c->error = VSMC_CUDA_EDEGENERATE;
+    a.hist_ess[a.t] = ess;
+    a.hist_resampled[a.t] = res;
+    a.hist_logz_inc[a.t] = dz;
+    c->logz = c_logz + dz;
+    c->lw_max = M;
+    c->s1 = S1;
+    c->s2 = S2;
+    c->ess = ess;
+    c->resampled = res;
+    if (!res) {
+        a.hist_mean_x[a.t] = ax1 + sx / S1;
+        a.hist_mean_y[a.t] = ay1 + sy / S1;
+    }
+    a.rctl->active = run;
+}
+
+// A step's finalisation and resampling.
+template <typename W, bool Residual, int U, int R>
+__global__ void __launch_bounds__(R == 8 ? 512 : kTile / R, 1)
+k_finish_cluster(FinalizeArgs fa, W wsrc, RcArgs a)
+{
+    extern __shared__ __align__(16) unsigned char rc_smem[];
+    RcShared &sm = *reinterpret_cast<RcShared *>(rc_smem);
+    if (threadIdx.x < 32)
+        rc_finalize(fa, sm, cg::this_cluster().block_rank() == 0);
+    __syncthreads();
+    if (!sm.run)
+        return; // (the whole cluster: every CTA takes the same decision)
+    wsrc.stats = sm.stats;
+    rc_resample<W, Residual, U, R>(wsrc, a, sm);
+}
+
 // The cluster of nt tiles: up to 16 a CTA of 1024 threads each (two
 // particles a thread), above two tiles a CTA of 512 threads (eight).
 struct RcShape {
@@ -1376,76 +1479,120 @@ inline bool rc_fits(long long N, long long Nout)
     return resample_ntiles(n) <= kRcMaxTiles;
 }
 
-template <typename W, bool Residual, int U>
-inline void rc_launch_shape(const RcShape &sh, const W &w, const RcArgs &a,
-                            cudaStream_t s)
+// The scheme's instance: f(residual, sequence) with compile-time constants.
+template <typename F>
+inline void rc_scheme(int scheme, F f)
 {
-    if (sh.r == 8)
-        rc_launch(k_resample_cluster<W, Residual, U, 8>, sh, 1, s, w, a);
-    else
-        rc_launch(k_resample_cluster<W, Residual, U, 2>, sh, 1, s, w, a);
+    typedef std::integral_constant<int, kRcSorted> Sorted;
+    typedef std::integral_constant<int, kRcStrat> Strat;
+    typedef std::integral_constant<int, kRcSys> Syst;
+    switch (scheme) {
+    case VSMC_CUDA_MULTINOMIAL:
+        f(std::false_type(), Sorted());
+        break;
+    case VSMC_CUDA_RESIDUAL:
+        f(std::true_type(), Sorted());
+        break;
+    case VSMC_CUDA_STRATIFIED:
+        f(std::false_type(), Strat());
+        break;
+    case VSMC_CUDA_SYSTEMATIC:
+        f(std::false_type(), Syst());
+        break;
+    case VSMC_CUDA_RESIDUAL_STRATIFIED:
+        f(std::true_type(), Strat());
+        break;
+    default:
+        f(std::true_type(), Syst());
+        break;
+    }
 }
 
-// A resampling: one cluster where it fits, the launch sequence of
-// resample.cuh otherwise (and for caller-supplied uniforms).
-template <typename W>
-inline void launch_resample(int scheme, W wsrc, long long N,
-                            const EngineRef &eng, ResampleWorkspace &ws,
-                            const double *u_given, long long n_given,
-                            bool spine_done, int32_t *rep_out,
-                            int32_t *copy_from, cudaStream_t s,
-                            bool cfrp = true, long long Nout = 0)
+inline RcArgs rc_args(long long N, const EngineRef &eng,
+                      const ResampleWorkspace &ws, int32_t *rep_out,
+                      int32_t *copy_from, bool cfrp)
 {
-    if (u_given != nullptr || !rc_fits(N, Nout) ||
-        (W::kExactNorm && !spine_done)) {
-        launch_resample_core(scheme, wsrc, N, eng, ws, u_given, n_given,
-                             spine_done, rep_out, copy_from, s, false, cfrp,
-                             Nout);
-        return;
-    }
     RcArgs a;
     a.N = N;
     a.nt = resample_ntiles(N);
     a.cfrp = cfrp ? 1 : 0;
-    a.spine_done = spine_done ? 1 : 0;
     a.ctl = ws.ctl;
     a.eng = eng;
-    a.tile_excl = ws.tile_excl;
     a.u = ws.u;
     a.bins = ws.bins;
     a.rec = ws.ex.rec;
     a.rep_out = rep_out;
     a.copy_from = copy_from;
-    const RcShape sh = rc_shape(resample_ntiles(Nout > N ? Nout : N));
-    switch (scheme) {
-    case VSMC_CUDA_MULTINOMIAL:
-        rc_launch_shape<W, false, kRcSorted>(sh, wsrc, a, s);
-        break;
-    case VSMC_CUDA_RESIDUAL:
-        rc_launch_shape<W, true, kRcSorted>(sh, wsrc, a, s);
-        break;
-    case VSMC_CUDA_STRATIFIED:
-        rc_launch_shape<W, false, kRcStrat>(sh, wsrc, a, s);
-        break;
-    case VSMC_CUDA_SYSTEMATIC:
-        rc_launch_shape<W, false, kRcSys>(sh, wsrc, a, s);
-        break;
-    case VSMC_CUDA_RESIDUAL_STRATIFIED:
-        rc_launch_shape<W, true, kRcStrat>(sh, wsrc, a, s);
-        break;
-    default:
-        rc_launch_shape<W, true, kRcSys>(sh, wsrc, a, s);
-        break;
-    }
+    return a;
 }
 
-// Kernels launch_resample issues (for the launch counters).
-inline int resample_launch_count(long long N, int scheme, bool exact_norm,
-                                 bool approx)
+// A resampling of given weights: one cluster where it fits, the launch
+// sequence of resample.cuh otherwise (and for caller-supplied uniforms).
+inline void launch_resample(int scheme, WeightsGiven w, long long N,
+                            const EngineRef &eng, ResampleWorkspace &ws,
+                            const double *u_given, long long n_given,
+                            int32_t *rep_out, int32_t *copy_from,
+                            cudaStream_t s, bool cfrp = true,
+                            long long Nout = 0)
 {
-    return rc_fits(N, 0)
-               ? 1
-               : resample_launches(scheme, false, exact_norm, approx);
+    if (u_given != nullptr || !rc_fits(N, Nout)) {
+        launch_resample_core(scheme, w, N, eng, ws, u_given, n_given, false,
+                             rep_out, copy_from, s, false, cfrp, Nout);
+        return;
+    }
+    const RcArgs a = rc_args(N, eng, ws, rep_out, copy_from, cfrp);
+    const RcShape sh = rc_shape(resample_ntiles(Nout > N ? Nout : N));
+    rc_scheme(scheme, [&](auto res, auto seq) {
+        constexpr bool Re = decltype(res)::value;
+        constexpr int U = decltype(seq)::value;
+        if (sh.r == 8)
+            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, s, w,
+                      a);
+        else
+            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, s, w,
+                      a);
+    });
+}
+
+// A filter step after its tile statistics: the finalisation (fa) and the
+// resampling of the weights w into copy_from.  One cluster where it fits;
+// else k_cv_finalize and the launch sequence (sorted_ready: the sorted
+// sequence is drawn elsewhere, `wait` orders the stream after it).
+// Returns the kernels launched (the caller's counter).
+template <typename W, typename Wait>
+inline int launch_finish(int scheme, const FinalizeArgs &fa, const W &w,
+                         ResampleWorkspace &ws, int32_t *copy_from,
+                         bool resample, bool sorted_ready, Wait wait,
+                         cudaStream_t s)
+{
+    const long long N = fa.N;
+    if (rc_fits(N, 0)) {
+        const RcArgs a = rc_args(N, fa.eng, ws, nullptr, copy_from, true);
+        const RcShape sh = rc_shape(fa.ntiles);
+        rc_scheme(scheme, [&](auto res, auto seq) {
+            constexpr bool Re = decltype(res)::value;
+            constexpr int U = decltype(seq)::value;
+            if (sh.r == 8)
+                rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, s, fa, w, a);
+            else
+                rc_launch(k_finish_cluster<W, Re, U, 2>, sh, 1, s, fa, w, a);
+        });
+        return 1;
+    }
+    const size_t smem = fa.ntiles <= kFinalSmemTiles
+                            ? (size_t)fa.ntiles * sizeof(double)
+                            : 0;
+    k_cv_finalize<<<1, kFinalThreads, smem, s>>>(fa);
+    if (!resample)
+        return 1;
+    if (sorted_ready)
+        wait();
+    launch_resample_core(scheme, w, N, fa.eng, ws, nullptr, 0,
+                         /*spine_done=*/true, nullptr, copy_from, s,
+                         sorted_ready);
+    return 1 +
+           resample_launches(scheme, false, W::kExactNorm, W::kApprox) -
+           (sorted_ready ? 5 : 0);
 }
 
 } // namespace vsmc_b200

@@ -160,7 +160,7 @@ extern "C" int vsmc_cuda_resample_noalloc(int scheme, uint64_t N,
     WeightsGiven w;
     w.w = weight;
     launch_resample(scheme, w, (long long)N, eng, ws, uniforms,
-                    (long long)n_uniforms, false, replication, cf, s);
+                    (long long)n_uniforms, replication, cf, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_noalloc: launch");

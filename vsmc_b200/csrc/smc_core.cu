@@ -267,16 +267,11 @@ int vsmc_cuda_smc_finish_step(vsmc_cuda_smc *s)
     fa.eng = s->eng;
     fa.replay_flags = nullptr;
     fa.compare = 0;
-    const size_t fin_smem = s->ntiles <= kFinalSmemTiles
-                                ? (size_t)s->ntiles * sizeof(double)
-                                : 0;
-    k_cv_finalize<<<1, kFinalThreads, fin_smem, s->stream>>>(fa);
     WeightsFromLog<double> w;
     w.lw = s->lw;
     w.stats = &s->ctl->lw_max;
-    launch_resample(sch, w, N, s->eng, s->rws, nullptr, 0,
-                    /*spine_done=*/true, nullptr, s->copy_from, s->stream);
-    s->launches += 1 + resample_launch_count(N, sch, true, false);
+    s->launches += launch_finish(sch, fa, w, s->rws, s->copy_from, true,
+                                 false, [] {}, s->stream);
     ++s->iter;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VSMC_CUDA_OK
