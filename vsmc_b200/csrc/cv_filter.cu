@@ -133,13 +133,15 @@ void launch_move_split(const MoveArgs<Real> &a, cudaStream_t s)
     c.gridDim = dim3((unsigned)(a.ntiles * S));
     c.blockDim = dim3(kMoveThreads);
     c.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = S;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
-    c.numAttrs = 1;
+    c.numAttrs = 2;
     cudaLaunchKernelEx(&c, k_cv_move_split<Real, Init, S>, a);
 }
 
@@ -148,10 +150,13 @@ void launch_move_split(const MoveArgs<Real> &a, cudaStream_t s)
 // and 8 CTAs a tile): 65536 particles 29.0, 20.8, 16.8, 16.7; 131072 29.2,
 // 21.0, 18.9, 26.9; 262144 30.3, 25.0, 33.7, 37.5; 524288 36.7, 45.1, 48.1,
 // 66.4.
+// (A Multinomial filter's sequence, drawn on its second stream meanwhile,
+// wants the SMs itself: split, the step at 131072 particles took 124 us
+// instead of 116.)
 template <typename Real, bool Init>
-void launch_move(const MoveArgs<Real> &a, cudaStream_t s)
+void launch_move(const MoveArgs<Real> &a, bool alone, cudaStream_t s)
 {
-    const int room = 2 * device_sms() / a.ntiles;
+    const int room = alone ? 2 * device_sms() / a.ntiles : 0;
     if (room >= 8)
         launch_move_split<Real, Init, 8>(a, s);
     else if (room >= 4)
@@ -208,9 +213,9 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
         cudaEventRecord(ev[0], s);
     }
     if (init)
-        launch_move<Real, true>(a, s);
+        launch_move<Real, true>(a, !speculate, s);
     else
-        launch_move<Real, false>(a, s);
+        launch_move<Real, false>(a, !speculate, s);
     if (ev)
         cudaEventRecord(ev[1], s);
     f->cur = dst;

@@ -107,22 +107,50 @@ __device__ __forceinline__ double polar_r2(double x, double y)
     return __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
 }
 
-// FP64 form: cv_move::move_state / cv_init::initialize_state
-// (pf_smp.hpp:150-173, 207-238).  The two polar transforms are evaluated
-// together (independent chains for the FP64 pipe); the state update keeps
-// the reference's evaluation order.
-template <bool Init>
-__device__ __forceinline__ void cv_particle(const CVParam &p,
-                                            const PolarPair &pp, double &x,
-                                            double &y, double &vx,
-                                            double &vy, double, double)
+// A particle's four standard normals in the reference's order (x, y, vx,
+// vy): they depend on its stream alone, not on its state.
+template <typename Real>
+struct CVNormals {
+    Real a, b, c, d;
+};
+
+// FP64: the two polar transforms are evaluated together (independent chains
+// for the FP64 pipe).
+__device__ __forceinline__ void cv_normals(const PolarPair &pp,
+                                           CVNormals<double> &n)
 {
     const double x1 = pp.x1, y1 = pp.y1, x2 = pp.x2, y2 = pp.y2;
     const double q1 = polar_r2(x1, y1), q2 = polar_r2(x2, y2);
     const double m1 = polar_mult_f64(q1);
     const double m2 = polar_mult_f64(q2);
-    const double a = __dmul_rn(y1, m1), b = __dmul_rn(x1, m1);
-    const double c = __dmul_rn(y2, m2), d = __dmul_rn(x2, m2);
+    n.a = __dmul_rn(y1, m1);
+    n.b = __dmul_rn(x1, m1);
+    n.c = __dmul_rn(y2, m2);
+    n.d = __dmul_rn(x2, m2);
+}
+
+__device__ __forceinline__ void cv_normals(const PolarPair &pp,
+                                           CVNormals<float> &n)
+{
+    const double x1 = pp.x1, y1 = pp.y1, x2 = pp.x2, y2 = pp.y2;
+    const double q1 = polar_r2(x1, y1), q2 = polar_r2(x2, y2);
+    const float m1 = polar_mult_f32(q1), m2 = polar_mult_f32(q2);
+    n.a = (float)y1 * m1;
+    n.b = (float)x1 * m1;
+    n.c = (float)y2 * m2;
+    n.d = (float)x2 * m2;
+}
+
+// FP64 form: cv_move::move_state / cv_init::initialize_state
+// (pf_smp.hpp:150-173, 207-238) from the normals; the state update keeps
+// the reference's evaluation order.
+template <bool Init>
+__device__ __forceinline__ void cv_update(const CVParam &p,
+                                          const CVNormals<double> &n,
+                                          double &x, double &y, double &vx,
+                                          double &vy, double, double)
+{
+    const double a = n.a, b = n.b, c = n.c, d = n.d;
     if (Init) {
         x = plus0(__dmul_rn(a, p.sd_pos0));
         y = plus0(__dmul_rn(b, p.sd_pos0));
@@ -138,6 +166,17 @@ __device__ __forceinline__ void cv_particle(const CVParam &p,
         vx = __dadd_rn(vx, n3);
         vy = __dadd_rn(vy, n4);
     }
+}
+
+template <bool Init>
+__device__ __forceinline__ void cv_particle(const CVParam &p,
+                                            const PolarPair &pp, double &x,
+                                            double &y, double &vx,
+                                            double &vy, double, double)
+{
+    CVNormals<double> n;
+    cv_normals(pp, n);
+    cv_update<Init>(p, n, x, y, vx, vy, 0.0, 0.0);
 }
 
 // cv_state::log_likelihood (pf_smp.hpp:96-112): the two Student-t terms
@@ -157,6 +196,19 @@ __device__ __forceinline__ double cv_loglik(const CVParam &p, double x,
 // residual); (shx, shy) = previous observation minus this one, in double
 // rounded once, re-anchors the loaded offsets.
 template <bool Init>
+__device__ __forceinline__ void cv_update(const CVParam &p,
+                                          const CVNormals<float> &n, float &x,
+                                          float &y, float &vx, float &vy,
+                                          double shx, double shy)
+{
+    const float dt = (float)p.dt;
+    x = (x + (float)shx) + (n.a * (float)p.sd_pos + dt * vx);
+    y = (y + (float)shy) + (n.b * (float)p.sd_pos + dt * vy);
+    vx = vx + n.c * (float)p.sd_vel;
+    vy = vy + n.d * (float)p.sd_vel;
+}
+
+template <bool Init>
 __device__ __forceinline__ void cv_particle(const CVParam &p,
                                             const PolarPair &pp, float &x,
                                             float &y, float &vx, float &vy,
@@ -172,12 +224,9 @@ __device__ __forceinline__ void cv_particle(const CVParam &p,
         vx = (float)(y2 * m2 * p.sd_vel0);
         vy = (float)(x2 * m2 * p.sd_vel0);
     } else {
-        const float m1 = polar_mult_f32(q1), m2 = polar_mult_f32(q2);
-        const float dt = (float)p.dt;
-        x = (x + (float)shx) + ((float)y1 * m1 * (float)p.sd_pos + dt * vx);
-        y = (y + (float)shy) + ((float)x1 * m1 * (float)p.sd_pos + dt * vy);
-        vx = vx + (float)y2 * m2 * (float)p.sd_vel;
-        vy = vy + (float)x2 * m2 * (float)p.sd_vel;
+        CVNormals<float> n;
+        cv_normals(pp, n);
+        cv_update<false>(p, n, x, y, vx, vy, shx, shy);
     }
 }
 
@@ -371,6 +420,11 @@ k_cv_move(MoveArgs<Real> a)
 // order, so every particle's log-weight and position go to the CTA that
 // folds its lane (distributed shared memory), whose warps fold and reduce
 // exactly as tile_stats_reduce's; the warps' results meet in CTA 0.
+//
+// The kernel is launched while the previous kernel of the stream still runs
+// (programmatic dependent launch): a particle's normals need its counter
+// stream only, so they are drawn before the wait for that kernel, on SMs a
+// small filter's resampling leaves idle.
 template <typename Real, int S>
 struct MoveSplitShared {
     static constexpr int kLanes = kMoveThreads / S; // folded by one CTA
@@ -421,7 +475,6 @@ __device__ __forceinline__ void move_fold(LseRef &acc, const Real (&l)[8],
 
 template <typename Real, bool Init, int S>
 __device__ __forceinline__ void cv_move_split(const MoveArgs<Real> &a,
-                                              const MoveStep<Real> &ms,
                                               int tile,
                                               MoveSplitShared<Real, S> &sm)
 {
@@ -436,6 +489,20 @@ __device__ __forceinline__ void cv_move_split(const MoveArgs<Real> &a,
     const int lane = tid % Sh::kLanes;
     // (no store into another CTA before it has started)
     cl.barrier_arrive();
+    // the normals, while the previous step's resampling still runs
+    CVNormals<Real> nrm[I];
+    if (!Init) {
+#pragma unroll
+        for (int q = 0; q < I; ++q) {
+            const long long i = base + move_item<Real>(rank * I + q, tid);
+            if (i < a.N)
+                cv_normals(polar_pair_draw(a.iter, (uint32_t)i, a.stream,
+                                           a.k0, a.k1),
+                           nrm[q]);
+        }
+    }
+    pdl_wait();
+    const MoveStep<Real> ms = move_step<Real, Init>(a);
 #pragma unroll
     for (int q = 0; q < I; ++q) {
         const int k = rank * I + q;
@@ -445,23 +512,28 @@ __device__ __forceinline__ void cv_move_split(const MoveArgs<Real> &a,
         if (in) {
             Real lw = Real(0);
             if (!Init) {
+                // (both read at once: the flag decides which counts)
+                const long long cf = a.copy_from[i];
+                const Real lw0 = a.lw[i];
                 long long src = i;
-                if (ms.gather) { // clamped: never leaves [0, N)
-                    src = a.copy_from[i];
-                    src = src < 0 ? 0 : (src >= a.N ? a.N - 1 : src);
-                } else {
-                    lw = a.lw[i];
-                }
+                if (ms.gather) // clamped: never leaves [0, N)
+                    src = cf < 0 ? 0 : (cf >= a.N ? a.N - 1 : cf);
+                else
+                    lw = lw0;
 #pragma unroll
                 for (int d = 0; d < 4; ++d)
                     s[d] = a.in[d][src];
                 gx = s[0];
                 gy = s[1];
             }
-            cv_particle<Init>(a.p,
-                              polar_pair_draw(a.iter, (uint32_t)i, a.stream,
-                                              a.k0, a.k1),
-                              s[0], s[1], s[2], s[3], ms.shx, ms.shy);
+            if (Init)
+                cv_particle<Init>(a.p,
+                                  polar_pair_draw(a.iter, (uint32_t)i,
+                                                  a.stream, a.k0, a.k1),
+                                  s[0], s[1], s[2], s[3], ms.shx, ms.shy);
+            else
+                cv_update<false>(a.p, nrm[q], s[0], s[1], s[2], s[3], ms.shx,
+                                 ms.shy);
             const Real inc = cv_loglik(a.p, s[0], s[1], ms.ox, ms.oy);
             lwn = Init ? inc : (lw - ms.mprev) + inc;
 #pragma unroll
@@ -518,8 +590,8 @@ __global__ void __launch_bounds__(kMoveThreads, 3)
 k_cv_move_split(MoveArgs<Real> a)
 {
     __shared__ MoveSplitShared<Real, S> sm;
-    const MoveStep<Real> ms = move_step<Real, Init>(a);
-    cv_move_split<Real, Init, S>(a, ms, (int)(blockIdx.x / S), sm);
+    pdl_launch();
+    cv_move_split<Real, Init, S>(a, (int)(blockIdx.x / S), sm);
 }
 
 struct FinalizeArgs {

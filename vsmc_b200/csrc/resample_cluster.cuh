@@ -1417,6 +1417,8 @@ k_finish_cluster(FinalizeArgs fa, W wsrc, RcArgs a)
 {
     extern __shared__ __align__(16) unsigned char rc_smem[];
     RcShared &sm = *reinterpret_cast<RcShared *>(rc_smem);
+    pdl_wait();
+    pdl_launch(); // the next move draws its normals meanwhile
     if (threadIdx.x < 32)
         rc_finalize(fa, sm, cg::this_cluster().block_rank() == 0);
     __syncthreads();
@@ -1443,9 +1445,10 @@ inline RcShape rc_shape(int nt)
     return s;
 }
 
-// Launches `k` with one cluster of `shape` per `clusters`.
+// Launches `k` with one cluster of `shape` per `clusters`; `early`: before
+// the stream's previous kernel has ended (k waits itself).
 template <typename K, typename... A>
-inline cudaError_t rc_launch(K k, RcShape shape, int clusters,
+inline cudaError_t rc_launch(K k, RcShape shape, int clusters, bool early,
                              cudaStream_t s, const A &...args)
 {
     const size_t smem = rc_smem_bytes(shape.groups);
@@ -1461,13 +1464,15 @@ inline cudaError_t rc_launch(K k, RcShape shape, int clusters,
     c.blockDim = dim3((unsigned)(kTile / shape.r * shape.groups));
     c.dynamicSmemBytes = smem;
     c.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)shape.ctas;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
-    c.numAttrs = 1;
+    c.numAttrs = early ? 2 : 1;
     return cudaLaunchKernelEx(&c, k, args...);
 }
 
@@ -1546,11 +1551,11 @@ inline void launch_resample(int scheme, WeightsGiven w, long long N,
         constexpr bool Re = decltype(res)::value;
         constexpr int U = decltype(seq)::value;
         if (sh.r == 8)
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, s, w,
-                      a);
+            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, false, s,
+                      w, a);
         else
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, s, w,
-                      a);
+            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, false, s,
+                      w, a);
     });
 }
 
@@ -1573,9 +1578,11 @@ inline int launch_finish(int scheme, const FinalizeArgs &fa, const W &w,
             constexpr bool Re = decltype(res)::value;
             constexpr int U = decltype(seq)::value;
             if (sh.r == 8)
-                rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, s, fa, w, a);
+                rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, true, s, fa, w,
+                          a);
             else
-                rc_launch(k_finish_cluster<W, Re, U, 2>, sh, 1, s, fa, w, a);
+                rc_launch(k_finish_cluster<W, Re, U, 2>, sh, 1, true, s, fa, w,
+                          a);
         });
         return 1;
     }

@@ -97,6 +97,18 @@ __device__ __forceinline__ float polar_mult_f32(double r2)
     return sqrtf(-2.0f * logf(r2f) / r2f);
 }
 
+// Programmatic dependent launch: let the stream's next kernel start its
+// independent part / wait until every kernel this one depends on is done.
+// Without the launch attribute both do nothing.
+__device__ __forceinline__ void pdl_launch()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // --------------------------------------------------------- reductions ------
 __device__ __forceinline__ double warp_sum(double v)
 {
