@@ -1,0 +1,138 @@
+// call_scratch.cu -- see call_scratch.hpp.
+#include "call_scratch.hpp"
+
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+
+namespace vsmc_b200 {
+
+namespace {
+
+constexpr int kEntries = 16; // (device, context) pairs served
+constexpr int kSlots = 64;   // calls in flight per pair
+
+struct Entry {
+    int dev;
+    void *ctx;
+    char *host;
+    uint64_t used;
+    cudaMemPool_t pool;
+    bool has_pool;
+};
+
+std::mutex g_mutex;
+Entry g_entries[kEntries];
+int g_n = 0;
+
+typedef int (*CtxGetCurrentFn)(void **);
+
+// The current context (cuCtxGetCurrent through the runtime's driver entry
+// point): what the entries belong to.  cudaDeviceReset ends a context and
+// its memory; the next one is another entry.
+void *context()
+{
+    static CtxGetCurrentFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault,
+                                    &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<CtxGetCurrentFn>(p);
+    }();
+    void *ctx = nullptr;
+    if (fn == nullptr || fn(&ctx) != 0)
+        return nullptr;
+    return ctx;
+}
+
+// The entry of the current device and context, or -1.  Called with the
+// mutex held.  A stream that is being captured gets none (creating it would
+// end the capture).
+int find_entry(cudaStream_t s)
+{
+    int dev = 0;
+    void *ctx = context();
+    if (ctx == nullptr || cudaGetDevice(&dev) != cudaSuccess)
+        return -1;
+    for (int k = 0; k < g_n; ++k)
+        if (g_entries[k].dev == dev && g_entries[k].ctx == ctx)
+            return k;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (g_n == kEntries || cudaStreamIsCapturing(s, &st) != cudaSuccess ||
+        st != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return -1;
+    }
+    Entry e;
+    std::memset(&e, 0, sizeof(e));
+    e.dev = dev;
+    e.ctx = ctx;
+    void *h = nullptr;
+    if (cudaHostAlloc(&h, kSlots * kSlotBytes,
+                      cudaHostAllocPortable | cudaHostAllocMapped) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    e.host = static_cast<char *>(h);
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&e.pool, &props) == cudaSuccess) {
+        uint64_t keep = kPoolKeep;
+        cudaMemPoolSetAttribute(e.pool, cudaMemPoolAttrReleaseThreshold,
+                                &keep);
+        e.has_pool = true;
+    } else {
+        cudaGetLastError();
+    }
+    g_entries[g_n] = e;
+    return g_n++;
+}
+
+} // namespace
+
+CallScratch::CallScratch(cudaStream_t s)
+    : s_(s), entry_(-1), index_(-1), slot_(nullptr), mem_(nullptr)
+{
+    std::lock_guard<std::mutex> lock(g_mutex);
+    entry_ = find_entry(s);
+    if (entry_ < 0)
+        return;
+    Entry &e = g_entries[entry_];
+    for (int k = 0; k < kSlots; ++k)
+        if (!((e.used >> k) & 1u)) {
+            e.used |= uint64_t(1) << k;
+            index_ = k;
+            slot_ = e.host + k * kSlotBytes;
+            break;
+        }
+}
+
+CallScratch::~CallScratch()
+{
+    if (mem_ != nullptr)
+        cudaFreeAsync(mem_, s_);
+    if (index_ >= 0) {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        g_entries[entry_].used &= ~(uint64_t(1) << index_);
+    }
+}
+
+cudaError_t CallScratch::alloc(size_t bytes, void **p)
+{
+    cudaError_t e =
+        entry_ >= 0 && g_entries[entry_].has_pool
+            ? cudaMallocFromPoolAsync(&mem_, bytes, g_entries[entry_].pool, s_)
+            : cudaMallocAsync(&mem_, bytes, s_);
+    if (e != cudaSuccess)
+        mem_ = nullptr;
+    *p = mem_;
+    return e;
+}
+
+} // namespace vsmc_b200

@@ -1,0 +1,43 @@
+// call_scratch.hpp -- memory for the generic entry points' calls: a small
+// pinned host slot a kernel or copy puts the call's result in, and scratch
+// device memory ordered on the caller's stream.
+//
+// cudaMallocAsync on the device's default pool gives freed memory back to
+// the system at every synchronisation (its release threshold is 0), so a
+// call that allocates, runs and waits paid for mapping and unmapping pages
+// each time: 0.5 to 3 ms a call.  The library's own pool keeps up to
+// kPoolKeep bytes.  Both are held per device and context (a handful),
+// created at the first call; every call works without them too.
+#pragma once
+
+#include <cstddef>
+#include <cuda_runtime.h>
+
+namespace vsmc_b200 {
+
+constexpr size_t kSlotBytes = 256;
+constexpr size_t kPoolKeep = 32u << 20;
+
+// A call's resources; released by the destructor (the scratch on `s`).
+class CallScratch {
+  public:
+    explicit CallScratch(cudaStream_t s);
+    ~CallScratch();
+    CallScratch(const CallScratch &) = delete;
+    CallScratch &operator=(const CallScratch &) = delete;
+
+    // Pinned host memory of kSlotBytes that device code can write, or
+    // nullptr (none free): then results go through device memory.
+    void *slot() const { return slot_; }
+    // `bytes` of device memory (once per call).
+    cudaError_t alloc(size_t bytes, void **p);
+
+  private:
+    cudaStream_t s_;
+    int entry_;
+    int index_;
+    void *slot_;
+    void *mem_;
+};
+
+} // namespace vsmc_b200

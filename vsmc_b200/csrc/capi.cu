@@ -1,7 +1,9 @@
 // capi.cu -- status handling and the generic C entry points of libvsmc_cuda:
 // RNG word streams, the device WeightSet update, the device resampler and
 // the particle gather.  The CV filter's entry points are in cv_filter.cu.
+#include "call_scratch.hpp"
 #include "resample_cluster.cuh"
+#include "weights.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -76,127 +78,28 @@ __global__ void k_threefry_words(u64x4 key, u64x4 c0, unsigned long long skip,
     }
 }
 
-// ------------------------------------------------------------- weights --
-struct WeightCtl {
-    double M, S1, S2;
-    int error;
-};
-
-__global__ void __launch_bounds__(kThreads)
-k_wadd_tiles(long long N, double *lw, const double *inc, LseAcc *tiles)
-{
-    __shared__ LseAcc sh[kThreads / 32];
-    const long long base = (long long)blockIdx.x * kTile;
-    LseAcc acc;
-    acc.init();
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-        const long long i = base + (long long)j * kThreads + threadIdx.x;
-        if (i < N) {
-            double l = lw[i];
-            if (inc != nullptr) {
-                l = __dadd_rn(l, inc[i]);
-                lw[i] = l;
-            }
-            acc.add(l, 0.0, 0.0);
-        }
-    }
-    const LseAcc r = block_reduce_lse(acc, sh);
-    if (threadIdx.x == 0)
-        tiles[blockIdx.x] = r;
-}
-
-__global__ void __launch_bounds__(kSpineThreads)
-k_wadd_reduce(const LseAcc *tiles, int ntiles, WeightCtl *ctl)
-{
-    __shared__ LseAcc sh[kSpineThreads / 32];
-    const int per = (ntiles + blockDim.x - 1) / blockDim.x;
-    const int b = threadIdx.x * per, e = min(b + per, ntiles);
-    LseAcc acc;
-    acc.init();
-    for (int t = b; t < e; ++t) {
-        if (tiles[t].s1 != tiles[t].s1)
-            acc.s1 = tiles[t].s1;
-        else
-            acc.merge(tiles[t]);
-    }
-    const LseAcc r = block_reduce_lse(acc, sh);
-    if (threadIdx.x == 0) {
-        ctl->M = r.m;
-        ctl->S1 = r.s1;
-        ctl->S2 = r.s2;
-        ctl->error = (r.m > -INFINITY && r.m < INFINITY && r.s1 > 0.0 &&
-                      r.s1 < INFINITY)
-                         ? 0
-                         : (int)VSMC_CUDA_EDEGENERATE;
-    }
-}
-
-// Sums of prospective weights b_i for WeightSet::ess(first, use_log) and
-// cess(first, use_log) (core/weight_set.hpp:132-186, compute_ess :385-409,
-// compute_cess :411-431):
-//   kind 0 (ESS, use_log):  b = exp(lw + inc - max), online log-sum-exp;
-//   kind 1 (ESS, linear):   b = w * inc;           s1 = sum |b|, s2 = sum b^2;
-//   kind 2 (CESS, use_log): s1 = sum w e^inc,      s2 = sum w e^inc e^inc;
-//   kind 3 (CESS, linear):  s1 = sum w inc,        s2 = sum w inc inc.
-// ESS = s1^2 / s2 (the reference's 1 / sum (b / asum b)^2), CESS = s1^2 / s2
-// (above^2 / below).
-__global__ void __launch_bounds__(kThreads)
-k_prospective_tiles(long long N, const double *lw, const double *w,
-                    const double *inc, int kind, LseAcc *tiles)
-{
-    __shared__ LseAcc sh[kThreads / 32];
-    const long long base = (long long)blockIdx.x * kTile;
-    LseAcc acc;
-    acc.init();
-    if (kind != 0)
-        acc.m = 0.0; // plain sums: every partial has the same reference 0
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-        const long long i = base + (long long)j * kThreads + threadIdx.x;
-        if (i >= N)
-            continue;
-        if (kind == 0) {
-            acc.add(__dadd_rn(lw[i], inc[i]), 0.0, 0.0);
-        } else if (kind == 1) {
-            // the reference normalises by asum, a sum of |b|
-            const double b = __dmul_rn(w[i], inc[i]);
-            acc.s1 = __dadd_rn(acc.s1, fabs(b));
-            acc.s2 = __dadd_rn(acc.s2, __dmul_rn(b, b));
-        } else {
-            const double b = kind == 2 ? exp(inc[i]) : inc[i];
-            const double wb = __dmul_rn(w[i], b);
-            acc.s1 = __dadd_rn(acc.s1, wb);
-            acc.s2 = __dadd_rn(acc.s2, __dmul_rn(wb, b));
-        }
-    }
-    const LseAcc r = block_reduce_lse(acc, sh);
-    if (threadIdx.x == 0)
-        tiles[blockIdx.x] = r;
-}
-
-// lw += -max (normalize_log_weight); w = exp(lw) * (1 / sum).
-__global__ void k_wadd_apply(long long N, double *lw, double *w,
-                             const WeightCtl *ctl)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N)
-        return;
-    const double l = __dadd_rn(lw[i], -ctl->M);
-    lw[i] = l;
-    if (w != nullptr)
-        w[i] = __dmul_rn(exp(l), __ddiv_rn(1.0, ctl->S1));
-}
-
-__global__ void k_copy_f64(long long N, unsigned dim, const double *src,
-                           double *dst, const int32_t *copy_from)
+// Slot i of every column from its parent: kCopyDims columns' reads in
+// flight per thread.
+constexpr int kCopyDims = 4;
+__global__ void __launch_bounds__(256)
+k_copy_f64(long long N, unsigned dim, const double *src, double *dst,
+           const int32_t *copy_from)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N)
         return;
     const long long c = copy_from[i];
-    for (unsigned d = 0; d < dim; ++d)
-        dst[(long long)d * N + i] = src[(long long)d * N + c];
+    for (unsigned d = 0; d < dim; d += kCopyDims) {
+        double v[kCopyDims];
+#pragma unroll
+        for (unsigned k = 0; k < kCopyDims; ++k)
+            if (d + k < dim)
+                v[k] = src[(long long)(d + k) * N + c];
+#pragma unroll
+        for (unsigned k = 0; k < kCopyDims; ++k)
+            if (d + k < dim)
+                dst[(long long)(d + k) * N + i] = v[k];
+    }
 }
 
 static __global__ void k_math_eval(int fn, long long n, const double *in,
@@ -216,6 +119,117 @@ namespace {
 size_t generic_resample_bytes(long long N)
 {
     return resample_workspace_bytes(N) + align256((size_t)N * 4);
+}
+
+} // namespace
+
+namespace {
+
+// Sums (and for kWAdd the normalisation) of one call; the result in `h`.
+template <int Kind>
+cudaError_t weight_call(uint64_t N, double *lw, double *w, const double *inc,
+                        cudaStream_t s, WeightCtl &h, const char *&what)
+{
+    CallScratch cs(s);
+    const long long nt = ((long long)N + kTile - 1) / kTile;
+    what = ": scratch";
+    // device memory: the result when no pinned slot is free, the joined
+    // sums and the tiles'
+    WeightCtl *out = static_cast<WeightCtl *>(cs.slot());
+    WeightCtl *ctl = nullptr;
+    WAcc *tiles = nullptr;
+    const bool cluster = nt <= kWcTiles;
+    cudaError_t e;
+    if (out == nullptr || !cluster) {
+        void *p = nullptr;
+        e = cs.alloc(2 * align256(sizeof(WeightCtl)) +
+                         sizeof(WAcc) * (size_t)nt,
+                     &p);
+        if (e != cudaSuccess)
+            return e;
+        char *q = static_cast<char *>(p);
+        if (out == nullptr)
+            out = reinterpret_cast<WeightCtl *>(q);
+        ctl = reinterpret_cast<WeightCtl *>(q + align256(sizeof(WeightCtl)));
+        tiles =
+            reinterpret_cast<WAcc *>(q + 2 * align256(sizeof(WeightCtl)));
+    }
+    what = "";
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at[1];
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    if (cluster) {
+        int ctas = 1;
+        while (ctas < nt && ctas < kWcCtas)
+            ctas *= 2;
+        if (ctas > 8)
+            cudaFuncSetAttribute(
+                k_weight_cluster<Kind>,
+                cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        c.gridDim = dim3((unsigned)ctas);
+        c.blockDim = dim3(kThreads);
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)ctas;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        e = cudaLaunchKernelEx(&c, k_weight_cluster<Kind>, (long long)N, lw,
+                               w, inc, out);
+    } else {
+        k_weight_tiles<Kind><<<(unsigned)nt, kThreads, 0, s>>>(
+            (long long)N, lw, static_cast<const double *>(w), inc, tiles);
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        c.gridDim = dim3(1);
+        c.blockDim = dim3(kSpineThreads);
+        e = cudaLaunchKernelEx(&c, k_weight_join,
+                               static_cast<const WAcc *>(tiles), (int)nt, ctl,
+                               out);
+        if (e == cudaSuccess && Kind == kWAdd) {
+            c.gridDim = dim3(
+                (unsigned)(((long long)N + 4 * kThreads - 1) / (4 * kThreads)));
+            c.blockDim = dim3(kThreads);
+            e = cudaLaunchKernelEx(&c, k_weight_apply, (long long)N, lw, w,
+                                   static_cast<const WeightCtl *>(ctl));
+        }
+    }
+    if (e == cudaSuccess)
+        e = cudaGetLastError();
+    if (e == cudaSuccess && cs.slot() == nullptr)
+        e = cudaMemcpyAsync(&h, out, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && cs.slot() != nullptr)
+        std::memcpy(&h, cs.slot(), sizeof(h));
+    return e;
+}
+
+template <int Kind>
+int prospective(uint64_t N, const double *lw, const double *w,
+                const double *inc, double *out, void *stream,
+                const char *where)
+{
+    WeightCtl h;
+    const char *what = "";
+    const cudaError_t e = weight_call<Kind>(
+        N, const_cast<double *>(lw), const_cast<double *>(w), inc,
+        static_cast<cudaStream_t>(stream), h, what); // (read only)
+    if (e != cudaSuccess)
+        return cuda_status(e, where);
+    *out = h.S1 * h.S1 / h.S2;
+    // the log form needs a finite maximum and a positive sum; the plain
+    // forms only finite sums (increments may be negative) and S2 > 0
+    const bool bad = Kind == kWEssLog
+                         ? h.error != 0
+                         : !(h.S1 == h.S1 && h.S1 > -INFINITY &&
+                             h.S1 < INFINITY && h.S2 < INFINITY);
+    if (bad || !(h.S2 > 0.0)) {
+        set_last_error(std::string(where) + ": degenerate weights");
+        *out = NAN;
+        return VSMC_CUDA_EDEGENERATE;
+    }
+    return VSMC_CUDA_OK;
 }
 
 } // namespace
@@ -297,27 +311,13 @@ int vsmc_cuda_weight_add_log(uint64_t N, double *lw, double *w,
         set_last_error("vsmc_cuda_weight_add_log: invalid arguments");
         return VSMC_CUDA_EINVAL;
     }
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int nt = (int)((N + kTile - 1) / kTile);
-    void *scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(
-        &scratch, align256(sizeof(WeightCtl)) + sizeof(LseAcc) * nt, s);
-    if (e != cudaSuccess)
-        return cuda_status(e, "vsmc_cuda_weight_add_log: scratch");
-    WeightCtl *ctl = static_cast<WeightCtl *>(scratch);
-    LseAcc *tiles = reinterpret_cast<LseAcc *>(
-        static_cast<char *>(scratch) + align256(sizeof(WeightCtl)));
-    k_wadd_tiles<<<nt, kThreads, 0, s>>>((long long)N, lw, inc, tiles);
-    k_wadd_reduce<<<1, kSpineThreads, 0, s>>>(tiles, nt, ctl);
-    k_wadd_apply<<<(unsigned)((N + 255) / 256), 256, 0, s>>>((long long)N, lw,
-                                                             w, ctl);
     WeightCtl h;
-    e = cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(scratch, s);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(s);
+    const char *what = "";
+    const cudaError_t e = weight_call<kWAdd>(
+        N, lw, w, inc, static_cast<cudaStream_t>(stream), h, what);
     if (e != cudaSuccess)
-        return cuda_status(e, "vsmc_cuda_weight_add_log");
+        return cuda_status(
+            e, (std::string("vsmc_cuda_weight_add_log") + what).c_str());
     if (h.error) {
         set_last_error("vsmc_cuda_weight_add_log: degenerate log-weights");
         *ess = NAN;
@@ -326,48 +326,6 @@ int vsmc_cuda_weight_add_log(uint64_t N, double *lw, double *w,
     *ess = h.S1 * h.S1 / h.S2;
     return VSMC_CUDA_OK;
 }
-
-namespace {
-
-int prospective(uint64_t N, const double *lw, const double *w,
-                const double *inc, int kind, double *out, void *stream,
-                const char *where)
-{
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int nt = (int)((N + kTile - 1) / kTile);
-    void *scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(
-        &scratch, align256(sizeof(WeightCtl)) + sizeof(LseAcc) * nt, s);
-    if (e != cudaSuccess)
-        return cuda_status(e, where);
-    WeightCtl *ctl = static_cast<WeightCtl *>(scratch);
-    LseAcc *tiles = reinterpret_cast<LseAcc *>(
-        static_cast<char *>(scratch) + align256(sizeof(WeightCtl)));
-    k_prospective_tiles<<<nt, kThreads, 0, s>>>((long long)N, lw, w, inc,
-                                                kind, tiles);
-    k_wadd_reduce<<<1, kSpineThreads, 0, s>>>(tiles, nt, ctl);
-    WeightCtl h;
-    e = cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(scratch, s);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess)
-        return cuda_status(e, where);
-    *out = h.S1 * h.S1 / h.S2;
-    // the log form needs a finite maximum and a positive sum; the plain
-    // forms only finite sums (increments may be negative) and S2 > 0
-    const bool bad = kind == 0 ? h.error != 0
-                               : !(h.S1 == h.S1 && h.S1 > -INFINITY &&
-                                   h.S1 < INFINITY && h.S2 < INFINITY);
-    if (bad || !(h.S2 > 0.0)) {
-        set_last_error(std::string(where) + ": degenerate weights");
-        *out = NAN;
-        return VSMC_CUDA_EDEGENERATE;
-    }
-    return VSMC_CUDA_OK;
-}
-
-} // namespace
 
 int vsmc_cuda_weight_ess(uint64_t N, const double *log_weight,
                          const double *weight, const double *inc, int use_log,
@@ -378,8 +336,10 @@ int vsmc_cuda_weight_ess(uint64_t N, const double *log_weight,
         set_last_error("vsmc_cuda_weight_ess: invalid arguments");
         return VSMC_CUDA_EINVAL;
     }
-    return prospective(N, log_weight, weight, inc, use_log ? 0 : 1, ess,
-                       stream, "vsmc_cuda_weight_ess");
+    return use_log ? prospective<kWEssLog>(N, log_weight, weight, inc, ess,
+                                           stream, "vsmc_cuda_weight_ess")
+                   : prospective<kWEssLinear>(N, log_weight, weight, inc, ess,
+                                              stream, "vsmc_cuda_weight_ess");
 }
 
 int vsmc_cuda_weight_cess(uint64_t N, const double *weight, const double *inc,
@@ -389,8 +349,11 @@ int vsmc_cuda_weight_cess(uint64_t N, const double *weight, const double *inc,
         set_last_error("vsmc_cuda_weight_cess: invalid arguments");
         return VSMC_CUDA_EINVAL;
     }
-    return prospective(N, nullptr, weight, inc, use_log ? 2 : 3, cess, stream,
-                       "vsmc_cuda_weight_cess");
+    return use_log ? prospective<kWCessLog>(N, nullptr, weight, inc, cess,
+                                            stream, "vsmc_cuda_weight_cess")
+                   : prospective<kWCessLinear>(N, nullptr, weight, inc, cess,
+                                               stream,
+                                               "vsmc_cuda_weight_cess");
 }
 
 size_t vsmc_cuda_resample_workspace_size(uint64_t N)

@@ -172,94 +172,4 @@ __device__ __forceinline__ T block_excl_scan(T v, T *sh, T &total)
     return wexcl + inc - v;
 }
 
-// Online log-sum-exp accumulator: m = running max, s1 = sum exp(lw - m),
-// s2 = sum exp(2 (lw - m)), sx/sy = sum exp(lw - m) * (x, y).
-struct LseAcc {
-    double m, s1, s2, sx, sy;
-
-    __device__ __forceinline__ void init()
-    {
-        m = -INFINITY;
-        s1 = s2 = sx = sy = 0.0;
-    }
-
-    __device__ __forceinline__ void rescale_to(double nm)
-    {
-        if (nm == m)
-            return;
-        const double f = (m == -INFINITY) ? 0.0 : exp(m - nm);
-        s1 *= f;
-        s2 *= f * f;
-        sx *= f;
-        sy *= f;
-        m = nm;
-    }
-
-    __device__ __forceinline__ void add(double lw, double x, double y)
-    {
-        if (!(lw <= m)) { // new max (or NaN: propagate below)
-            if (lw != lw) {
-                s1 = lw;
-                return;
-            }
-            rescale_to(lw);
-        }
-        if (lw == -INFINITY)
-            return;
-        const double e = exp(lw - m);
-        s1 += e;
-        s2 += e * e;
-        sx += e * x;
-        sy += e * y;
-    }
-
-    __device__ __forceinline__ void merge(const LseAcc &o)
-    {
-        if (o.m == -INFINITY && o.s1 == 0.0)
-            return;
-        const double nm = fmax(m, o.m);
-        const double fa = (m == -INFINITY) ? 0.0 : exp(m - nm);
-        const double fb = (o.m == -INFINITY) ? 0.0 : exp(o.m - nm);
-        s1 = s1 * fa + o.s1 * fb;
-        s2 = s2 * fa * fa + o.s2 * fb * fb;
-        sx = sx * fa + o.sx * fb;
-        sy = sy * fa + o.sy * fb;
-        m = nm;
-    }
-};
-
-__device__ __forceinline__ LseAcc shfl_xor(const LseAcc &a, int o)
-{
-    LseAcc b;
-    b.m = __shfl_xor_sync(0xffffffffu, a.m, o);
-    b.s1 = __shfl_xor_sync(0xffffffffu, a.s1, o);
-    b.s2 = __shfl_xor_sync(0xffffffffu, a.s2, o);
-    b.sx = __shfl_xor_sync(0xffffffffu, a.sx, o);
-    b.sy = __shfl_xor_sync(0xffffffffu, a.sy, o);
-    return b;
-}
-
-// Deterministic block reduction of LseAcc (fixed shuffle tree, fixed warp
-// order), result valid in thread 0.
-__device__ __forceinline__ LseAcc block_reduce_lse(LseAcc a, LseAcc *sh)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        a.merge(shfl_xor(a, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-        sh[wid] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        LseAcc r = sh[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            r.merge(sh[w]);
-        sh[0] = r;
-    }
-    __syncthreads();
-    LseAcc r = sh[0];
-    __syncthreads();
-    return r;
-}
-
 } // namespace vsmc_b200
