@@ -232,6 +232,25 @@ int prospective(uint64_t N, const double *lw, const double *w,
     return VSMC_CUDA_OK;
 }
 
+// A resampling call's result once its stream is done: in the slot already
+// (`done`), or copied from the workspace's control block.
+static_assert(sizeof(ResampleCtl) <= kSlotBytes, "result fits a slot");
+cudaError_t resample_result(const ResampleWorkspace &ws, ResampleCtl *slot,
+                            bool done, cudaStream_t s, ResampleCtl &h)
+{
+    cudaError_t e = cudaSuccess;
+    if (!done)
+        e = cudaMemcpyAsync(slot != nullptr ? slot : &h, ws.ctl, sizeof(h),
+                            cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && slot != nullptr) {
+        h.error = slot->error;
+        h.offset = slot->offset;
+    }
+    return e;
+}
+
 } // namespace
 
 extern "C" {
@@ -389,10 +408,8 @@ int vsmc_cuda_resample(int scheme, uint64_t N, const double *weight,
     std::memset(&h, 0, sizeof(h));
     h.active = 1;
     h.offset = rng->offset;
-    cudaError_t e =
-        cudaMemcpyAsync(ws.ctl, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess)
-        return cuda_status(e, "vsmc_cuda_resample: control block");
+    CallScratch cs(s);
+    ResampleCtl *slot = static_cast<ResampleCtl *>(cs.slot());
     EngineRef eng;
     for (int i = 0; i < 4; ++i) {
         eng.key.v[i] = rng->key[i];
@@ -400,14 +417,13 @@ int vsmc_cuda_resample(int scheme, uint64_t N, const double *weight,
     }
     WeightsGiven w;
     w.w = weight;
-    launch_resample(scheme, w, (long long)N, eng, ws, uniforms,
-                    (long long)n_uniforms, replication, cf, s);
-    e = cudaGetLastError();
+    const bool done =
+        launch_resample(scheme, w, (long long)N, eng, ws, h, slot, uniforms,
+                        (long long)n_uniforms, replication, cf, s);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample: launch");
-    e = cudaMemcpyAsync(&h, ws.ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(s);
+    e = resample_result(ws, slot, done, s, h);
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample");
     if (h.error != 0) {
@@ -476,9 +492,8 @@ int vsmc_cuda_resample_mn(int scheme, uint64_t M, uint64_t N,
     h.active = 1;
     h.offset = rng->offset;
     h.Nout = (long long)N;
-    e = cudaMemcpyAsync(ws.ctl, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess)
-        return cuda_status(e, "vsmc_cuda_resample_mn: control block");
+    CallScratch cs(s);
+    ResampleCtl *slot = static_cast<ResampleCtl *>(cs.slot());
     EngineRef eng;
     for (int i = 0; i < 4; ++i) {
         eng.key.v[i] = rng->key[i];
@@ -486,17 +501,16 @@ int vsmc_cuda_resample_mn(int scheme, uint64_t M, uint64_t N,
     }
     WeightsGiven w;
     w.w = weight;
-    launch_resample(scheme, w, (long long)M, eng, ws, uniforms,
-                    (long long)n_uniforms, rep, cf_scratch, s,
-                    /*cfrp=*/false, (long long)N);
+    const bool done =
+        launch_resample(scheme, w, (long long)M, eng, ws, h, slot, uniforms,
+                        (long long)n_uniforms, rep, cf_scratch, s,
+                        /*cfrp=*/false);
     if (copy_from != nullptr)
         launch_expand(rep, (long long)M, (long long)N, ws, copy_from, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_mn: launch");
-    e = cudaMemcpyAsync(&h, ws.ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(s);
+    e = resample_result(ws, slot, done, s, h);
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_mn");
     if (h.error != 0) {

@@ -122,6 +122,11 @@ struct RcArgs {
     int nt;           // their tiles
     int cfrp;         // copy_from too (0: the counts only)
     ResampleCtl *ctl;
+    // given weights: the call's engine position and number of children (0:
+    // as many as weights), and where its error and new position go
+    unsigned long long offset;
+    long long Nout;
+    ResampleCtl *out;
     EngineRef eng;
     double *u;        // the U01 sequence and its bins
     int32_t *bins;
@@ -621,23 +626,26 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     const bool act = tile < nt;
     const long long base = (long long)tile * kTile;
     const long long i0 = base + (long long)gtid * R;
-    const long long Nout = resample_children(a.ctl, N);
+    constexpr bool Given = std::is_same<W, WeightsGiven>::value;
+    const long long Nout = Given && a.Nout > 0 ? a.Nout : N;
     const double Nd = (double)Nout;
     wsrc.prepare();
     if (threadIdx.x == 0) {
-        const ResampleCtl *c = a.ctl;
-        sm.offset = c->offset;
+        sm.offset = Given ? a.offset : a.ctl->offset;
         if (!Residual) {
             sm.NN = Nout;
             sm.delta = __ddiv_rn(1.0, Nd);
             sm.kbits = bin_kbits(Nout);
             sm.u0 = Sys ? __dmul_rn(canonical_u64(threefry_word(
-                                        a.eng.key, a.eng.ctr, c->offset)),
+                                        a.eng.key, a.eng.ctr, sm.offset)),
                                     sm.delta)
                         : 0.0;
         }
-        if (rank == 0)
+        if (rank == 0) {
             a.ctl->words = Sys ? 1 : 0;
+            if (Given)
+                a.ctl->error = 0;
+        }
     }
     __syncthreads();
 
@@ -1199,8 +1207,16 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             rc_store(a.rep_out, i0, N, rep);
     }
     cl.sync();
-    if (rank == 0 && threadIdx.x == 0)
-        a.ctl->offset += *(volatile unsigned long long *)&a.ctl->words;
+    // the engine position (the words are final)
+    if (rank == 0 && threadIdx.x == 0) {
+        const unsigned long long off =
+            sm.offset + *(volatile unsigned long long *)&a.ctl->words;
+        a.ctl->offset = off;
+        if (Given) {
+            a.out->offset = off;
+            a.out->error = 0;
+        }
+    }
     if (!a.cfrp)
         return;
 
@@ -1307,6 +1323,8 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         rc_store(a.copy_from, i0, N, cf);
     }
     cl.sync(); // no CTA leaves while another reads its shared memory
+    if (Given && rank == 0 && threadIdx.x == 0)
+        a.out->error = *(volatile int *)&a.ctl->error;
 }
 
 template <typename W, bool Residual, int U, int R>
@@ -1522,6 +1540,9 @@ inline RcArgs rc_args(long long N, const EngineRef &eng,
     a.nt = resample_ntiles(N);
     a.cfrp = cfrp ? 1 : 0;
     a.ctl = ws.ctl;
+    a.offset = 0;
+    a.Nout = 0;
+    a.out = ws.ctl;
     a.eng = eng;
     a.u = ws.u;
     a.bins = ws.bins;
@@ -1533,30 +1554,46 @@ inline RcArgs rc_args(long long N, const EngineRef &eng,
 
 // A resampling of given weights: one cluster where it fits, the launch
 // sequence of resample.cuh otherwise (and for caller-supplied uniforms).
-inline void launch_resample(int scheme, WeightsGiven w, long long N,
+// `h` holds the call's initial control block; `slot` is a call's pinned
+// memory, or nullptr.  Returns whether the result is in *slot (else in the
+// workspace's control block) once the stream gets there.
+inline bool launch_resample(int scheme, WeightsGiven w, long long N,
                             const EngineRef &eng, ResampleWorkspace &ws,
+                            const ResampleCtl &h, ResampleCtl *slot,
                             const double *u_given, long long n_given,
                             int32_t *rep_out, int32_t *copy_from,
-                            cudaStream_t s, bool cfrp = true,
-                            long long Nout = 0)
+                            cudaStream_t s, bool cfrp = true)
 {
-    if (u_given != nullptr || !rc_fits(N, Nout)) {
-        launch_resample_core(scheme, w, N, eng, ws, u_given, n_given, false,
-                             rep_out, copy_from, s, false, cfrp, Nout);
-        return;
+    if (u_given != nullptr || !rc_fits(N, h.Nout)) {
+        const ResampleCtl *src = &h;
+        if (slot != nullptr) { // (pinned: copied without staging)
+            *slot = h;
+            src = slot;
+        }
+        // a failed copy leaves its error for the caller's check
+        if (cudaMemcpyAsync(ws.ctl, src, sizeof(h), cudaMemcpyHostToDevice,
+                            s) == cudaSuccess)
+            launch_resample_core(scheme, w, N, eng, ws, u_given, n_given,
+                                 false, rep_out, copy_from, s, false, cfrp,
+                                 h.Nout);
+        return false;
     }
-    const RcArgs a = rc_args(N, eng, ws, rep_out, copy_from, cfrp);
-    const RcShape sh = rc_shape(resample_ntiles(Nout > N ? Nout : N));
+    RcArgs a = rc_args(N, eng, ws, rep_out, copy_from, cfrp);
+    a.offset = h.offset;
+    a.Nout = h.Nout;
+    a.out = slot != nullptr ? slot : ws.ctl;
+    const RcShape sh = rc_shape(resample_ntiles(h.Nout > N ? h.Nout : N));
     rc_scheme(scheme, [&](auto res, auto seq) {
         constexpr bool Re = decltype(res)::value;
         constexpr int U = decltype(seq)::value;
         if (sh.r == 8)
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, false, s,
-                      w, a);
+            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, false,
+                      s, w, a);
         else
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, false, s,
-                      w, a);
+            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, false,
+                      s, w, a);
     });
+    return slot != nullptr;
 }
 
 // A filter step after its tile statistics: the finalisation (fa) and the

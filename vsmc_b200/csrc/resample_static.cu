@@ -148,10 +148,6 @@ extern "C" int vsmc_cuda_resample_noalloc(int scheme, uint64_t N,
     std::memset(&h, 0, sizeof(h));
     h.active = 1;
     h.offset = rng->offset;
-    cudaError_t e =
-        cudaMemcpyAsync(ws.ctl, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess)
-        return cuda_status(e, "vsmc_cuda_resample_noalloc: control block");
     EngineRef eng;
     for (int i = 0; i < 4; ++i) {
         eng.key.v[i] = rng->key[i];
@@ -159,9 +155,9 @@ extern "C" int vsmc_cuda_resample_noalloc(int scheme, uint64_t N,
     }
     WeightsGiven w;
     w.w = weight;
-    launch_resample(scheme, w, (long long)N, eng, ws, uniforms,
+    launch_resample(scheme, w, (long long)N, eng, ws, h, nullptr, uniforms,
                     (long long)n_uniforms, replication, cf, s);
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_noalloc: launch");
     e = cudaMemcpyAsync(&h, ws.ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
