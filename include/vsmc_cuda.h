@@ -686,8 +686,8 @@ typedef struct {
     int form;         /* VSMC_CUDA_FP64, or VSMC_CUDA_MIXED: each data
                          point's mixture density in float, the per-particle
                          sum of log terms in double */
-    int group;        /* lanes per particle (1, 2, 4, 8, 16); 0 = pick the
-                         fastest at initialize (results do not depend on it) */
+    int group;        /* lanes per particle (1, 2, 4, 8, 16); 0 = chosen from
+                         N and the data (results do not depend on it) */
 } vsmc_cuda_gmm_config;
 
 /* N 2^16, iters 100, power 4, sweeps 5, sd 0.1, Systematic, threshold 0.5,
@@ -728,7 +728,7 @@ int vsmc_cuda_gmm_read_params(vsmc_cuda_gmm *g, double *params, double *lw,
  * doubles), for precision comparisons.  Synchronises. */
 int vsmc_cuda_gmm_loglik(vsmc_cuda_gmm *g, int form, double *out);
 
-/* Lanes per particle in use (the autotuned value when group was 0). */
+/* Lanes per particle in use (the chosen value when group was 0). */
 int vsmc_cuda_gmm_group(vsmc_cuda_gmm *g, int *group);
 
 /* CUDA-event timing of the MCMC kernels (as vsmc_cuda_cv_set_timing). */

@@ -26,14 +26,22 @@
 //                    loop split over the group; per-CTA acceptance counts
 //   k_gmm_path       acceptance totals, path integrand, trapezoid rule
 //
-// Forms: FP64 evaluates the likelihood in double throughout (the reference
-// arithmetic, one rounding per operation in the reference's order); MIXED
+// Forms: FP64 evaluates the likelihood in double throughout (ll_density:
+// densities by a table-driven 2^t, one logarithm per particle); MIXED
 // evaluates each data point's mixture density in float (exp2 / log2 on the
 // special-function units, one log2 per pair of points) and accumulates the
 // log terms of a particle in double.  Everything else is double in both.
+//
+// The MCMC kernel at 65536 particles, 1000 points, 5 sweeps (one B200, ms a
+// step, first -> now): FP64 11.8 -> 4.5 (the reference's order of operations
+// with exp() and a log() a point took 125 FP64 operations a point, now 45;
+// bound by the FP64 pipe, 60% on average, 70% on the SMs with 16 warps),
+// mixed 2.4 -> 1.73 (no bounds test in whole rounds; bound by the
+// special-function unit, 72%).
 #include "cv_kernels.cuh"
 #include "resample_cluster.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -71,10 +79,19 @@ struct GmmArgs {
     int n;
     long long N;
     double mu0, sd0, shape0, scale0;
+    double xmin, xmax; // of the data
     double alpha, sd;
     int sweeps;
     uint32_t seed_base; // Seed after Seed::set(seed), before any get()
     long long *tile_acc; // per CTA: 3 * sweeps acceptance counts
+};
+
+// The data as the likelihood reads them: staged in shared memory, with (FP64)
+// their range and the lane's copy of the 2^(j/256) table.
+struct GmmData {
+    const void *x;
+    const double *tab;
+    double xmin, xmax;
 };
 
 struct GmmState {
@@ -244,69 +261,203 @@ __device__ __forceinline__ float mix_density(float x, const float *m,
 // lane adds those subtrees pairwise.  G only changes the speed.
 constexpr int kLlClasses = 16;
 
-template <int G, bool F32>
-__device__ __forceinline__ double gmm_loglik(const GmmState &s,
-                                             const void *data, int n, int g,
-                                             unsigned mask)
+// FP64 form: the mixture densities by a table-driven 2^t of few operations
+// and one logarithm per particle instead of one per point.
+//
+// A component's density at x is W 2^t with W = w sqrt(lambda) and t = -B r^2,
+// B = lambda log2(e) / 2, r = x - mu.  t is rounded to the nearest 1/256 by
+// the 1.5 2^44 constant (one FMA), f = t minus that is one more FMA on the
+// exact product, 2^f - 1 = f (c1 + f (c2 + f (c3 + f c4))) on |f| <= 2^-9
+// (the Taylor series, its f^5 term economised by Chebyshev's T5: error
+// 2.4e-18), and 2^(j/256) comes from a table in shared memory with one copy
+// per bank pair, so that a warp's random rows meet no bank conflict.  11
+// FP64 operations a component and point; exp() and the reference's order
+// of operations took about 23.
+//
+// log-likelihood = sum log p_i = log prod p_i: each class multiplies its
+// points' densities (>= 1e-13), moving the exponent into an integer every
+// kLlRenorm points; the classes' products are multiplied in a balanced tree
+// and one logarithm is taken.  A product's rounding errors (2^-53 relative
+// each) are far below those of adding a thousand logarithms to a sum of
+// thousands.  Bound: the FP64 pipe (45 operations a point).
+constexpr int kLlTab = 256;     // table entries, 2^(j/256)
+constexpr int kLlCopies = 16;   // one per pair of banks
+constexpr int kLlRenorm = 8;
+constexpr int kLlChunk = 4;  // classes a lane multiplies at a time
+constexpr int kLlPoints = 4; // points evaluated together
+constexpr size_t kLlTabBytes = (size_t)kLlTab * kLlCopies * sizeof(double);
+
+struct LlPoint {
+    double mu[kGmmK], B[kGmmK], W[kGmmK];
+};
+
+// The density of one point (plus the reference's 1e-13 floor).  tab: the
+// lane's copy of the table, whose entry j has j << 12 taken off its high
+// word: adding n << 12 for n = 256 k + j then gives 2^k 2^(j/256) in one
+// integer operation.
+template <int M>
+__device__ __forceinline__ void ll_density(const double (&x)[M],
+                                           const LlPoint &q,
+                                           const double *tab, double (&p)[M])
+{
+    constexpr double kRound = 0x1.8p44;
+    constexpr double ln2 = 0.69314718055994530942;
+    constexpr double c5 = ln2 * ln2 * ln2 * ln2 * ln2 / 120.0;
+    constexpr double c1 = ln2 - c5 * 0.3125 * 0x1p-36;
+    constexpr double c2 = ln2 * ln2 / 2.0;
+    constexpr double c3 = ln2 * ln2 * ln2 / 6.0 + c5 * 1.25 * 0x1p-18;
+    constexpr double c4 = ln2 * ln2 * ln2 * ln2 / 24.0;
+    constexpr int K = kGmmK;
+    double r[M][K], b[M][K], u[M][K], t[M][K], h[M][K];
+    // stage by stage over the M points' components: 4 M independent chains
+#define VSMC_LL_EACH                                                          \
+    _Pragma("unroll") for (int m = 0; m < M; ++m)                             \
+        _Pragma("unroll") for (int d = 0; d < K; ++d)
+    VSMC_LL_EACH r[m][d] = __dsub_rn(x[m], q.mu[d]);
+    VSMC_LL_EACH b[m][d] = __dmul_rn(q.B[d], r[m][d]);
+    VSMC_LL_EACH u[m][d] = __fma_rn(-b[m][d], r[m][d], kRound);
+    VSMC_LL_EACH
+    {
+        // (2^-1000 and below add nothing to 1e-13)
+        const int n = max(__double2loint(u[m][d]), -1000 * kLlTab);
+        const double t0 = tab[(n & (kLlTab - 1)) * kLlCopies];
+        t[m][d] = __hiloint2double(__double2hiint(t0) + n * (1 << 12),
+                                   __double2loint(t0));
+    }
+    VSMC_LL_EACH u[m][d] = __dadd_rn(u[m][d], -kRound);
+    VSMC_LL_EACH r[m][d] = __fma_rn(-b[m][d], r[m][d], -u[m][d]); // f
+    VSMC_LL_EACH h[m][d] = __fma_rn(r[m][d], c4, c3);
+    VSMC_LL_EACH h[m][d] = __fma_rn(r[m][d], h[m][d], c2);
+    VSMC_LL_EACH h[m][d] = __fma_rn(r[m][d], h[m][d], c1);
+    VSMC_LL_EACH h[m][d] = __dmul_rn(r[m][d], h[m][d]);
+    VSMC_LL_EACH h[m][d] = __fma_rn(t[m][d], h[m][d], t[m][d]);
+#undef VSMC_LL_EACH
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+        p[m] = 1e-13;
+#pragma unroll
+    for (int d = 0; d < K; ++d)
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            p[m] = __fma_rn(q.W[d], h[m][d], p[m]);
+}
+
+template <int G>
+__device__ __forceinline__ double
+ll_product(const LlPoint &q, const double *x, int n, int g, unsigned mask,
+           const double *tab)
+{
+    // kLlChunk of the lane's classes at a time (their subtrees of the
+    // product tree, kept in T)
+    constexpr int J = kLlClasses / G;
+    constexpr int C = J < kLlChunk ? J : kLlChunk;
+    double T[J / C];
+    int E = 0;
+#pragma unroll 1
+    for (int c = 0; c < J / C; ++c) {
+        double P[C];
+#pragma unroll
+        for (int j = 0; j < C; ++j)
+            P[j] = 1.0;
+        const auto renorm = [&]() {
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+                const int hi = __double2hiint(P[j]);
+                E += (hi >> 20) - 1023;
+                P[j] = __hiloint2double((hi & 0xfffff) | 0x3ff00000,
+                                        __double2loint(P[j]));
+            }
+        };
+        const double *xc = x + g + c * C * G;
+        int base = 0, since = 0;
+#pragma unroll 1
+        for (; base + kLlClasses <= n; base += kLlClasses) {
+            constexpr int M = C < kLlPoints ? C : kLlPoints;
+#pragma unroll
+            for (int j0 = 0; j0 < C; j0 += M) {
+                double v[M], p[M];
+#pragma unroll
+                for (int m = 0; m < M; ++m)
+                    v[m] = xc[base + (j0 + m) * G];
+                ll_density<M>(v, q, tab, p);
+#pragma unroll
+                for (int m = 0; m < M; ++m)
+                    P[j0 + m] = __dmul_rn(P[j0 + m], p[m]);
+            }
+            if (++since == kLlRenorm) {
+                since = 0;
+                renorm();
+            }
+        }
+        // the last, incomplete round
+#pragma unroll 1
+        for (int i = base + g + c * C * G, k = 0; k < C && i < n;
+             i += G, ++k) {
+            const double v[1] = {x[i]};
+            double p[1];
+            ll_density<1>(v, q, tab, p);
+#pragma unroll
+            for (int j = 0; j < C; ++j)
+                if (j == k)
+                    P[j] = __dmul_rn(P[j], p[0]);
+        }
+        renorm();
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < C; ++j)
+                P[j] = __dmul_rn(P[j], __shfl_xor_sync(mask, P[j], o));
+#pragma unroll
+        for (int w = 1; w < C; w <<= 1)
+#pragma unroll
+            for (int j = 0; j + w < C; j += 2 * w)
+                P[j] = __dmul_rn(P[j], P[j + w]);
+        T[c] = P[0];
+    }
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1)
+        E += __shfl_xor_sync(mask, E, o);
+#pragma unroll
+    for (int w = 1; w < J / C; w <<= 1)
+#pragma unroll
+        for (int c = 0; c + w < J / C; c += 2 * w)
+            T[c] = __dmul_rn(T[c], T[c + w]);
+    const double e = (double)E;
+    return __fma_rn(e, fm::kLn2Hi, __fma_rn(e, fm::kLn2Lo, mh_log(T[0])));
+}
+
+// The values of one likelihood; false when a component lies outside what
+// ll_density is made for (t below -2^22, where its integer would wrap, or
+// a W that could overflow a class's product): then the reference's own
+// operations evaluate it.
+__device__ __forceinline__ bool ll_prepare(const GmmState &s, double xmin,
+                                           double xmax, LlPoint &q)
+{
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < kGmmK; ++d) {
+        const double r = fmax(fabs(xmin - s.mu[d]), fabs(xmax - s.mu[d]));
+        q.mu[d] = s.mu[d];
+        q.B[d] = __dmul_rn(s.lam[d], 0.72134752044448170368); // log2(e) / 2
+        q.W[d] = __dmul_rn(s.w[d], mh_sqrt(s.lam[d]));
+        const double t = q.B[d] * r * r;
+        ok = ok && t < 0x1p22 && s.lam[d] > 0.0 && q.W[d] >= 0.0 &&
+             q.W[d] < 0x1p90;
+    }
+    return ok;
+}
+
+// The parameters of a likelihood outside ll_prepare's range.
+struct LlGeneral {
+    double mu[kGmmK], lam[kGmmK], loglam[kGmmK], w[kGmmK];
+};
+
+// The class sums acc[] of a group's lanes added in the fixed order.
+template <int G>
+__device__ __forceinline__ double ll_join(double (&acc)[kLlClasses / G],
+                                          unsigned mask)
 {
     constexpr int J = kLlClasses / G;
-    double acc[J];
-#pragma unroll
-    for (int j = 0; j < J; ++j)
-        acc[j] = 0.0;
-    if (F32) {
-        // w_d exp(0.5 log lambda_d - 0.5 lambda_d r^2) = exp2(A_d - B_d r^2)
-        constexpr double kLog2e = 1.4426950408889634074;
-        float m[kGmmK], A[kGmmK], B[kGmmK];
-#pragma unroll
-        for (int d = 0; d < kGmmK; ++d) {
-            m[d] = (float)s.mu[d];
-            A[d] = (float)(log2(s.w[d]) + 0.5 * s.loglam[d] * kLog2e);
-            B[d] = (float)(0.5 * s.lam[d] * kLog2e);
-        }
-        // Points i and i + 16 of a class share one log: log2 of the
-        // product of their densities (each >= 1e-13, so the product stays
-        // a normal float); the class adds these pair terms in double.
-        const float *x = static_cast<const float *>(data);
-        for (int base = 0; base < n; base += 2 * kLlClasses) {
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                const int i = base + g + j * G;
-                if (i < n) {
-                    float p = mix_density(x[i], m, A, B);
-                    if (i + kLlClasses < n)
-                        p = __fmul_rn(p, mix_density(x[i + kLlClasses], m, A, B));
-                    acc[j] = __dadd_rn(acc[j], (double)sfu_lg2(p));
-                }
-            }
-        }
-    } else {
-        const double *x = static_cast<const double *>(data);
-        double c[kGmmK], h[kGmmK];
-#pragma unroll
-        for (int d = 0; d < kGmmK; ++d) {
-            c[d] = __dmul_rn(0.5, s.loglam[d]);
-            h[d] = __dmul_rn(0.5, s.lam[d]);
-        }
-        for (int base = 0; base < n; base += kLlClasses) {
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                const int i = base + g + j * G;
-                if (i < n) {
-                    // lli += w_d exp(0.5 log lambda_d - 0.5 lambda_d r r)
-                    double lli = 0.0;
-#pragma unroll
-                    for (int d = 0; d < kGmmK; ++d) {
-                        const double r = __dsub_rn(x[i], s.mu[d]);
-                        const double t = __dmul_rn(__dmul_rn(h[d], r), r);
-                        const double e = exp(__dsub_rn(c[d], t));
-                        lli = __dadd_rn(lli, __dmul_rn(s.w[d], e));
-                    }
-                    acc[j] = __dadd_rn(acc[j], log(__dadd_rn(lli, 1e-13)));
-                }
-            }
-        }
-    }
 #pragma unroll
     for (int j = 0; j < J; ++j)
 #pragma unroll
@@ -317,7 +468,110 @@ __device__ __forceinline__ double gmm_loglik(const GmmState &s,
 #pragma unroll
         for (int j = 0; j + w < J; j += 2 * w)
             acc[j] = __dadd_rn(acc[j], acc[j + w]);
-    return F32 ? __dmul_rn(acc[0], 0.69314718055994530942) : acc[0];
+    return acc[0];
+}
+
+// The reference's operations one by one (out of line: rarely needed, and
+// inlined its registers would be the hot loop's).
+template <int G>
+__device__ __noinline__ double ll_general(LlGeneral s, const double *x, int n,
+                                          int g, unsigned mask)
+{
+    constexpr int J = kLlClasses / G;
+    double acc[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+        acc[j] = 0.0;
+    for (int base = 0; base < n; base += kLlClasses) {
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int i = base + g + j * G;
+            if (i < n) {
+                // lli += w_d exp(0.5 log lambda_d - 0.5 lambda_d r r)
+                double lli = 0.0;
+#pragma unroll 1
+                for (int d = 0; d < kGmmK; ++d) {
+                    const double r = __dsub_rn(x[i], s.mu[d]);
+                    const double t = __dmul_rn(
+                        __dmul_rn(__dmul_rn(0.5, s.lam[d]), r), r);
+                    const double e = mh_exp(
+                        __dsub_rn(__dmul_rn(0.5, s.loglam[d]), t));
+                    lli = __dadd_rn(lli, __dmul_rn(s.w[d], e));
+                }
+                acc[j] = __dadd_rn(acc[j], mh_log(__dadd_rn(lli, 1e-13)));
+            }
+        }
+    }
+    return ll_join<G>(acc, mask);
+}
+
+template <int G, bool F32>
+__device__ __forceinline__ double gmm_loglik(const GmmState &s,
+                                             const GmmData &data, int n, int g,
+                                             unsigned mask)
+{
+    constexpr int J = kLlClasses / G;
+    if constexpr (!F32) {
+        const double *x = static_cast<const double *>(data.x);
+        LlPoint q;
+        if (ll_prepare(s, data.xmin, data.xmax, q))
+            return ll_product<G>(q, x, n, g, mask, data.tab);
+        LlGeneral a;
+#pragma unroll
+        for (int d = 0; d < kGmmK; ++d) {
+            a.mu[d] = s.mu[d];
+            a.lam[d] = s.lam[d];
+            a.loglam[d] = s.loglam[d];
+            a.w[d] = s.w[d];
+        }
+        return ll_general<G>(a, x, n, g, mask);
+    } else {
+        double acc[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            acc[j] = 0.0;
+        // w_d exp(0.5 log lambda_d - 0.5 lambda_d r^2) = exp2(A_d - B_d r^2)
+        constexpr double kLog2e = 1.4426950408889634074;
+        float m[kGmmK], A[kGmmK], B[kGmmK];
+#pragma unroll
+        for (int d = 0; d < kGmmK; ++d) {
+            m[d] = (float)s.mu[d];
+            A[d] = (float)(log2(s.w[d]) + 0.5 * s.loglam[d] * kLog2e);
+            B[d] = (float)(0.5 * s.lam[d] * kLog2e);
+        }
+        // Points i and i + 16 of a class share one log: log2 of the product of
+        // their densities (each >= 1e-13, so the product stays a normal float);
+        // the class adds these pair terms in double.
+        // Whole rounds of 32 points carry no bounds test, so that the lane's
+        // pairs overlap in the special-function unit.
+        const float *x = static_cast<const float *>(data.x);
+        int base = 0;
+#pragma unroll 1
+        for (; base + 2 * kLlClasses <= n; base += 2 * kLlClasses) {
+            const float *xb = x + base + g;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const float p =
+                    __fmul_rn(mix_density(xb[j * G], m, A, B),
+                              mix_density(xb[j * G + kLlClasses], m, A, B));
+                acc[j] = __dadd_rn(acc[j], (double)sfu_lg2(p));
+            }
+        }
+        if (base < n) {
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const int i = base + g + j * G;
+                if (i < n) {
+                    float p = mix_density(x[i], m, A, B);
+                    if (i + kLlClasses < n)
+                        p = __fmul_rn(p,
+                                      mix_density(x[i + kLlClasses], m, A, B));
+                    acc[j] = __dadd_rn(acc[j], (double)sfu_lg2(p));
+                }
+            }
+        }
+        return __dmul_rn(ll_join<G>(acc, mask), 0.69314718055994530942);
+    }
 }
 
 // gmm_state::log_prior (gmm_state.hpp:67-80)
@@ -341,7 +595,7 @@ __device__ __forceinline__ double gmm_log_prior(const GmmState &s,
 // refreshes log lambda).
 template <int G, bool F32>
 __device__ __forceinline__ void gmm_log_target(GmmState &s, const GmmArgs &a,
-                                               const void *data, int g,
+                                               const GmmData &data, int g,
                                                unsigned mask)
 {
 #pragma unroll
@@ -370,7 +624,7 @@ template <int G, bool F32>
 __device__ __forceinline__ int gmm_move_block(int block, GmmState &s,
                                               ParticleRng &rng,
                                               const GmmArgs &a,
-                                              const void *data, int g,
+                                              const GmmData &data, int g,
                                               unsigned mask)
 {
     const GmmState o = s; // save_old
@@ -468,24 +722,45 @@ __device__ __forceinline__ void store_state(const GmmState &s, GmmBuf &b,
     b.base[13 * N + i] = s.ll;
 }
 
-// Stage the data in shared memory.
+// Stage the data in shared memory, after (FP64) the table's copies.
 template <bool F32>
-__device__ __forceinline__ const void *stage_data(const GmmArgs &a,
-                                                  unsigned char *smem)
+__device__ __forceinline__ GmmData stage_data(const GmmArgs &a,
+                                              unsigned char *smem)
 {
+    GmmData d;
+    d.xmin = a.xmin;
+    d.xmax = a.xmax;
+    d.tab = nullptr;
     if (F32) {
         float *x = reinterpret_cast<float *>(smem);
         const float *src = static_cast<const float *>(a.data);
         for (int i = threadIdx.x; i < a.n; i += blockDim.x)
             x[i] = src[i];
+        d.x = x;
     } else {
-        double *x = reinterpret_cast<double *>(smem);
+        double *t = reinterpret_cast<double *>(smem);
+        for (int i = threadIdx.x; i < kLlTab * kLlCopies; i += blockDim.x)
+        {
+            const int j = i / kLlCopies;
+            const double v = __ldg(&fm::kExpTab[j][0]);
+            t[i] = __hiloint2double(__double2hiint(v) - (j << 12),
+                                    __double2loint(v));
+        }
+        double *x = reinterpret_cast<double *>(smem + kLlTabBytes);
         const double *src = static_cast<const double *>(a.data);
         for (int i = threadIdx.x; i < a.n; i += blockDim.x)
             x[i] = src[i];
+        d.x = x;
+        d.tab = t + threadIdx.x % kLlCopies;
     }
     __syncthreads();
-    return smem;
+    return d;
+}
+
+// Dynamic shared memory stage_data takes for n points.
+constexpr size_t gmm_smem_bytes(int n, bool f32)
+{
+    return f32 ? (size_t)n * 4 : kLlTabBytes + (size_t)n * 8;
 }
 
 // Per-CTA acceptance counts (integer sums: any order gives the same).  Bit
@@ -518,7 +793,7 @@ __global__ void __launch_bounds__(kGmmThreads, VSMC_GMM_MIN_BLOCKS)
 k_gmm_init(GmmArgs a, double *lw)
 {
     extern __shared__ __align__(16) unsigned char gmm_smem[];
-    const void *data = stage_data<F32>(a, gmm_smem);
+    const GmmData data = stage_data<F32>(a, gmm_smem);
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i0 = gt / G;
     const int g = (int)(gt % G);
@@ -560,7 +835,7 @@ __global__ void __launch_bounds__(kGmmThreads, VSMC_GMM_MIN_BLOCKS)
 k_gmm_mcmc(GmmArgs a)
 {
     extern __shared__ __align__(16) unsigned char gmm_smem[];
-    const void *data = stage_data<F32>(a, gmm_smem);
+    const GmmData data = stage_data<F32>(a, gmm_smem);
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i0 = gt / G;
     const int g = (int)(gt % G);
@@ -603,7 +878,7 @@ __global__ void __launch_bounds__(kGmmThreads)
 k_gmm_loglik(GmmArgs a, double *out)
 {
     extern __shared__ __align__(16) unsigned char gmm_smem[];
-    const void *data = stage_data<F32>(a, gmm_smem);
+    const GmmData data = stage_data<F32>(a, gmm_smem);
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i0 = gt / G;
     const int g = (int)(gt % G);
@@ -691,15 +966,30 @@ k_gmm_path(const long long *tile_acc, int ntiles, int nacc,
            int64_t *hist_accept, double *hist_integrand, double *hist_grid)
 {
     __shared__ double sh[2][32];
-    __shared__ long long sha[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int resampled = ctl->resampled;
     const double M = ctl->lw_max;
     double p0 = 0.0, p1 = 0.0;
-    for (long long i = threadIdx.x; i < N; i += blockDim.x) {
-        const double w = resampled ? 1.0 : exp(lw[i] - M);
-        p0 = __dadd_rn(p0, __dmul_rn(w, ll[i]));
-        p1 = __dadd_rn(p1, w);
+    // a thread's particles in order, eight at a time (their loads and
+    // exponentials overlap)
+    constexpr int B = 8;
+    for (long long i0 = threadIdx.x; i0 < N; i0 += B * (long long)blockDim.x) {
+        double l[B], w[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const long long i = i0 + (long long)k * blockDim.x;
+            l[k] = i < N ? ll[i] : 0.0;
+            w[k] = i < N && !resampled ? lw[i] : M;
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+            w[k] = resampled ? 1.0 : exp(w[k] - M);
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+            if (i0 + (long long)k * blockDim.x < N) {
+                p0 = __dadd_rn(p0, __dmul_rn(w[k], l[k]));
+                p1 = __dadd_rn(p1, w[k]);
+            }
     }
     p0 = warp_sum(p0);
     p1 = warp_sum(p1);
@@ -707,22 +997,14 @@ k_gmm_path(const long long *tile_acc, int ntiles, int nacc,
         sh[0][wid] = p0;
         sh[1][wid] = p1;
     }
-    for (int m = 0; m < nacc; ++m) {
-        __syncthreads();
+    // acceptance totals: a warp per move
+    for (int m = wid; m < nacc; m += (int)(blockDim.x >> 5)) {
         long long v = 0;
-        for (int k = threadIdx.x; k < ntiles; k += blockDim.x)
+        for (int k = lane; k < ntiles; k += 32)
             v += tile_acc[(long long)k * kGmmMaxAcc + m];
-        for (int o = 16; o > 0; o >>= 1)
-            v += __shfl_xor_sync(0xffffffffu, v, o);
+        v = warp_sum_ll(v);
         if (lane == 0)
-            sha[wid] = v;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            long long tot = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-                tot += sha[w];
-            hist_accept[t * (1 + nacc) + 1 + m] = tot;
-        }
+            hist_accept[t * (1 + nacc) + 1 + m] = v;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -768,6 +1050,7 @@ struct vsmc_cuda_gmm {
     float *data32;   // and in float (MIXED form)
     int n;
     double mu0, sd0, shape0, scale0;
+    double xmin, xmax;
     double *hist_ess, *hist_zinc, *hist_integrand, *hist_grid;
     double *hist_mx, *hist_my; // finalize's monitor slots (unused)
     int32_t *hist_resampled;
@@ -812,6 +1095,8 @@ GmmArgs gmm_args(vsmc_cuda_gmm *g, int src, int dst)
     a.sd0 = g->sd0;
     a.shape0 = g->shape0;
     a.scale0 = g->scale0;
+    a.xmin = g->xmin;
+    a.xmax = g->xmax;
     a.alpha = g->alpha;
     a.sd = g->cfg.sd;
     a.sweeps = g->cfg.sweeps;
@@ -842,7 +1127,7 @@ GmmArgs gmm_args(vsmc_cuda_gmm *g, int src, int dst)
 template <bool F32>
 void launch_init_t(vsmc_cuda_gmm *g, const GmmArgs &a, int G, unsigned grid)
 {
-    const size_t smem = (size_t)a.n * (F32 ? 4 : 8);
+    const size_t smem = gmm_smem_bytes(a.n, F32);
 #define VSMC_CALL(K)                                                          \
     k_gmm_init<K, F32><<<grid, kGmmThreads, smem, g->stream>>>(a, g->lw)
     VSMC_GMM_SWITCH(G, VSMC_CALL)
@@ -852,7 +1137,7 @@ void launch_init_t(vsmc_cuda_gmm *g, const GmmArgs &a, int G, unsigned grid)
 template <bool F32>
 void launch_mcmc_t(vsmc_cuda_gmm *g, const GmmArgs &a, int G, unsigned grid)
 {
-    const size_t smem = (size_t)a.n * (F32 ? 4 : 8);
+    const size_t smem = gmm_smem_bytes(a.n, F32);
 #define VSMC_CALL(K)                                                          \
     k_gmm_mcmc<K, F32><<<grid, kGmmThreads, smem, g->stream>>>(a)
     VSMC_GMM_SWITCH(G, VSMC_CALL)
@@ -863,7 +1148,7 @@ template <bool F32>
 void launch_loglik_t(vsmc_cuda_gmm *g, const GmmArgs &a, int G, double *out)
 {
     const unsigned grid = (unsigned)gmm_ntiles_mcmc(a.N, G);
-    const size_t smem = (size_t)a.n * (F32 ? 4 : 8);
+    const size_t smem = gmm_smem_bytes(a.n, F32);
 #define VSMC_CALL(K)                                                          \
     k_gmm_loglik<K, F32><<<grid, kGmmThreads, smem, g->stream>>>(a, out)
     VSMC_GMM_SWITCH(G, VSMC_CALL)
@@ -913,49 +1198,35 @@ double alpha_at(uint64_t t, uint64_t iters, int power)
     return a;
 }
 
-// Picks the lanes per particle with the fastest MCMC sweep on the current
-// particles (CUDA events, best of 3 per candidate).  The trial sweeps write
-// into the spare parameter buffer and a copy of the engine positions, so
-// the sampler's state is untouched; and the choice changes no result, the
-// likelihood's summation order not depending on it.  The proposal and
-// acceptance work is repeated in every lane of a group, so the fastest G
-// balances it against the split data loop.
-int autotune_group(vsmc_cuda_gmm *g)
+// The lanes per particle G (a choice of speed alone: no result depends on
+// it).  A thread's time is that of n / G points plus `over` points' worth of
+// proposal and acceptance work, which every lane repeats; a CTA alone on its
+// SM runs at latency, two take `two` times as long, and more follow at
+// `rate` per CTA and SM.  The constants are fitted to measured sweeps (both
+// forms, n = 250 and 1000, N = 1000 to 300000, one B200): the pick is 1% (FP64)
+// and 2% (mixed) slower than the fastest G on average, 16% at most.  Timing
+// every G at each initialize, as before, cost 15 sweeps (12% of a run of 20
+// steps) and two waits of the host.
+int pick_group(const vsmc_cuda_gmm *g)
 {
-    GmmArgs a = gmm_args(g, g->cur, 1 - g->cur);
-    a.words = reinterpret_cast<uint64_t *>(g->scratch);
-    a.sweeps = 1;
-    cudaMemcpyAsync(a.words, g->words, g->cfg.N * 8, cudaMemcpyDeviceToDevice,
-                    g->stream);
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    const int cand[5] = {1, 2, 4, 8, 16};
-    int best = 4;
-    float best_ms = 1e30f;
-    for (int c = 0; c < 5; ++c) {
-        const unsigned grid = (unsigned)gmm_ntiles_mcmc(a.N, cand[c]);
-        float ms_min = 1e30f;
-        for (int r = 0; r < 3; ++r) {
-            cudaEventRecord(e0, g->stream);
-            if (gmm_f32(g))
-                launch_mcmc_t<true>(g, a, cand[c], grid);
-            else
-                launch_mcmc_t<false>(g, a, cand[c], grid);
-            cudaEventRecord(e1, g->stream);
-            cudaEventSynchronize(e1);
-            float ms = 0.0f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            ms_min = ms < ms_min ? ms : ms_min;
-            g->launches++;
-        }
-        if (ms_min < best_ms) {
-            best_ms = ms_min;
-            best = cand[c];
+    const bool f32 = gmm_f32(g);
+    const double over = f32 ? 160.0 : 30.0;
+    const double two = f32 ? 1.5 : 1.3, rate = f32 ? 0.9 : 0.8;
+    const int sms = device_sms();
+    int best = 1;
+    double least = 0.0;
+    for (int G = 1; G <= kLlClasses; G *= 2) {
+        const int c = gmm_ntiles_mcmc((long long)g->cfg.N, G);
+        const double per = (double)c / sms;
+        const double load =
+            c <= sms ? 1.0
+                     : (c <= 2 * sms ? two : rate * std::max(per, 2.0));
+        const double cost = ((double)g->n / G + over) * load;
+        if (G == 1 || cost < least) {
+            least = cost;
+            best = G;
         }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     return best;
 }
 
@@ -1072,7 +1343,7 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
     g->timing = false;
     g->ev_used = 0;
     g->launches = 0;
-    g->group = cfg->group == 0 ? 4 : cfg->group;
+    g->group = cfg->group == 0 ? pick_group(g) : cfg->group;
     // gmm_state::read_data (gmm_state.hpp:118-157)
     double xmax = data[0], xmin = data[0];
     for (uint64_t i = 0; i != n; ++i) {
@@ -1082,6 +1353,8 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
             xmin = data[i];
     }
     const double kappa = 1 / ((xmax - xmin) * (xmax - xmin));
+    g->xmin = xmin;
+    g->xmax = xmax;
     g->mu0 = 0.5 * (xmin + xmax);
     g->sd0 = 1 / std::sqrt(kappa);
     g->shape0 = 2;
@@ -1106,8 +1379,8 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
         delete g;
         return cuda_status(e, "vsmc_cuda_gmm_create");
     }
-    set_smem_attrs<true>((size_t)n * 4);
-    set_smem_attrs<false>((size_t)n * 8);
+    set_smem_attrs<true>(gmm_smem_bytes((int)n, true));
+    set_smem_attrs<false>(gmm_smem_bytes((int)n, false));
     cudaFuncSetAttribute(k_cv_finalize,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kFinalSmemTiles * (int)sizeof(double));
@@ -1162,7 +1435,6 @@ int vsmc_cuda_gmm_initialize(vsmc_cuda_gmm *g)
         return cuda_status(e, "vsmc_cuda_gmm_initialize");
     g->cur = 0;
     g->alpha = 0.0;
-    g->group = g->cfg.group == 0 ? 4 : g->cfg.group;
     GmmArgs a = gmm_args(g, 0, 0);
     const unsigned grid = (unsigned)gmm_ntiles_mcmc(N, g->group);
     if (gmm_f32(g))
@@ -1175,8 +1447,6 @@ int vsmc_cuda_gmm_initialize(vsmc_cuda_gmm *g)
         g->hist_grid);
     g->launches += 2;
     e = cudaGetLastError();
-    if (e == cudaSuccess && g->cfg.group == 0)
-        g->group = autotune_group(g);
     g->iter = 1;
     if (e == cudaSuccess)
         e = cudaGetLastError();
