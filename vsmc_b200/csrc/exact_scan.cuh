@@ -95,75 +95,15 @@ __device__ __forceinline__ int exact_window(double g, double d)
     return exact_binade(lo) == e ? e : kNoBinade;
 }
 
-// Block-wide exclusive max-scan of one value per thread (0 before the
-// first); `sh` needs blockDim.x/32 entries.
-__device__ __forceinline__ unsigned long long
-block_excl_max(unsigned long long v, unsigned long long *sh)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    unsigned long long inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long n = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o)
-            inc = max(inc, n);
-    }
-    if (lane == 31)
-        sh[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        unsigned long long s = lane < nw ? sh[lane] : 0ull;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long n = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o)
-                s = max(s, n);
-        }
-        if (lane < nw)
-            sh[lane] = s;
-    }
-    __syncthreads();
-    unsigned long long ex = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane == 0)
-        ex = 0;
-    if (wid > 0)
-        ex = max(ex, sh[wid - 1]);
-    __syncthreads();
-    return ex;
-}
-
-// The classification of a thread's kItems consecutive elements of a tile
+// The classification of a thread's R consecutive elements of a tile
 // (global index i0 + j): approximate tile start `a`, the thread's exclusive
 // prefix `pre` of the tile's weights, the weights `w`.  Elements at or past
 // N count as clean with k = 0 and the previous element's binade.
-struct ExactThread {
-    unsigned long long kincl[kItems]; // clean k of the tile through j
-    int e[kItems];
-    unsigned special;                 // bit j
-    int rank0;                        // specials of the tile before j = 0
-    int nspec;                        // specials of the tile
-    unsigned long long ktile;         // clean k of the tile
-    unsigned long long kb_in;         // kincl at the tile's last special
-                                      // before j = 0 (0: none)
-    int e_before;                     // binade of the element before j = 0
-};
-
-struct SmemExactThread {
-    unsigned long long shk[kThreads / 32];
-    unsigned long long shm[kThreads / 32];
-    int shi[kThreads / 32];
-    int elast[kThreads];
-};
-
-// A thread's own part of the classification of its R elements: e and
-// special as in ExactThread, kloc[j] the clean k of its elements through j,
-// nsp its specials.
 template <int R>
 struct ExactLocal {
-    unsigned long long kloc[R];
-    int e[R];
-    unsigned special;
+    unsigned long long kloc[R]; // clean k of the thread's elements through j
+    int e[R];                   // binades
+    unsigned special;           // bit j
     int nsp;
 };
 
@@ -272,83 +212,129 @@ exact_classify(long long i0, long long N, const double (&w)[R], double a,
     x.nsp = nsp;
 }
 
-__device__ __forceinline__ void
-exact_thread(long long i0, long long N, const double (&w)[kItems], double a,
-             double pre, double rel, ExactThread &x, SmemExactThread &sm)
-{
-    ExactLocal<kItems> l;
-    exact_classify(i0, N, w, a, pre, rel, l);
-#pragma unroll
-    for (int j = 0; j < kItems; ++j)
-        x.e[j] = l.e[j];
-    x.special = l.special;
-    const unsigned long long kr = l.kloc[kItems - 1];
-    const unsigned long long (&kloc)[kItems] = l.kloc;
-    const int nsp = l.nsp;
-    int nspec;
-    x.rank0 = block_excl_scan(nsp, sm.shi, nspec);
-    x.nspec = nspec;
-    unsigned long long ktile;
-    const unsigned long long kex = block_excl_scan(kr, sm.shk, ktile);
-    x.ktile = ktile;
-    unsigned long long vlast = 0;
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-        x.kincl[j] = kex + kloc[j];
-        if ((x.special >> j) & 1u)
-            vlast = x.kincl[j];
-    }
-    // kincl is non-decreasing, so the last special before the chunk holds
-    // the largest kincl of the earlier threads' last specials
-    x.kb_in = block_excl_max(vlast, sm.shm);
-    sm.elast[threadIdx.x] =
-        (x.special >> (kItems - 1)) & 1u ? kNoBinade : x.e[kItems - 1];
-    __syncthreads();
-    x.e_before = threadIdx.x > 0 ? sm.elast[threadIdx.x - 1] : kNoBinade;
-    __syncthreads();
-}
+// Shared memory of one tile's scan (NW warps).
+template <int NW>
+struct SmemExactScan {
+    unsigned long long k[NW]; // clean k of the warp
+    unsigned long long s[NW]; // the warp's clean k at its last special
+    int n[NW];                // its specials
+    int e[NW];                // binade of its last element
+};
 
-// Phase A: one tile's specials and sums, and the thread's element records
-// (the exact offset from the base, -1 at a special) into `rec`.
+// A thread's share of a tile's scan: its element records (the exact offset
+// from the last special before it or the tile's start, -1 at a special),
+// the specials of the tile before its first element, and the tile's sums.
+template <int R>
+struct ExactRec {
+    double rec[R];
+    int rank0, nspec;
+    unsigned long long ktile;
+};
+
+// Phase A for a tile of NW warps with R elements a thread: one scan of the
+// clean k over the group; the last special before a thread is found by
+// ballots, so the usual warp without specials pays nothing for them.
+// sync() is the group's barrier (called twice); special r goes to
+// out.spec(r, ...) and the binade of the tile's last element to out.last.
+template <int R, int NW, typename Sync, typename Out>
 __device__ __forceinline__ void
-exact_tile_record(const ExactThread &x, const double (&w)[kItems],
-                  long long base, long long i0, long long N, int tile,
-                  const ExactScan &ex, double (&rec)[kItems])
+exact_scan_tile(long long base, long long i0, long long N,
+                const double (&w)[R], double a, double pre, double rel,
+                int lane, int wid, SmemExactScan<NW> &sm, Sync sync, Out out,
+                ExactRec<R> &r)
 {
-    int r = x.rank0;
-    unsigned long long kb = x.kb_in;
+    constexpr unsigned kAll = 0xffffffffu;
+    ExactLocal<R> x;
+    exact_classify(i0, N, w, a, pre, rel, x);
+    const unsigned long long kr = x.kloc[R - 1];
+    const unsigned long long ki = warp_incl_scan(kr);
+    const unsigned long long ke = ki - kr;
+    const int elast = (x.special >> (R - 1)) & 1u ? kNoBinade : x.e[R - 1];
+    int e_before = __shfl_up_sync(kAll, elast, 1);
+    // specials of the warp: their count before the thread and the warp's
+    // clean k at the last of them
+    const unsigned any = __ballot_sync(kAll, x.nsp != 0);
+    int ne = 0;
+    bool has = false;
+    unsigned long long kb = 0;
+    if (any != 0) {
+        unsigned long long kat = 0; // kloc at the thread's last special
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-        if ((x.special >> j) & 1u) {
-            if (r < kExactCap) {
-                ExactSpecial s;
-                s.w = w[j];
-                s.k_before = x.kincl[j];
-                s.idx = (int)(i0 + j - base);
-                s.e_seg = j == 0 ? x.e_before
-                                 : ((x.special >> (j - 1)) & 1u
-                                        ? kNoBinade
-                                        : x.e[j - 1]);
-                ex.spec[(size_t)tile * kExactCap + r] = s;
-            }
-            ++r;
-            kb = x.kincl[j];
-            rec[j] = -1.0;
-        } else {
-            const unsigned long long K = x.kincl[j] - kb;
-            rec[j] = K == 0 ? 0.0
-                            : __dmul_rn((double)K, exact_pow2(x.e[j] - 52));
+        for (int j = 0; j < R; ++j)
+            if ((x.special >> j) & 1u)
+                kat = x.kloc[j];
+        const int ni = warp_incl_scan(x.nsp);
+        const unsigned before = any & ((1u << lane) - 1u);
+        const unsigned long long q =
+            __shfl_sync(kAll, ke + kat, 31 - __clz(before | 1u));
+        has = before != 0;
+        kb = has ? q : 0ull;
+        ne = ni - x.nsp;
+        if (lane == 31) {
+            sm.n[wid] = ni;
+            sm.s[wid] = x.nsp ? ke + kat : q;
         }
+    } else if (lane == 31) {
+        sm.n[wid] = 0;
     }
+    if (lane == 31) {
+        sm.k[wid] = ki;
+        sm.e[wid] = elast;
+    }
+    sync();
+    const unsigned long long wk = lane < NW ? sm.k[lane] : 0ull;
+    const int wn = lane < NW ? sm.n[lane] : 0;
+    const unsigned long long wki = warp_incl_scan(wk);
+    r.ktile = __shfl_sync(kAll, wki, 31);
+    const unsigned long long kp = __shfl_sync(kAll, wki - wk, wid);
+    const unsigned wany = __ballot_sync(kAll, wn != 0);
+    int np = 0;
+    unsigned long long kbw = 0; // the tile's clean k at the last special
+                                // of the earlier warps
+    r.nspec = 0;
+    if (wany != 0) {
+        const int wni = warp_incl_scan(wn);
+        r.nspec = __shfl_sync(kAll, wni, 31);
+        np = __shfl_sync(kAll, wni - wn, wid);
+        const unsigned before = wany & ((1u << wid) - 1u);
+        const unsigned long long at =
+            wki - wk + (wn != 0 ? sm.s[lane] : 0ull);
+        const unsigned long long q =
+            __shfl_sync(kAll, at, 31 - __clz(before | 1u));
+        kbw = before != 0 ? q : 0ull;
+    }
+    if (lane == 0)
+        e_before = wid > 0 ? sm.e[wid - 1] : kNoBinade;
+    sync(); // sm is free again
+    const unsigned long long k0 = kp + ke; // clean k before the thread
+    unsigned long long kl = has ? kp + kb : kbw; // ... at the last special
+    r.rank0 = np + ne;
     const long long last = min(base + (long long)kTile, N) - 1;
+    int rank = r.rank0;
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) // (constant indices keep x in registers)
+    for (int j = 0; j < R; ++j) {
+        if ((x.special >> j) & 1u) {
+            if (rank < kExactCap) {
+                ExactSpecial q;
+                q.w = w[j];
+                q.k_before = k0 + x.kloc[j];
+                q.idx = (int)(i0 + j - base);
+                q.e_seg = j == 0 ? e_before
+                                 : ((x.special >> (j > 0 ? j - 1 : 0)) & 1u
+                                        ? kNoBinade
+                                        : x.e[j > 0 ? j - 1 : 0]);
+                out.spec(rank, q);
+            }
+            ++rank;
+            kl = k0 + x.kloc[j];
+            r.rec[j] = -1.0;
+        } else {
+            const unsigned long long K = k0 + x.kloc[j] - kl;
+            r.rec[j] = K == 0 ? 0.0
+                              : __dmul_rn((double)K, exact_pow2(x.e[j] - 52));
+        }
         if (i0 + j == last)
-            ex.tiles[tile].e_last =
-                (x.special >> j) & 1u ? kNoBinade : x.e[j];
-    if (threadIdx.x == 0) {
-        ex.tiles[tile].k_total = x.ktile;
-        ex.tiles[tile].nspec = x.nspec;
+            out.last((x.special >> j) & 1u ? kNoBinade : x.e[j]);
     }
 }
 

@@ -1099,7 +1099,43 @@ __device__ __forceinline__ int pad8(int l) { return l + (l >> 3); }
 
 struct SmemExactCore {
     double shd[kThreads / 32];
-    SmemExactThread et;
+    SmemExactScan<kThreads / 32> et;
+};
+
+// Block-wide exclusive prefix of one double per thread of 256 and the
+// block's total, where the association does not matter (two barriers).
+__device__ __forceinline__ double block_prefix(double v, double *sh,
+                                               double &total)
+{
+    constexpr int NW = kThreads / 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double inc = warp_incl_scan(v);
+    if (lane == 31)
+        sh[wid] = inc;
+    __syncthreads();
+    double before = 0.0, all = 0.0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) {
+        const double x = sh[q];
+        before += q < wid ? x : 0.0;
+        all += x;
+    }
+    total = all;
+    return before + inc - v;
+}
+
+// Where a tile's scan puts its specials and last binade in global memory.
+struct ExactOut {
+    const ExactScan &ex;
+    int tile;
+    __device__ __forceinline__ void spec(int r, const ExactSpecial &q) const
+    {
+        ex.spec[(size_t)tile * kExactCap + r] = q;
+    }
+    __device__ __forceinline__ void last(int e) const
+    {
+        ex.tiles[tile].e_last = e;
+    }
 };
 
 template <bool Residual>
@@ -1252,13 +1288,14 @@ exact_tile_compute(const W &wsrc, long long N, const ResampleCtl *ctl,
     for (int j = 0; j < kItems; ++j)
         run += w[j];
     double total;
-    const double pre = block_excl_scan(run, sm.shd, total);
     const long long i0 = base + (long long)threadIdx.x * kItems;
     if (W::kApprox) {
+        const double pre = block_excl_scan(run, sm.shd, total);
         if (!Raw)
             approx_tile_record<Residual>(w, kk, pre, total, N, i0, tile, ex);
         return;
     }
+    const double pre = block_prefix(run, sm.shd, total);
     double a_apx;
     if (Residual)
         a_apx = Raw ? __ddiv_rn(tile_excl[tile], ctl->coeff_r_apx)
@@ -1267,15 +1304,19 @@ exact_tile_compute(const W &wsrc, long long N, const ResampleCtl *ctl,
     else
         a_apx = Raw ? __dmul_rn(tile_excl[tile], wsrc.spine_unnorm())
                     : __dmul_rn(tile_excl[tile], wsrc.spine_ratio());
-    ExactThread x;
-    exact_thread(i0, N, w, a_apx, pre, ExactMargin<W>::rel, x, sm.et);
-    double rec[kItems];
-    exact_tile_record(x, w, base, i0, N, tile, ex, rec);
+    ExactRec<kItems> x;
+    exact_scan_tile(base, i0, N, w, a_apx, pre, ExactMargin<W>::rel,
+                    (int)(threadIdx.x & 31), (int)(threadIdx.x >> 5), sm.et,
+                    [] { __syncthreads(); }, ExactOut{ex, tile}, x);
+    if (threadIdx.x == 0) {
+        ex.tiles[tile].k_total = x.ktile;
+        ex.tiles[tile].nspec = x.nspec;
+    }
     if (i0 < N) {
         if (Raw && !Residual && W::kExactNorm)
             store8(ex.rec, i0, N, w);
         if (!Raw && x.nspec <= kExactCap)
-            store8(ex.rec, i0, N, rec);
+            store8(ex.rec, i0, N, x.rec);
         if (!Raw && Residual)
             store8(ex.kint, i0, N, kk);
     }

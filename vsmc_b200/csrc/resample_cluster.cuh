@@ -74,8 +74,9 @@ struct alignas(16) RcGroup {
     double sv_w[kExactCap], sv_u[kExactCap]; // (rc_walk_slow) exact S at
                                              // the tile's specials
     double red_d[32];
-    unsigned long long red_k[32], red_s[32];
+    unsigned long long red_k[32];
     int red_n[32], red_e[32];
+    SmemExactScan<32> scn; // (a group of fewer warps uses its front)
     long long bound[2];
     // engine words, overflow tiles' S, uniforms, rank table in turn
     alignas(16) double buf[kUStage];
@@ -219,131 +220,40 @@ __device__ __forceinline__ void rc_plain_scan(const double (&w)[R],
     th.sync(); // vr and red_d are free again
 }
 
-// A thread's share of an exact scan: its element records (exact_scan.cuh)
-// and the specials of the tile before them.
-template <int R>
-struct RcRec {
-    double rec[R];
-    int rank0;
+// Where a group's scan puts its specials and last binade.
+struct RcOut {
+    RcScan &sc;
+    __device__ __forceinline__ void spec(int r, const ExactSpecial &q) const
+    {
+        sc.spec[r] = q;
+    }
+    __device__ __forceinline__ void last(int e) const { sc.tile.e_last = e; }
 };
 
-// Classification of the group's tile (weights w, approximate start a and
-// exclusive prefix pre): the tile's record and specials into `out`, the
-// thread's records into r.  The clean k is scanned over the group; the last
-// special before a thread is found by ballots, so the usual warp without
-// specials pays nothing for them.
+// The scan of the group's tile (weights w, approximate start a and exclusive
+// prefix pre): the tile's record and specials into `out`, the thread's
+// records into r.
 template <int R>
 __device__ __forceinline__ void
 rc_classify(long long base, long long N, const double (&w)[R], double a,
             double pre, double rel, const RcThread<R> &th, RcGroup &g,
-            RcScan &out, double *dump, RcRec<R> &r)
+            RcScan &out, double *dump, ExactRec<R> &r)
 {
-    constexpr int NW = RcThread<R>::NW;
-    constexpr unsigned kAll = 0xffffffffu;
-    const int lane = th.lane;
     const long long i0 = base + (long long)th.tid * R;
-    ExactLocal<R> x;
-    exact_classify(i0, N, w, a, pre, rel, x);
-    const unsigned long long kr = x.kloc[R - 1];
-    unsigned long long kat = 0; // kloc at the thread's last special
-#pragma unroll
-    for (int j = 0; j < R; ++j)
-        if ((x.special >> j) & 1u)
-            kat = x.kloc[j];
-    const unsigned long long ki = warp_incl_scan(kr);
-    const unsigned long long ke = ki - kr;
-    const int elast = (x.special >> (R - 1)) & 1u ? kNoBinade : x.e[R - 1];
-    int e_before = __shfl_up_sync(kAll, elast, 1);
-    // specials of the warp: their count before the thread and the warp's
-    // clean k at the last of them
-    const unsigned any = __ballot_sync(kAll, x.nsp != 0);
-    int ne = 0;
-    bool has = false;
-    unsigned long long kb = 0;
-    if (any != 0) {
-        const int ni = warp_incl_scan(x.nsp);
-        const unsigned before = any & ((1u << lane) - 1u);
-        const int src = 31 - __clz(before | 1u);
-        const unsigned long long q = __shfl_sync(kAll, ke + kat, src);
-        has = before != 0;
-        kb = has ? q : 0ull;
-        ne = ni - x.nsp;
-        if (lane == 31) {
-            g.red_n[th.wid] = ni;
-            g.red_s[th.wid] = x.nsp ? ke + kat : q;
-        }
-    } else if (lane == 31) {
-        g.red_n[th.wid] = 0;
-    }
-    if (lane == 31) {
-        g.red_k[th.wid] = ki;
-        g.red_e[th.wid] = elast;
-    }
-    th.sync();
-    const unsigned long long wk = lane < NW ? g.red_k[lane] : 0ull;
-    const int wn = lane < NW ? g.red_n[lane] : 0;
-    const unsigned long long wki = warp_incl_scan(wk);
-    const unsigned long long ktile = __shfl_sync(kAll, wki, 31);
-    const unsigned long long kp = __shfl_sync(kAll, wki - wk, th.wid);
-    const unsigned wany = __ballot_sync(kAll, wn != 0);
-    int nspec = 0, np = 0;
-    unsigned long long kbw = 0; // the tile's clean k at the last special
-                                // of the earlier warps
-    if (wany != 0) {
-        const int wni = warp_incl_scan(wn);
-        nspec = __shfl_sync(kAll, wni, 31);
-        np = __shfl_sync(kAll, wni - wn, th.wid);
-        const unsigned before = wany & ((1u << th.wid) - 1u);
-        const unsigned long long at =
-            wki - wk + (wn != 0 ? g.red_s[lane] : 0ull);
-        const unsigned long long q =
-            __shfl_sync(kAll, at, 31 - __clz(before | 1u));
-        kbw = before != 0 ? q : 0ull;
-    }
-    if (lane == 0)
-        e_before = th.wid > 0 ? g.red_e[th.wid - 1] : kNoBinade;
-    const unsigned long long k0 = kp + ke; // clean k before the thread
-    unsigned long long kl = has ? kp + kb : kbw; // ... at the last special
-    r.rank0 = np + ne;
-    const long long last = min(base + (long long)kTile, N) - 1;
-    int rank = r.rank0;
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-        if ((x.special >> j) & 1u) {
-            if (rank < kExactCap) {
-                ExactSpecial q;
-                q.w = w[j];
-                q.k_before = k0 + x.kloc[j];
-                q.idx = (int)(i0 + j - base);
-                q.e_seg = j == 0 ? e_before
-                                 : ((x.special >> (j > 0 ? j - 1 : 0)) & 1u
-                                        ? kNoBinade
-                                        : x.e[j > 0 ? j - 1 : 0]);
-                out.spec[rank] = q;
-            }
-            ++rank;
-            kl = k0 + x.kloc[j];
-            r.rec[j] = -1.0;
-        } else {
-            const unsigned long long K = k0 + x.kloc[j] - kl;
-            r.rec[j] = K == 0 ? 0.0
-                              : __dmul_rn((double)K, exact_pow2(x.e[j] - 52));
-        }
-        if (i0 + j == last)
-            out.tile.e_last = (x.special >> j) & 1u ? kNoBinade : x.e[j];
-    }
+    exact_scan_tile(base, i0, N, w, a, pre, rel, th.lane, th.wid,
+                    reinterpret_cast<SmemExactScan<RcThread<R>::NW> &>(g.scn),
+                    [&] { th.sync(); }, RcOut{out}, r);
     if (th.tid == 0) {
-        out.tile.k_total = ktile;
-        out.tile.nspec = nspec;
+        out.tile.k_total = r.ktile;
+        out.tile.nspec = r.nspec;
     }
     // a tile with more specials than kept: its values for the walk
-    if (nspec > kExactCap) {
+    if (r.nspec > kExactCap) {
 #pragma unroll
         for (int j = 0; j < R; ++j)
             if (i0 + j < N)
                 dump[i0 + j] = w[j];
     }
-    th.sync(); // the red_* arrays are free again
 }
 
 // The records of every tile's scan into the CTA's shared memory (after the
@@ -486,7 +396,7 @@ __device__ __forceinline__ double rc_start(const RcWalk &k, int t)
 template <bool U, int R>
 __device__ __forceinline__ void rc_values(const RcWalk &k, const RcGroup &g,
                                           int tile, const RcThread<R> &th,
-                                          const RcRec<R> &r, double (&S)[R])
+                                          const ExactRec<R> &r, double (&S)[R])
 {
     if (k.t[tile].nspec > kExactCap) {
         const double *o = g.buf + (U ? kTile : 0) + th.tid * R;
@@ -652,7 +562,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     // ---- the weights --------------------------------------------------
     double w[R]; // as scanned
     int kk[R];   // floor(N w) (residual)
-    RcRec<R> rw;
+    ExactRec<R> rw;
     double pre = 0.0, coeff_r = 1.0;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
@@ -685,7 +595,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
     // the drawn sequence's first stage, beside the weights' (its length is
     // known unless the scheme is residual)
     double tv[R]; // negated terms
-    RcRec<R> ru;
+    ExactRec<R> ru;
     double pre_u = 0.0;
     const auto terms = [&]() {
         // log(1 - U_n) / (NN - n), negated, and the tile's sum
