@@ -110,18 +110,23 @@ struct ExactLocal {
 template <int R>
 __device__ __forceinline__ void
 exact_classify(long long i0, long long N, const double (&w)[R], double a,
-               double pre, double rel, ExactLocal<R> &x)
+               double pre, double run, double rel, ExactLocal<R> &x)
 {
-    // one error bound for the thread's elements
-    double p = pre, wmax = 0.0;
-    bool bad = false;
+    // one error bound for the thread's elements (run: their sum).  A
+    // negative weight (the sign bits) or one that is not finite (m) leaves
+    // every element to the spine.
+    int signs = 0;
 #pragma unroll
-    for (int j = 0; j < R; ++j) {
-        p += w[j];
-        wmax = fmax(wmax, w[j]);
-        bad |= !(w[j] >= 0.0);
+    for (int j = 0; j < R; ++j)
+        signs |= __double2hiint(w[j]);
+    bool bad = false;
+    if (signs < 0) { // (a negative zero is a zero)
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            bad |= !(w[j] >= 0.0);
     }
-    const double m = fmax(__dadd_rn(a, p), wmax);
+    double p = __dadd_rn(pre, run);
+    const double m = __dadd_rn(a, p);
     const bool ok = !bad && m > 0x1p-960 && m < 0x1p960;
     double d = 0.0;
     if (ok) {
@@ -141,21 +146,22 @@ exact_classify(long long i0, long long N, const double (&w)[R], double a,
     bool fast = false;
     if (ok && i0 > 0 && i0 + R <= N) {
         const int e0 = exact_window(gp, d);
-        if (e0 != kNoBinade && e0 == exact_window(__dadd_rn(a, p), d)) {
+        if (e0 != kNoBinade && e0 == exact_window(m, d)) {
             const double sc = exact_pow2(52 - e0);
             bool slow = false;
+            int over = 0; // a high word outside [2^52, 2^53)
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 const double kf = __dmul_rn(w[j], sc);
                 const double t = __dadd_rn(kf, 0x1p52);
-                slow |= !(kf < 0x1p52) ||
-                        fabs(__dadd_rn(__dadd_rn(t, -0x1p52), -kf)) == 0.5;
+                over |= __double2hiint(t) ^ 0x43300000;
+                slow |= fabs(__dadd_rn(__dadd_rn(t, -0x1p52), -kf)) == 0.5;
                 kr += (unsigned long long)(__double_as_longlong(t) -
                                            __double_as_longlong(0x1p52));
                 kloc[j] = kr;
                 x.e[j] = e0;
             }
-            fast = !slow;
+            fast = !slow && (over & 0xfff00000) == 0;
         }
     }
     int ep = ok && !fast ? exact_window(gp, d) : kNoBinade;
@@ -239,13 +245,13 @@ struct ExactRec {
 template <int R, int NW, typename Sync, typename Out>
 __device__ __forceinline__ void
 exact_scan_tile(long long base, long long i0, long long N,
-                const double (&w)[R], double a, double pre, double rel,
-                int lane, int wid, SmemExactScan<NW> &sm, Sync sync, Out out,
-                ExactRec<R> &r)
+                const double (&w)[R], double a, double pre, double run,
+                double rel, int lane, int wid, SmemExactScan<NW> &sm,
+                Sync sync, Out out, ExactRec<R> &r)
 {
     constexpr unsigned kAll = 0xffffffffu;
     ExactLocal<R> x;
-    exact_classify(i0, N, w, a, pre, rel, x);
+    exact_classify(i0, N, w, a, pre, run, rel, x);
     const unsigned long long kr = x.kloc[R - 1];
     const unsigned long long ki = warp_incl_scan(kr);
     const unsigned long long ke = ki - kr;

@@ -1305,7 +1305,7 @@ exact_tile_compute(const W &wsrc, long long N, const ResampleCtl *ctl,
         a_apx = Raw ? __dmul_rn(tile_excl[tile], wsrc.spine_unnorm())
                     : __dmul_rn(tile_excl[tile], wsrc.spine_ratio());
     ExactRec<kItems> x;
-    exact_scan_tile(base, i0, N, w, a_apx, pre, ExactMargin<W>::rel,
+    exact_scan_tile(base, i0, N, w, a_apx, pre, run, ExactMargin<W>::rel,
                     (int)(threadIdx.x & 31), (int)(threadIdx.x >> 5), sm.et,
                     [] { __syncthreads(); }, ExactOut{ex, tile}, x);
     if (threadIdx.x == 0) {

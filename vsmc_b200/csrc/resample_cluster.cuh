@@ -240,7 +240,11 @@ rc_classify(long long base, long long N, const double (&w)[R], double a,
             RcScan &out, double *dump, ExactRec<R> &r)
 {
     const long long i0 = base + (long long)th.tid * R;
-    exact_scan_tile(base, i0, N, w, a, pre, rel, th.lane, th.wid,
+    double run = 0.0;
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+        run += w[j];
+    exact_scan_tile(base, i0, N, w, a, pre, run, rel, th.lane, th.wid,
                     reinterpret_cast<SmemExactScan<RcThread<R>::NW> &>(g.scn),
                     [&] { th.sync(); }, RcOut{out}, r);
     if (th.tid == 0) {
