@@ -43,7 +43,7 @@ namespace vsmc_b200 {
 
 constexpr int kExactCap = 64;         // specials kept per tile
 constexpr int kNoBinade = -100000;    // binade of a special element
-constexpr int kExactStage = 1024;     // specials the spine stages
+constexpr int kExactStage = 1280;     // additions the spine stages
 
 struct ExactTile {
     unsigned long long k_total; // sum of the clean elements' k
@@ -56,6 +56,12 @@ struct ExactSpecial {
     unsigned long long k_before;  // clean k of the tile before it
     int idx;                      // index in the tile
     int e_seg;                    // binade of the clean elements before it
+};
+
+// One step of the walk over the specials: the clean run before a special,
+// then the special's weight (0 where a run ends without one).
+struct ExactStep {
+    double seg, w;
 };
 
 // Device arrays of the exact scan (part of the resampling workspace).

@@ -401,7 +401,7 @@ __device__ __forceinline__ void cp_async_wait_all()
 
 template <bool Residual>
 struct SmemInvert {
-    double sw[kUStage];               // uniforms, then the outputs
+    alignas(16) double sw[kUStage];   // uniforms, then the outputs
     long long shl[kThreads / 32];
     long long bound[2];
     long long last[kThreads / 32];
@@ -1511,6 +1511,12 @@ k_exact_tiles(W wsrc, long long N, const ResampleCtl *ctl,
 
 constexpr int kExactDirtyStage = 256; // tiles with specials the spine stages
 
+// The sum of K clean units of binade e's last place.
+__device__ __forceinline__ double exact_clean(unsigned long long K, int e)
+{
+    return K == 0 ? 0.0 : __dmul_rn((double)K, exact_pow2(e - 52));
+}
+
 // Per tile with specials (its rank q among them, in order): the tile d, its
 // record, the clean k before it (pk: tiles with specials count 0), the
 // binade of the clean tiles after it and the exact S after it.  Ranks below
@@ -1527,9 +1533,11 @@ struct SmemExactSpine {
     unsigned long long pkq[kExactDirtyStage];
     int eaft[kExactDirtyStage];
     double sout[kExactDirtyStage];
-    // the specials of the staged tiles, when they fit: tile q's at
-    // st[st_off[q]...]
-    ExactSpecial st[kExactStage];
+    // the walk's additions, when they fit: tile q's from st_off[q], first
+    // the clean tiles before it, then its specials (each after the clean
+    // run before it), then its clean tail; S after each
+    ExactStep st[kExactStage];
+    double S[kExactStage];
     int st_off[kExactDirtyStage];
 };
 
@@ -1644,31 +1652,76 @@ k_exact_spine_body(W wsrc, long long N, ResampleCtl *ctl, int nt,
     }
     __syncthreads();
     const bool staged_all = ndt <= kExactDirtyStage;
-    // 2. stage the staged tiles' specials when they all fit
+    // 2. stage the walk's additions when they all fit (a tile with more
+    // specials than kept is summed element by element)
     int nsq = 0;
     if ((int)threadIdx.x < min(ndt, kExactDirtyStage)) {
         const ExactTile et = sm.tq[threadIdx.x];
-        nsq = et.nspec <= kExactCap ? et.nspec : 0;
+        nsq = et.nspec <= kExactCap ? et.nspec + 2 : kExactStage;
     }
     int nst;
     const int soff = block_excl_scan(nsq, sm.shi, nst); // ends with a barrier
-    const bool fits = staged_all && nst <= kExactStage;
+    const bool fits = staged_all && nst <= kExactStage - 4;
     if (fits && (int)threadIdx.x < ndt)
         sm.st_off[threadIdx.x] = soff;
     __syncthreads();
     if (fits) { // a warp per tile with specials
         for (int q = wq; q < ndt; q += nw) {
-            const int ns = sm.tq[q].nspec;
-            if (ns > kExactCap)
-                continue;
-            for (int r = lane; r < ns; r += 32)
-                sm.st[sm.st_off[q] + r] =
-                    ex.spec[(size_t)sm.dq[q] * kExactCap + r];
+            const ExactTile et = sm.tq[q];
+            const ExactSpecial *sp = ex.spec + (size_t)sm.dq[q] * kExactCap;
+            ExactStep *st = sm.st + sm.st_off[q];
+            for (int r = lane; r < et.nspec + 2; r += 32) {
+                ExactStep x;
+                x.w = 0.0;
+                if (r == 0) {
+                    x.seg = q == 0 ? 0.0
+                                   : exact_clean(sm.pkq[q] - sm.pkq[q - 1],
+                                                 sm.eaft[q - 1]);
+                } else {
+                    const unsigned long long kb =
+                        r > 1 ? sp[r - 2].k_before : 0ull;
+                    if (r <= et.nspec) {
+                        x.seg = exact_clean(sp[r - 1].k_before - kb,
+                                            sp[r - 1].e_seg);
+                        x.w = sp[r - 1].w;
+                    } else {
+                        x.seg = exact_clean(et.k_total - kb, et.e_last);
+                    }
+                }
+                st[r] = x;
+            }
         }
     }
     __syncthreads();
-    // 3. the walk over the tiles with specials
-    if (threadIdx.x == 0) {
+    // 3. the walk over the tiles with specials: one chain of additions
+    if (fits) {
+        if (threadIdx.x == 0) {
+            double S = 0.0;
+            for (int i = 0; i < nst; i += 4) { // (the array is padded by 4)
+                ExactStep q[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m)
+                    q[m] = sm.st[i + m];
+#pragma unroll
+                for (int m = 0; m < 4; ++m)
+                    if (i + m < nst) {
+                        S = __dadd_rn(__dadd_rn(S, q[m].seg), q[m].w);
+                        sm.S[i + m] = S;
+                    }
+            }
+        }
+        __syncthreads();
+        for (int q = wq; q < ndt; q += nw) {
+            const int d = sm.dq[q], ns = sm.tq[q].nspec;
+            const double *Sq = sm.S + sm.st_off[q];
+            for (int r = lane; r < ns; r += 32)
+                ex.s_spec[(size_t)d * kExactCap + r] = Sq[r + 1];
+            if (lane == 0) {
+                ex.start[d] = Sq[0];
+                sm.sout[q] = Sq[ns + 1];
+            }
+        }
+    } else if (threadIdx.x == 0) {
         const double Nd = (double)resample_children(ctl, N);
         const double coeff_r = Residual && !Raw ? ctl->coeff_r : 1.0;
         double S = 0.0;
@@ -1687,8 +1740,7 @@ k_exact_spine_body(W wsrc, long long N, ResampleCtl *ctl, int nt,
                 unsigned long long kb = 0;
                 for (int r = 0; r < et.nspec; ++r) {
                     const ExactSpecial sp =
-                        fits ? sm.st[sm.st_off[q] + r]
-                             : ex.spec[(size_t)d * kExactCap + r];
+                        ex.spec[(size_t)d * kExactCap + r];
                     const unsigned long long seg = sp.k_before - kb;
                     if (seg != 0)
                         S = __dadd_rn(S, __dmul_rn((double)seg,
@@ -1767,6 +1819,31 @@ k_exact_spine(W wsrc, long long N, ResampleCtl *ctl, int nt, ExactScan ex)
 {
     __shared__ SmemExactSpine sm;
     k_exact_spine_body<W, Residual, Raw>(wsrc, N, ctl, nt, ex, sm);
+}
+
+// A thread's eight ints of a tile to shared memory, and the tile from there
+// to a caller's array of any alignment.
+__device__ __forceinline__ void stage8(int4 *s4, const int32_t (&v)[kItems])
+{
+    s4[2 * threadIdx.x] = make_int4(v[0], v[1], v[2], v[3]);
+    s4[2 * threadIdx.x + 1] = make_int4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void unstage8(int32_t *dst, long long base,
+                                         long long N, const int4 *s4)
+{
+    if (base + kTile <= N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        int4 *d = reinterpret_cast<int4 *>(dst + base);
+        d[threadIdx.x] = s4[threadIdx.x];
+        d[threadIdx.x + kThreads] = s4[threadIdx.x + kThreads];
+    } else {
+        const int32_t *s = reinterpret_cast<const int32_t *>(s4);
+#pragma unroll
+        for (int j = 0; j < kItems; ++j) {
+            const long long i = base + (long long)j * kThreads + threadIdx.x;
+            if (i < N)
+                dst[i] = s[j * kThreads + threadIdx.x];
+        }
+    }
 }
 
 // The inversion kernel (internal::inversion, common.hpp:57-84, on the FP64
@@ -1875,7 +1952,12 @@ k_invert_body(W wsrc, long long N, ResampleCtl *ctl, const double *tile_excl,
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
         Cx[j] = 0.0;
-    if (exact) {
+    if (exact && nsp_tile == 0) {
+        // (the usual tile: no special, every record is from the start)
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+            Cx[j] = __dadd_rn(a, rv[j]);
+    } else if (exact) {
         int nsp = 0;
 #pragma unroll
         for (int j = 0; j < kItems; ++j)
@@ -1983,35 +2065,20 @@ k_invert_body(W wsrc, long long N, ResampleCtl *ctl, const double *tile_excl,
         if (i == tile_last)
             tile_sinc_last[tile] = sc[j];
     }
-    // stage the outputs through shared memory for coalesced stores
+    // stage the outputs through shared memory for coalesced stores (16
+    // bytes a thread where the caller's array allows)
     __syncthreads();
-    int32_t *s32 = reinterpret_cast<int32_t *>(sw);
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-        s32[threadIdx.x * kItems + j] = cf[j];
-        s32[kTile + threadIdx.x * kItems + j] = sc[j];
-    }
+    int4 *s4 = reinterpret_cast<int4 *>(sw);
+    stage8(s4, cf);
+    stage8(s4 + kTile / 4, sc);
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-        const long long i = base + (long long)j * kThreads + threadIdx.x;
-        if (i < N) {
-            copy_from[i] = s32[j * kThreads + threadIdx.x];
-            sinc_local[i] = s32[kTile + j * kThreads + threadIdx.x];
-        }
-    }
+    unstage8(copy_from, base, N, s4);
+    unstage8(sinc_local, base, N, s4 + kTile / 4);
     if (rep_out != nullptr) {
         __syncthreads();
-#pragma unroll
-        for (int j = 0; j < kItems; ++j)
-            s32[threadIdx.x * kItems + j] = rp[j];
+        stage8(s4, rp);
         __syncthreads();
-#pragma unroll
-        for (int j = 0; j < kItems; ++j) {
-            const long long i = base + (long long)j * kThreads + threadIdx.x;
-            if (i < N)
-                rep_out[i] = s32[j * kThreads + threadIdx.x];
-        }
+        unstage8(rep_out, base, N, s4);
     }
 }
 
@@ -2046,8 +2113,8 @@ struct SmemZeroSpine {
     int32_t S[kSpineStage]; // zero counts, then surplus ends E
 };
 struct SmemFill {
-    int32_t ss[kTile];  // sinc of one parent tile
-    int32_t tab[kTile]; // parent of each zero-slot rank of this tile
+    int4 tab[kTile / 4]; // parent of each zero-slot rank of this tile
+    int wm[kThreads / 32];
 };
 
 __device__ __forceinline__ void
@@ -2139,10 +2206,12 @@ k_zero_spine(const int32_t *tile_zeros, const int32_t *tile_sinc_last,
 // the k-th such slot takes the k-th surplus child in parent order, i.e. the
 // first parent p with sinc(p) > k, sinc(p) = sinc_local[p] + zexcl[tile(p)].
 // The zero slots of tile t hold the consecutive ranks [zexcl[t],
-// zexcl[t + 1]).  The CTA of tile t stages the parent tiles tfirst[t]..
-// tlast[t] one at a time in shared memory; parent p owns the ranks
-// [sinc(p - 1), sinc(p)) and writes itself into a rank -> parent table for
-// those that fall in the tile's window, so no slot searches.
+// zexcl[t + 1]).  Parent p of the tiles tfirst[t] .. tlast[t] owns the ranks
+// [sinc(p - 1), sinc(p)) and marks the first of them that falls in the tile's
+// window; parents increase with the rank, so the running maximum of the
+// marks is each rank's parent.  A parent with thousands of children costs no
+// more than one with two (writing every rank took a skewed step's fill from
+// 78 to 118 us at 2^24).
 __device__ __forceinline__ void
 k_cfrp_fill_body(long long N, ResampleCtl *ctl, const int32_t *sinc_local,
                  const int32_t *zexcl, const int32_t *tfirst,
@@ -2151,8 +2220,8 @@ k_cfrp_fill_body(long long N, ResampleCtl *ctl, const int32_t *sinc_local,
 {
     if (!ctl->active)
         return;
-    int32_t *ss = sm.ss;
-    int32_t *tab = sm.tab;
+    int32_t *tab = reinterpret_cast<int32_t *>(sm.tab);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int tile = tile_bid;
     const int t0 = tfirst[tile], t1 = tlast[tile];
     if (t1 < t0)
@@ -2166,23 +2235,67 @@ k_cfrp_fill_body(long long N, ResampleCtl *ctl, const int32_t *sinc_local,
         const long long i = base + (long long)j * kThreads + threadIdx.x;
         cf[j] = i < N ? copy_from[i] : 0;
     }
-    for (int k = threadIdx.x; k < z; k += kThreads)
-        tab[k] = -1;
-    int prev_top = INT_MIN; // ranks below the first staged tile map to it
+    sm.tab[2 * threadIdx.x] = make_int4(-1, -1, -1, -1);
+    sm.tab[2 * threadIdx.x + 1] = make_int4(-1, -1, -1, -1);
+    __syncthreads();
+    int prev_top = INT_MIN; // ranks below the first parent tile map to it
     for (int pt = t0; pt <= t1; ++pt) {
         const long long pb = (long long)pt * kTile;
         const int len = (int)min((long long)kTile, N - pb);
         const int32_t zoff = zexcl[pt];
-        for (int j = threadIdx.x; j < len; j += kThreads)
-            ss[j] = sinc_local[pb + j] + zoff;
-        __syncthreads();
-        for (int j = threadIdx.x; j < len; j += kThreads) {
-            const int lo = max(j > 0 ? ss[j - 1] : prev_top, Z0);
-            const int hi = min(ss[j], Z0 + z);
-            for (int r = lo; r < hi; ++r)
-                tab[r - Z0] = (int32_t)(pb + j);
+        int cur[kItems], edge[kItems];
+#pragma unroll
+        for (int j = 0; j < kItems; ++j) {
+            const int l = j * kThreads + threadIdx.x;
+            cur[j] = l < len ? sinc_local[pb + l] + zoff : INT_MIN;
+            // the value before the warp's first
+            edge[j] = prev_top;
+            if (lane == 0 && l > 0 && l < len)
+                edge[j] = sinc_local[pb + l - 1] + zoff;
         }
-        prev_top = max(prev_top, ss[len - 1]);
+        const int top = sinc_local[pb + len - 1] + zoff;
+#pragma unroll
+        for (int j = 0; j < kItems; ++j) {
+            int before = __shfl_up_sync(0xffffffffu, cur[j], 1);
+            if (lane == 0)
+                before = edge[j];
+            const int lo = max(before, Z0);
+            if (lo < min(cur[j], Z0 + z))
+                tab[lo - Z0] = (int32_t)(pb + j * kThreads + threadIdx.x);
+        }
+        prev_top = max(prev_top, top);
+    }
+    const int covered = prev_top - Z0; // ranks with a parent
+    __syncthreads();
+    // running maximum of the marks, kItems consecutive ranks per thread
+    {
+        int4 q0 = sm.tab[2 * threadIdx.x], q1 = sm.tab[2 * threadIdx.x + 1];
+        q0.y = max(q0.x, q0.y);
+        q0.z = max(q0.y, q0.z);
+        q0.w = max(q0.z, q0.w);
+        q1.x = max(q0.w, q1.x);
+        q1.y = max(q1.x, q1.y);
+        q1.z = max(q1.y, q1.z);
+        q1.w = max(q1.z, q1.w);
+        int in = q1.w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int q = __shfl_up_sync(0xffffffffu, in, o);
+            if (lane >= o)
+                in = max(in, q);
+        }
+        if (lane == 31)
+            sm.wm[wid] = in;
+        int ex = __shfl_up_sync(0xffffffffu, in, 1);
+        if (lane == 0)
+            ex = -1;
+        __syncthreads();
+        ex = max(ex, __reduce_max_sync(0xffffffffu,
+                                       lane < wid ? sm.wm[lane] : -1));
+        sm.tab[2 * threadIdx.x] = make_int4(max(q0.x, ex), max(q0.y, ex),
+                                            max(q0.z, ex), max(q0.w, ex));
+        sm.tab[2 * threadIdx.x + 1] = make_int4(
+            max(q1.x, ex), max(q1.y, ex), max(q1.z, ex), max(q1.w, ex));
         __syncthreads();
     }
 #pragma unroll
@@ -2190,7 +2303,7 @@ k_cfrp_fill_body(long long N, ResampleCtl *ctl, const int32_t *sinc_local,
         const long long i = base + (long long)j * kThreads + threadIdx.x;
         if (i < N && cf[j] < 0) {
             const int k = -cf[j] - 1; // rank - Z0
-            const int32_t p = k < z ? tab[k] : -1;
+            const int32_t p = k < min(z, covered) ? tab[k] : -1;
             if (p >= 0) {
                 copy_from[i] = p;
             } else { // no parent found: replication != N

@@ -83,15 +83,11 @@ struct alignas(16) RcGroup {
 };
 
 // The gathered records of one exact scan and its walk: the additions in
-// order, first the clean run `seg` before a special (or the end of the
-// tile), then the special's weight (0 at the end of a tile).
-struct RcStep {
-    double seg, w;
-};
+// order: each tile's specials, then its clean tail.
 struct RcWalk {
     ExactTile t[kRcMaxTiles];
     int off[kRcMaxTiles + 1]; // specials before tile t
-    RcStep step[kRcStage + kRcMaxTiles + 8];
+    ExactStep step[kRcStage + kRcMaxTiles + 8];
     double S[kRcStage + kRcMaxTiles + 8]; // after each step
     double start[kRcMaxTiles + 1];        // before each tile
     int slow; // overflow tiles, or more specials than staged
@@ -290,11 +286,6 @@ __device__ __forceinline__ void rc_gather_tiles(cg::cluster_group &cl,
     }
 }
 
-__device__ __forceinline__ double rc_clean(unsigned long long K, int e)
-{
-    return K == 0 ? 0.0 : __dmul_rn((double)K, exact_pow2(e - 52));
-}
-
 // The walk's additions: a warp per tile.
 template <int B>
 __device__ __forceinline__ void rc_gather_specials(cg::cluster_group &cl,
@@ -312,12 +303,12 @@ __device__ __forceinline__ void rc_gather_specials(cg::cluster_group &cl,
         const ExactSpecial *sp = rg->scan[B].spec;
         for (int r = lane; r <= n; r += 32) {
             const unsigned long long kb = r > 0 ? sp[r - 1].k_before : 0ull;
-            RcStep st;
+            ExactStep st;
             if (r < n) {
-                st.seg = rc_clean(sp[r].k_before - kb, sp[r].e_seg);
+                st.seg = exact_clean(sp[r].k_before - kb, sp[r].e_seg);
                 st.w = sp[r].w;
             } else {
-                st.seg = rc_clean(et.k_total - kb, et.e_last);
+                st.seg = exact_clean(et.k_total - kb, et.e_last);
                 st.w = 0.0;
             }
             k.step[b + t + r] = st;
@@ -331,7 +322,7 @@ __device__ __forceinline__ void rc_walk(RcWalk &k, int nt)
     const int n = k.off[nt] + nt;
     double S = 0.0;
     for (int i = 0; i < n; i += 4) { // (reads past n stay in the array)
-        RcStep q[4];
+        ExactStep q[4];
 #pragma unroll
         for (int m = 0; m < 4; ++m)
             q[m] = k.step[i + m];
@@ -363,7 +354,7 @@ __device__ __noinline__ void rc_walk_slow(cg::cluster_group cl, RcShared &sm,
             unsigned long long kb = 0;
             for (int r = 0; r < et.nspec; ++r) {
                 const ExactSpecial sp = rg->scan[B].spec[r];
-                S = __dadd_rn(S, rc_clean(sp.k_before - kb, sp.e_seg));
+                S = __dadd_rn(S, exact_clean(sp.k_before - kb, sp.e_seg));
                 S = __dadd_rn(S, sp.w);
                 if (keep) {
                     if (U)
@@ -373,7 +364,7 @@ __device__ __noinline__ void rc_walk_slow(cg::cluster_group cl, RcShared &sm,
                 }
                 kb = sp.k_before;
             }
-            S = __dadd_rn(S, rc_clean(et.k_total - kb, et.e_last));
+            S = __dadd_rn(S, exact_clean(et.k_total - kb, et.e_last));
         } else {
             const long long b0 = (long long)t * kTile;
             const int n = (int)(min(b0 + (long long)kTile, N) - b0);
