@@ -71,6 +71,7 @@ struct vsmc_cuda_cv_filter {
 namespace {
 
 constexpr int kMonParts = 1184;
+static_assert(kMonParts <= kMonMaxParts, "monitor partial sums fit");
 
 size_t filter_bytes(const vsmc_cuda_cv_config &c)
 {
@@ -290,7 +291,7 @@ void launch_monitor_flush(vsmc_cuda_cv_filter *f)
         static_cast<const Real *>(f->state[f->cur][1]), f->copy_from, N,
         f->mon_part, f->ctl, t);
     const bool anch = f->cfg.form == VSMC_CUDA_MIXED;
-    k_cv_monitor_finish<<<1, 32, 0, f->stream>>>(
+    k_cv_monitor_finish<<<1, kThreads, 0, f->stream>>>(
         f->mon_part, kMonParts, N, t, f->ctl,
         anch ? f->obs_x : nullptr, anch ? f->obs_y : nullptr,
         f->hist_mean_x, f->hist_mean_y);

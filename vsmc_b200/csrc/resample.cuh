@@ -82,6 +82,15 @@ __device__ __forceinline__ long long bin_floor(double u, int kb)
     return v >= K ? (1ll << kb) : (long long)v;
 }
 
+// ... in 32 bits (sequences of at most 2^30 uniforms: K <= 2^27).
+__device__ __forceinline__ int bin_floor32(double u, int K)
+{
+    const double v = __dmul_rn(u, (double)K);
+    if (!(v >= 0.0))
+        return -1;
+    return v >= (double)K ? K : (int)v;
+}
+
 // Bins (klo - 1, khi] start at u_n: klo - 1 = bin_floor(u_{n-1}) (0 for
 // n = 0), khi = bin_floor(u_n); callers carry khi on to the next n.
 __device__ __forceinline__ void bin_fill(int32_t *L, int kb, long long klo,
@@ -346,6 +355,47 @@ __device__ __forceinline__ double residual_split(double w, double Nd,
     return modf(__dmul_rn(Nd, w), &k);
 }
 
+// A tile's values in shared memory are padded by one slot per 8, so that a
+// thread reading its kItems consecutive values meets no bank conflict.
+constexpr int kTilePad = kTile + kTile / 8;
+__device__ __forceinline__ int pad8(int l) { return l + (l >> 3); }
+
+// Eight values of a thread to global memory (vector stores when all are
+// below N).
+template <typename T>
+__device__ __forceinline__ void store8(T *dst, long long i0, long long N,
+                                       const T (&v)[kItems])
+{
+    if (i0 + kItems <= N) {
+        if (sizeof(T) == 8) {
+            double2 *d = reinterpret_cast<double2 *>(dst + i0);
+#pragma unroll
+            for (int j = 0; j < kItems / 2; ++j) {
+                double2 q;
+                q.x = *reinterpret_cast<const double *>(&v[2 * j]);
+                q.y = *reinterpret_cast<const double *>(&v[2 * j + 1]);
+                d[j] = q;
+            }
+        } else {
+            int4 *d = reinterpret_cast<int4 *>(dst + i0);
+#pragma unroll
+            for (int j = 0; j < kItems / 4; ++j) {
+                int4 q;
+                q.x = *reinterpret_cast<const int *>(&v[4 * j]);
+                q.y = *reinterpret_cast<const int *>(&v[4 * j + 1]);
+                q.z = *reinterpret_cast<const int *>(&v[4 * j + 2]);
+                q.w = *reinterpret_cast<const int *>(&v[4 * j + 3]);
+                d[j] = q;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+            if (i0 + j < N)
+                dst[i0 + j] = v[j];
+    }
+}
+
 // The latency-bound per-tile kernels of the sorted sequence and the cfrp
 // fill are compiled for eight CTAs per SM (32 registers): more warps in
 // flight hide their dependent loads.
@@ -370,6 +420,7 @@ struct SmemNone {
 };
 struct SmemSortedSums {
     double sh[kThreads / 32];
+    uint64_t w[kTile + 4 + (kTile + 4) / 8 + 1]; // engine words, padded
 };
 struct SmemSortedUniforms {
     double sh[kThreads / 32];
@@ -597,28 +648,6 @@ k_spine_weights(const double *tile_sum, const long long *tile_k,
         ntiles, N, eng, ctl, blockIdx.x, sm);
 }
 
-// Words at stream positions pos0 .. pos0+7 of a Threefry4x64 engine (two or
-// three block evaluations).
-__device__ __forceinline__ void threefry_words8(const EngineRef &eng,
-                                                unsigned long long pos0,
-                                                uint64_t w[8])
-{
-    const unsigned long long b0 = pos0 / 4;
-    const int s = (int)(pos0 % 4);
-    const u64x4 x = threefry4x64_20(ctr64_add(eng.ctr, b0 + 1), eng.key);
-    const u64x4 y = threefry4x64_20(ctr64_add(eng.ctr, b0 + 2), eng.key);
-    u64x4 z;
-    z.v[0] = z.v[1] = z.v[2] = z.v[3] = 0;
-    if (s > 0)
-        z = threefry4x64_20(ctr64_add(eng.ctr, b0 + 3), eng.key);
-    const uint64_t q[12] = {x.v[0], x.v[1], x.v[2], x.v[3], y.v[0], y.v[1],
-                            y.v[2], y.v[3], z.v[0], z.v[1], z.v[2], z.v[3]};
-    // w[j] = q[s + j] with constant indices only (register selects)
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        w[j] = s == 0 ? q[j] : s == 1 ? q[j + 1] : s == 2 ? q[j + 2] : q[j + 3];
-}
-
 // Stratified U01 sequence (U01SequenceStratified, u01.hpp:212-243):
 // u_n = U_n * delta + n * delta, U_n from engine word offset + n.  One
 // Threefry block per thread gives four consecutive u_n.  Adjacent values can
@@ -699,21 +728,11 @@ k_uniforms_stratified(EngineRef eng, const ResampleCtl *ctl, double *u,
 // sum_{k<=n} log(1 - U_k) / (NN - k); u_n = 1 - exp(lmax_n).  Two passes
 // over tiles of kTile uniforms around a deterministic spine; each thread owns
 // 8 consecutive n.
-__device__ __forceinline__ void sorted_terms8(const EngineRef &eng,
-                                              unsigned long long off,
-                                              long long n0, long long NN,
-                                              double t[8])
+__device__ __forceinline__ double sorted_term(uint64_t word, long long n,
+                                              long long NN)
 {
-    uint64_t w[8];
-    threefry_words8(eng, off + (unsigned long long)n0, w);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const long long n = n0 + j;
-        const double U = canonical_u64(w[j]);
-        t[j] = n < NN ? __ddiv_rn(fm::fm_log(__dadd_rn(1.0, -U)),
-                                  (double)(NN - n))
-                      : 0.0;
-    }
+    const double U = canonical_u64(word);
+    return __ddiv_rn(fm::fm_log(__dadd_rn(1.0, -U)), (double)(NN - n));
 }
 
 // Which sorted sequence a launch builds: the step's (ctl->active, NN,
@@ -758,20 +777,60 @@ k_sorted_tile_sums_body(EngineRef eng, const ResampleCtl *ctl, double *tile_sum,
     const long long base = (long long)bid * kTile;
     if (base >= NN)
         return;
+    // the tile's engine words: each Threefry block once, whatever the
+    // engine's position within a block (a thread's 8 words straddle three
+    // blocks three times out of four)
+    const unsigned long long first =
+        ctl->offset + (unsigned long long)base;
+    const int lead = (int)(first % 4);
+    const int count = (int)min((long long)kTile, NN - base);
+    const auto block = [&](int b) {
+        return threefry4x64_20(
+            ctr64_add(eng.ctr, first / 4 + (unsigned)b + 1), eng.key);
+    };
+    const auto put = [&](int b, const u64x4 &x) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            sm.w[pad8(4 * b + l)] = x.v[l];
+    };
+    const int nb = (lead + count + 3) / 4; // at most 2 kThreads + 1
+    {
+        const int b = threadIdx.x;
+        // (two independent chains)
+        const u64x4 x = block(b), y = block(b + kThreads);
+        if (b < nb)
+            put(b, x);
+        if (b + kThreads < nb)
+            put(b + kThreads, y);
+        if (b == 0 && nb > 2 * kThreads)
+            put(2 * kThreads, block(2 * kThreads));
+    }
+    __syncthreads();
     double t[kItems];
     const long long n0 = base + (long long)threadIdx.x * kItems;
-    sorted_terms8(eng, ctl->offset, n0, NN, t);
     double s = 0.0;
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
+        const long long n = n0 + j;
+        t[j] = n < NN ? sorted_term(
+                            sm.w[pad8(lead + threadIdx.x * kItems + j)], n,
+                            NN)
+                      : 0.0;
         s += t[j];
-        if (n0 + j < NN)
-            u[n0 + j] = t[j];
     }
-    double total;
-    block_excl_scan(s, sh, total);
-    if (threadIdx.x == 0)
+    if (n0 < NN)
+        store8(u, n0, NN, t);
+    // (for the exact scan's classification: any association)
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0)
+        sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double total = 0.0;
+        for (int k = 0; k < kThreads / 32; ++k)
+            total += sh[k];
         tile_sum[bid] = total;
+    }
 }
 
 static __global__ void __launch_bounds__(VSMC_SCAN_BOUNDS)
@@ -837,15 +896,22 @@ k_sorted_uniforms_body(const ResampleCtl *ctl, const ExactScan exu,
     const int nsp_tile = exu.tiles[bid].nspec;
     if (nsp_tile <= kExactCap && (int)threadIdx.x < nsp_tile)
         sm.sv[threadIdx.x] = exu.s_spec[(size_t)bid * kExactCap + threadIdx.x];
-    int nsp = 0;
-#pragma unroll
-    for (int j = 0; j < kItems; ++j)
-        nsp += rv[j] < 0.0;
-    int nspec;
-    const int rank0 = block_excl_scan(nsp, sm.shi, nspec); // ends with a barrier
     const double a = exu.start[bid]; // -lmax before the tile
     double S[kItems];
-    exact_values(rv, rank0, a, sm.sv, nsp_tile > kExactCap, S);
+    if (nsp_tile == 0) {
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+            S[j] = __dadd_rn(a, rv[j]);
+    } else {
+        int nsp = 0;
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+            nsp += rv[j] < 0.0;
+        int nspec;
+        const int rank0 =
+            block_excl_scan(nsp, sm.shi, nspec); // ends with a barrier
+        exact_values(rv, rank0, a, sm.sv, nsp_tile > kExactCap, S);
+    }
     // carry: the previous tile ends exactly at lmax = -a
     const double umax = bid > 0 ? __dadd_rn(1.0, -fm::fm_exp(-a)) : -INFINITY;
     double uv[kItems];
@@ -874,19 +940,26 @@ k_sorted_uniforms_body(const ResampleCtl *ctl, const ExactScan exu,
     for (int w = 0; w < wid; ++w)
         exc = fmax(exc, shm[w]);
     double m = fmax(umax, exc);
-    const int kb = q.kbits;
-    long long kprev = bin_floor(m, kb); // bin of u_{n-1}
+    const int kb = q.kbits, K = 1 << kb, iNN = (int)NN, in0 = (int)n0;
+    int kprev = bin_floor32(m, K); // bin of u_{n-1}
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
         m = fmax(m, uv[j]);
-        const long long n = n0 + j;
-        if (n < NN) {
-            u[n] = m;
-            const long long khi = bin_floor(m, kb);
-            bin_fill(L, kb, n == 0 ? 0 : kprev + 1, khi, n, NN);
+        uv[j] = m;
+        const int n = in0 + j;
+        if (n < iNN) {
+            const int khi = bin_floor32(m, K);
+            // (bin_fill: the bins that start at u_n)
+            for (int k = n == 0 ? 0 : kprev + 1; k <= khi && k <= K; ++k)
+                L[k] = n;
+            if (n == iNN - 1)
+                for (int k = max(khi + 1, 0); k <= K; ++k)
+                    L[k] = iNN;
             kprev = khi;
         }
     }
+    if (n0 < NN)
+        store8(u, n0, NN, uv);
 }
 
 static __global__ void __launch_bounds__(VSMC_SCAN_BOUNDS)
@@ -1092,11 +1165,6 @@ __device__ __forceinline__ double scan_weight(const W &wsrc, long long i,
     return w;
 }
 
-// A tile's values in shared memory are padded by one slot per 8, so that a
-// thread reading its kItems consecutive values meets no bank conflict.
-constexpr int kTilePad = kTile + kTile / 8;
-__device__ __forceinline__ int pad8(int l) { return l + (l >> 3); }
-
 struct SmemExactCore {
     double shd[kThreads / 32];
     SmemExactScan<kThreads / 32> et;
@@ -1161,42 +1229,6 @@ scan_weight_staged(const W &wsrc, typename W::stage_t x, double Nd,
     }
     kint = k;
     return w;
-}
-
-// Eight values of a thread to global memory (vector stores when all are
-// below N).
-template <typename T>
-__device__ __forceinline__ void store8(T *dst, long long i0, long long N,
-                                       const T (&v)[kItems])
-{
-    if (i0 + kItems <= N) {
-        if (sizeof(T) == 8) {
-            double2 *d = reinterpret_cast<double2 *>(dst + i0);
-#pragma unroll
-            for (int j = 0; j < kItems / 2; ++j) {
-                double2 q;
-                q.x = *reinterpret_cast<const double *>(&v[2 * j]);
-                q.y = *reinterpret_cast<const double *>(&v[2 * j + 1]);
-                d[j] = q;
-            }
-        } else {
-            int4 *d = reinterpret_cast<int4 *>(dst + i0);
-#pragma unroll
-            for (int j = 0; j < kItems / 4; ++j) {
-                int4 q;
-                q.x = *reinterpret_cast<const int *>(&v[4 * j]);
-                q.y = *reinterpret_cast<const int *>(&v[4 * j + 1]);
-                q.z = *reinterpret_cast<const int *>(&v[4 * j + 2]);
-                q.w = *reinterpret_cast<const int *>(&v[4 * j + 3]);
-                d[j] = q;
-            }
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < kItems; ++j)
-            if (i0 + j < N)
-                dst[i0 + j] = v[j];
-    }
 }
 
 // The mixed form's cumulative weight: a plain FP64 scan.  Each element's
