@@ -168,7 +168,7 @@ void launch_move(const MoveArgs<Real> &a, bool alone, cudaStream_t s)
         // the block scheduler hands tiles to SMs as they free, which
         // balances the rejection loops' uneven cost better than a
         // persistent grid striding over tiles (measured 5% faster at 2^24)
-        k_cv_move<Real, Init><<<a.ntiles, kMoveThreads, 0, s>>>(a);
+        launch_pdl(k_cv_move<Real, Init>, a.ntiles, kMoveThreads, s, a);
 }
 
 template <typename Real>

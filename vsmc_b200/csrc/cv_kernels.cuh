@@ -403,6 +403,7 @@ k_cv_move(MoveArgs<Real> a)
 {
     // double-buffered warp partials: one barrier per tile
     __shared__ double sh_w[2][7 * kMoveWarps];
+    pdl_enter();
     const MoveStep<Real> ms = move_step<Real, Init>(a);
     int buf = 0;
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
@@ -838,6 +839,7 @@ k_cv_finalize(FinalizeArgs a)
 {
     extern __shared__ double agg[]; // ntiles shares (when staged)
     __shared__ SmemFinal sm;
+    pdl_enter();
     k_cv_finalize_body(a, agg, kFinalSmemTiles, sm);
 }
 

@@ -516,6 +516,7 @@ __global__ void __launch_bounds__(kThreads)
 k_tile_sums(W wsrc, long long N, const ResampleCtl *ctl, double *tile_sum,
             long long *tile_k)
 {
+    pdl_enter();
     __shared__ SmemTileSums sm;
     k_tile_sums_body<W, Residual>(wsrc, N, ctl, tile_sum, tile_k, blockIdx.x,
         sm);
@@ -643,6 +644,7 @@ k_spine_weights(const double *tile_sum, const long long *tile_k,
                 double *tile_excl, long long *tile_kexcl, int ntiles,
                 long long N, EngineRef eng, ResampleCtl *ctl)
 {
+    pdl_enter();
     __shared__ SmemSpine sm;
     k_spine_weights_body<Residual, Sys>(tile_sum, tile_k, tile_excl, tile_kexcl,
         ntiles, N, eng, ctl, blockIdx.x, sm);
@@ -719,6 +721,7 @@ static __global__ void __launch_bounds__(kThreads)
 k_uniforms_stratified(EngineRef eng, const ResampleCtl *ctl, double *u,
                       int32_t *L)
 {
+    pdl_enter();
     __shared__ SmemNone sm;
     k_uniforms_stratified_body(eng, ctl, u, L,
         (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x, sm);
@@ -837,6 +840,7 @@ static __global__ void __launch_bounds__(VSMC_SCAN_BOUNDS)
 k_sorted_tile_sums(EngineRef eng, const ResampleCtl *ctl, double *tile_sum,
                    double *u)
 {
+    pdl_enter();
     __shared__ SmemSortedSums sm;
     k_sorted_tile_sums_body(eng, ctl, tile_sum, u, blockIdx.x, sm);
 }
@@ -858,6 +862,7 @@ static __global__ void __launch_bounds__(kSpineThreads)
 k_sorted_spine(const double *tile_sum, double *tile_excl,
                const ResampleCtl *ctl)
 {
+    pdl_enter();
     __shared__ SmemSpine sm;
     k_sorted_spine_body(tile_sum, tile_excl, ctl, blockIdx.x, sm);
 }
@@ -966,6 +971,7 @@ static __global__ void __launch_bounds__(VSMC_SCAN_BOUNDS)
 k_sorted_uniforms(const ResampleCtl *ctl, ExactScan exu, double *u,
                   int32_t *L)
 {
+    pdl_enter();
     __shared__ SmemSortedUniforms sm;
     k_sorted_uniforms_body(ctl, exu, u, L, blockIdx.x, sm);
 }
@@ -976,6 +982,7 @@ static __global__ void __launch_bounds__(VSMC_SCAN_BOUNDS)
 k_spec_tile_sums(EngineRef eng, const ResampleCtl *ctl, long long N,
                  double *tile_sum, double *u)
 {
+    pdl_enter();
     __shared__ SmemSortedSums sm;
     k_sorted_tile_sums_body(eng, ctl, tile_sum, u, blockIdx.x, sm, N);
 }
@@ -984,6 +991,7 @@ static __global__ void __launch_bounds__(kSpineThreads)
 k_spec_spine(const double *tile_sum, double *tile_excl,
              const ResampleCtl *ctl, long long N)
 {
+    pdl_enter();
     __shared__ SmemSpine sm;
     k_sorted_spine_body(tile_sum, tile_excl, ctl, blockIdx.x, sm, N);
 }
@@ -992,6 +1000,7 @@ static __global__ void __launch_bounds__(VSMC_SCAN_BOUNDS)
 k_spec_uniforms(const ResampleCtl *ctl, long long N, ExactScan exu, double *u,
                 int32_t *L)
 {
+    pdl_enter();
     __shared__ SmemSortedUniforms sm;
     k_sorted_uniforms_body(ctl, exu, u, L, blockIdx.x, sm, N);
 }
@@ -1000,12 +1009,14 @@ k_spec_uniforms(const ResampleCtl *ctl, long long N, ExactScan exu, double *u,
 // after the three kernels above, which all test the same condition).
 static __global__ void k_spec_commit(ResampleCtl *ctl)
 {
+    pdl_enter();
     ctl->spec_offset = ctl->offset;
 }
 
 // No sequence held (a fresh workspace).
 static __global__ void k_spec_invalidate(ResampleCtl *ctl)
 {
+    pdl_enter();
     ctl->spec_offset = ~0ull;
 }
 
@@ -1478,6 +1489,7 @@ __global__ void __launch_bounds__(kThreads, VSMC_EXACT_STAGE_MIN_BLOCKS)
 k_exact_tiles(W wsrc, long long N, const ResampleCtl *ctl,
               const double *tile_excl, ExactScan ex)
 {
+    pdl_enter();
     typedef typename W::stage_t S;
     __shared__ SmemExactStage sm;
     if (!wsrc.active(ctl))
@@ -1849,6 +1861,7 @@ template <typename W, bool Residual, bool Raw = false>
 __global__ void __launch_bounds__(kSpineThreads)
 k_exact_spine(W wsrc, long long N, ResampleCtl *ctl, int nt, ExactScan ex)
 {
+    pdl_enter();
     __shared__ SmemExactSpine sm;
     k_exact_spine_body<W, Residual, Raw>(wsrc, N, ctl, nt, ex, sm);
 }
@@ -2127,6 +2140,7 @@ k_invert(W wsrc, long long N, ResampleCtl *ctl, const double *tile_excl,
          int32_t *sinc_local, int32_t *tile_zeros, int32_t *tile_sinc_last,
          ExactScan ex)
 {
+    pdl_enter();
     __shared__ SmemInvert<Residual> sm;
     k_invert_body<W, Residual, Sys>(wsrc, N, ctl, tile_excl, tile_kexcl, u, n_u,
         L, rep_out, copy_from, sinc_local, tile_zeros, tile_sinc_last, ex,
@@ -2227,6 +2241,7 @@ k_zero_spine(const int32_t *tile_zeros, const int32_t *tile_sinc_last,
              int32_t *zexcl, int32_t *tfirst, int32_t *tlast, int ntiles,
              ResampleCtl *ctl)
 {
+    pdl_enter();
     __shared__ SmemZeroSpine sm;
     k_zero_spine_body(tile_zeros, tile_sinc_last, zexcl, tfirst, tlast, ntiles,
         ctl, blockIdx.x, sm);
@@ -2351,6 +2366,7 @@ k_cfrp_fill(long long N, ResampleCtl *ctl, const int32_t *sinc_local,
             const int32_t *zexcl, const int32_t *tfirst, const int32_t *tlast,
             int32_t *copy_from)
 {
+    pdl_enter();
     __shared__ SmemFill sm;
     k_cfrp_fill_body(N, ctl, sinc_local, zexcl, tfirst, tlast, copy_from,
         blockIdx.x, sm);
@@ -2359,6 +2375,7 @@ k_cfrp_fill(long long N, ResampleCtl *ctl, const int32_t *sinc_local,
 // Finalise the engine position.
 static __global__ void k_resample_done(ResampleCtl *ctl)
 {
+    pdl_enter();
     if (!ctl->active)
         return;
     ctl->offset += ctl->words;
@@ -2369,6 +2386,7 @@ static __global__ void k_resample_done(ResampleCtl *ctl)
 static __global__ void __launch_bounds__(kThreads)
 k_tile_max(const double *u, long long n, double *tile_max)
 {
+    pdl_enter();
     __shared__ double sh[kThreads / 32];
     const long long base = (long long)blockIdx.x * kTile;
     double m = -INFINITY;
@@ -2393,6 +2411,7 @@ static __global__ void __launch_bounds__(kThreads)
 k_apply_max(const double *u, long long n, const double *tile_max, double *out,
             const ResampleCtl *ctl, int32_t *L)
 {
+    pdl_enter();
     __shared__ double carry_sh;
     __shared__ double shm[kThreads];
     if (threadIdx.x == 0) {
@@ -2594,6 +2613,37 @@ inline int resample_launches(int scheme, bool parity, bool exact_norm = false,
     return n;
 }
 
+// Launches a kernel whose start may overlap the end of the stream's previous
+// kernel (programmatic dependent launch).  Every kernel launched so begins
+// with pdl_enter(): it reads and writes nothing before the previous kernel
+// is done, so only the launch latency and the start of its CTAs overlap.
+// `early` false: an ordinary launch (the first after a wait for another
+// stream's event).
+template <typename... P, typename... A>
+inline void launch_early(bool early, void (*k)(P...), unsigned grid,
+                         unsigned block, size_t smem, cudaStream_t s,
+                         A... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+
+template <typename... P, typename... A>
+inline void launch_pdl(void (*k)(P...), unsigned grid, unsigned block,
+                       cudaStream_t s, A... args)
+{
+    launch_early(true, k, grid, block, 0, s, args...);
+}
+
 // Launch the scheme-specific part of a resampling (everything after the
 // weight tile sums and spine when `spine_done`).  `u_given` (parity mode)
 // replaces the device-drawn U01 sequence.
@@ -2628,76 +2678,74 @@ inline void launch_resample_core(int scheme, W wsrc, long long N,
     W wx = wsrc;
     if (W::kExactNorm) {
         if (!spine_done) {
-            k_tile_sums<W, false><<<nt, kThreads, 0, s>>>(
-                wsrc, N, ws.ctl, ws.tile_sum, nullptr);
+            launch_pdl(k_tile_sums<W, false>, nt, kThreads, s, wsrc, N, ws.ctl,
+                       ws.tile_sum, nullptr);
             if (sys)
-                k_spine_weights<false, true><<<1, spt, 0, s>>>(
-                    ws.tile_sum, nullptr, ws.tile_excl, nullptr, nt, N, eng,
-                    ws.ctl);
+                launch_pdl(k_spine_weights<false, true>, 1, spt, s,
+                           ws.tile_sum, nullptr, ws.tile_excl, nullptr, nt, N,
+                           eng, ws.ctl);
             else
-                k_spine_weights<false, false><<<1, spt, 0, s>>>(
-                    ws.tile_sum, nullptr, ws.tile_excl, nullptr, nt, N, eng,
-                    ws.ctl);
+                launch_pdl(k_spine_weights<false, false>, 1, spt, s,
+                           ws.tile_sum, nullptr, ws.tile_excl, nullptr, nt, N,
+                           eng, ws.ctl);
         }
-        k_exact_tiles<W, false, true><<<exact_grid(nt), kThreads, 0, s>>>(
-            wsrc, N, ws.ctl, ws.tile_excl, ws.ex);
-        k_exact_spine<W, false, true><<<1, spt, 0, s>>>(
-            wsrc, N, ws.ctl, nt, ws.ex);
+        launch_early(!sorted_ready, k_exact_tiles<W, false, true>,
+                     exact_grid(nt), kThreads, 0, s, wsrc, N, ws.ctl,
+                     ws.tile_excl, ws.ex);
+        launch_pdl(k_exact_spine<W, false, true>, 1, spt, s, wsrc, N, ws.ctl,
+                   nt, ws.ex);
         wx = with_exact_coeff(wsrc, &ws.ctl->coeff_w, ws.ex.rec);
     }
     if (residual) {
-        k_tile_sums<W, true><<<nt, kThreads, 0, s>>>(wx, N, ws.ctl,
-                                                    ws.tile_sum, ws.tile_k);
+        launch_pdl(k_tile_sums<W, true>, nt, kThreads, s, wx, N, ws.ctl,
+                   ws.tile_sum, ws.tile_k);
         if (sys)
-            k_spine_weights<true, true><<<1, spt, 0, s>>>(
-                ws.tile_sum, ws.tile_k, ws.tile_excl, ws.tile_kexcl, nt, N,
-                eng, ws.ctl);
+            launch_pdl(k_spine_weights<true, true>, 1, spt, s, ws.tile_sum,
+                       ws.tile_k, ws.tile_excl, ws.tile_kexcl, nt, N, eng,
+                       ws.ctl);
         else
-            k_spine_weights<true, false><<<1, spt, 0, s>>>(
-                ws.tile_sum, ws.tile_k, ws.tile_excl, ws.tile_kexcl, nt, N,
-                eng, ws.ctl);
+            launch_pdl(k_spine_weights<true, false>, 1, spt, s, ws.tile_sum,
+                       ws.tile_k, ws.tile_excl, ws.tile_kexcl, nt, N, eng,
+                       ws.ctl);
     } else if (!spine_done && !W::kExactNorm) {
-        k_tile_sums<W, false><<<nt, kThreads, 0, s>>>(wx, N, ws.ctl,
-                                                     ws.tile_sum, nullptr);
+        launch_pdl(k_tile_sums<W, false>, nt, kThreads, s, wx, N, ws.ctl,
+                   ws.tile_sum, nullptr);
         if (sys)
-            k_spine_weights<false, true><<<1, spt, 0, s>>>(
-                ws.tile_sum, nullptr, ws.tile_excl, nullptr, nt, N, eng,
-                ws.ctl);
+            launch_pdl(k_spine_weights<false, true>, 1, spt, s, ws.tile_sum,
+                       nullptr, ws.tile_excl, nullptr, nt, N, eng, ws.ctl);
         else
-            k_spine_weights<false, false><<<1, spt, 0, s>>>(
-                ws.tile_sum, nullptr, ws.tile_excl, nullptr, nt, N, eng,
-                ws.ctl);
+            launch_pdl(k_spine_weights<false, false>, 1, spt, s, ws.tile_sum,
+                       nullptr, ws.tile_excl, nullptr, nt, N, eng, ws.ctl);
     }
     const double *u = ws.u;
     long long n_u = Nu;
     if (u_given != nullptr) {
         const int ntu = (int)((n_given + kTile - 1) / kTile);
         if (n_given > 0) {
-            k_tile_max<<<ntu, kThreads, 0, s>>>(u_given, n_given,
-                                                ws.u_tile_sum);
-            k_apply_max<<<ntu, kThreads, 0, s>>>(u_given, n_given,
-                                                 ws.u_tile_sum, ws.u, ws.ctl,
-                                                 ws.bins);
+            launch_pdl(k_tile_max, ntu, kThreads, s, u_given, n_given,
+                       ws.u_tile_sum);
+            launch_pdl(k_apply_max, ntu, kThreads, s, u_given, n_given,
+                       ws.u_tile_sum, ws.u, ws.ctl, ws.bins);
         }
         n_u = n_given;
     } else if (strat) {
         const long long blocks = Nu / 4 + 2;
-        k_uniforms_stratified<<<(unsigned)((blocks + kThreads - 1) / kThreads),
-                                kThreads, 0, s>>>(eng, ws.ctl, ws.u,
-                                                  ws.bins);
+        launch_pdl(k_uniforms_stratified,
+                   (unsigned)((blocks + kThreads - 1) / kThreads), kThreads, s,
+                   eng, ws.ctl, ws.u, ws.bins);
     } else if (!sys && !sorted_ready) {
-        k_sorted_tile_sums<<<ntu_dev, kThreads, 0, s>>>(eng, ws.ctl,
-                                                        ws.u_tile_sum, ws.u);
-        k_sorted_spine<<<1, sptu, 0, s>>>(ws.u_tile_sum,
-                                                   ws.u_tile_excl, ws.ctl);
+        launch_pdl(k_sorted_tile_sums, ntu_dev, kThreads, s, eng, ws.ctl,
+                   ws.u_tile_sum, ws.u);
+        launch_pdl(k_sorted_spine, 1, sptu, s, ws.u_tile_sum, ws.u_tile_excl,
+                   ws.ctl);
         // lmax exactly: the exact scan of the negated terms
         const TermsNeg tn{ws.u, 0};
-        k_exact_tiles<TermsNeg, false><<<exact_grid(ntu_dev), kThreads, 0, s>>>(
-            tn, Nu, ws.ctl, ws.u_tile_excl, ws.exu);
-        k_exact_spine<TermsNeg, false><<<1, sptu, 0, s>>>(
-            tn, Nu, ws.ctl, ntu_dev, ws.exu);
-        k_sorted_uniforms<<<ntu_dev, kThreads, 0, s>>>(ws.ctl, ws.exu, ws.u,
-                                                       ws.bins);
+        launch_pdl(k_exact_tiles<TermsNeg, false>, exact_grid(ntu_dev),
+                   kThreads, s, tn, Nu, ws.ctl, ws.u_tile_excl, ws.exu);
+        launch_pdl(k_exact_spine<TermsNeg, false>, 1, sptu, s, tn, Nu, ws.ctl,
+                   ntu_dev, ws.exu);
+        launch_pdl(k_sorted_uniforms, ntu_dev, kThreads, s, ws.ctl, ws.exu,
+                   ws.u, ws.bins);
     }
     const long long *kex = residual ? ws.tile_kexcl : nullptr;
     // the reference's sequential cumulative weight, exactly (for the
@@ -2705,23 +2753,24 @@ inline void launch_resample_core(int scheme, W wsrc, long long N,
     // scales them)
     if (residual) {
         if (!W::kApprox) {
-            k_exact_tiles<W, true, true><<<exact_grid(nt), kThreads, 0, s>>>(
-                wx, N, ws.ctl, ws.tile_excl, ws.ex);
-            k_exact_spine<W, true, true><<<1, spt, 0, s>>>(
-                wx, N, ws.ctl, nt, ws.ex);
+            launch_pdl(k_exact_tiles<W, true, true>, exact_grid(nt), kThreads,
+                       s, wx, N, ws.ctl, ws.tile_excl, ws.ex);
+            launch_pdl(k_exact_spine<W, true, true>, 1, spt, s, wx, N, ws.ctl,
+                       nt, ws.ex);
         }
-        k_exact_tiles<W, true><<<exact_grid(nt), kThreads, 0, s>>>(wx, N, ws.ctl,
-                                                       ws.tile_excl, ws.ex);
-        k_exact_spine<W, true><<<1, spt, 0, s>>>(wx, N, ws.ctl,
-                                                           nt, ws.ex);
+        launch_pdl(k_exact_tiles<W, true>, exact_grid(nt), kThreads, s, wx, N,
+                   ws.ctl, ws.tile_excl, ws.ex);
+        launch_pdl(k_exact_spine<W, true>, 1, spt, s, wx, N, ws.ctl, nt,
+                   ws.ex);
     } else {
-        k_exact_tiles<W, false><<<exact_grid(nt), kThreads, 0, s>>>(wx, N, ws.ctl,
-                                                        ws.tile_excl, ws.ex);
-        k_exact_spine<W, false><<<1, spt, 0, s>>>(wx, N, ws.ctl,
-                                                            nt, ws.ex);
+        launch_early(W::kExactNorm || !sorted_ready, k_exact_tiles<W, false>,
+                     exact_grid(nt), kThreads, 0, s, wx, N, ws.ctl,
+                     ws.tile_excl, ws.ex);
+        launch_pdl(k_exact_spine<W, false>, 1, spt, s, wx, N, ws.ctl, nt,
+                   ws.ex);
     }
 #define VSMC_INVERT(R, S)                                                     \
-    k_invert<W, R, S><<<nt, kThreads, 0, s>>>(                                \
+    launch_pdl(k_invert<W, R, S>, nt, kThreads, s,                            \
         wx, N, ws.ctl, ws.tile_excl, kex, u, n_u, ws.bins, rep_out,        \
         copy_from, ws.sinc, ws.tile_zeros, ws.tile_sinc_last, ws.ex)
     if (residual && sys)
@@ -2735,13 +2784,12 @@ inline void launch_resample_core(int scheme, W wsrc, long long N,
 #undef VSMC_INVERT
     if (cfrp) {
         // the spine kernel also advances the engine position
-        k_zero_spine<<<1, spt, 0, s>>>(
-            ws.tile_zeros, ws.tile_sinc_last, ws.zexcl, ws.tfirst, ws.tlast,
-            nt, ws.ctl);
-        k_cfrp_fill<<<nt, kThreads, 0, s>>>(N, ws.ctl, ws.sinc, ws.zexcl,
-                                            ws.tfirst, ws.tlast, copy_from);
+        launch_pdl(k_zero_spine, 1, spt, s, ws.tile_zeros, ws.tile_sinc_last,
+                   ws.zexcl, ws.tfirst, ws.tlast, nt, ws.ctl);
+        launch_pdl(k_cfrp_fill, nt, kThreads, s, N, ws.ctl, ws.sinc, ws.zexcl,
+                   ws.tfirst, ws.tlast, copy_from);
     } else {
-        k_resample_done<<<1, 1, 0, s>>>(ws.ctl);
+        launch_pdl(k_resample_done, 1, 1, s, ws.ctl);
     }
 }
 
@@ -2754,6 +2802,7 @@ inline void launch_resample_core(int scheme, W wsrc, long long N,
 static __global__ void __launch_bounds__(kThreads)
 k_rep_tile_sums(const int32_t *rep, long long M, long long *tile_sum)
 {
+    pdl_enter();
     __shared__ long long sh[kThreads / 32];
     const long long base = (long long)blockIdx.x * kTile;
     long long v = 0;
@@ -2772,6 +2821,7 @@ k_rep_tile_sums(const int32_t *rep, long long M, long long *tile_sum)
 static __global__ void __launch_bounds__(kSpineThreads)
 k_rep_spine(const long long *tile_sum, long long *tile_excl, int ntiles)
 {
+    pdl_enter();
     __shared__ long long sh[kSpineThreads / 32];
     spine_scan_ll(tile_sum, tile_excl, ntiles, sh);
 }
@@ -2780,6 +2830,7 @@ static __global__ void __launch_bounds__(kThreads)
 k_rep_prefix(const int32_t *rep, long long M, const long long *tile_excl,
              int32_t *incl)
 {
+    pdl_enter();
     __shared__ long long sh[kThreads / 32];
     const long long base = (long long)blockIdx.x * kTile;
     const long long i0 = base + (long long)threadIdx.x * kItems;
@@ -2803,6 +2854,7 @@ k_rep_prefix(const int32_t *rep, long long M, const long long *tile_excl,
 static __global__ void k_expand_fill(const int32_t *incl, long long M,
                                      long long N, int32_t *copy_from)
 {
+    pdl_enter();
     const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= N)
         return;
@@ -2823,11 +2875,11 @@ inline void launch_expand(const int32_t *rep, long long M, long long N,
                           cudaStream_t s)
 {
     const int nt = resample_ntiles(M);
-    k_rep_tile_sums<<<nt, kThreads, 0, s>>>(rep, M, ws.tile_k);
-    k_rep_spine<<<1, kSpineThreads, 0, s>>>(ws.tile_k, ws.tile_kexcl, nt);
-    k_rep_prefix<<<nt, kThreads, 0, s>>>(rep, M, ws.tile_kexcl, ws.sinc);
-    k_expand_fill<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(ws.sinc, M, N,
-                                                               copy_from);
+    launch_pdl(k_rep_tile_sums, nt, kThreads, s, rep, M, ws.tile_k);
+    launch_pdl(k_rep_spine, 1, kSpineThreads, s, ws.tile_k, ws.tile_kexcl, nt);
+    launch_pdl(k_rep_prefix, nt, kThreads, s, rep, M, ws.tile_kexcl, ws.sinc);
+    launch_pdl(k_expand_fill, (unsigned)((N + 255) / 256), 256, s, ws.sinc, M,
+               N, copy_from);
 }
 
 // The speculative Multinomial sequence for the next resampling (see
@@ -2836,18 +2888,19 @@ inline void launch_spec_sorted(long long N, const EngineRef &eng,
                                ResampleWorkspace &ws, cudaStream_t s)
 {
     const int nt = resample_ntiles(N);
-    k_spec_tile_sums<<<nt, kThreads, 0, s>>>(eng, ws.ctl, N, ws.u_tile_sum,
-                                             ws.u);
-    k_spec_spine<<<1, kSpineThreads, 0, s>>>(ws.u_tile_sum, ws.u_tile_excl,
-                                             ws.ctl, N);
+    // (after a wait for the filter's stream)
+    launch_early(false, k_spec_tile_sums, nt, kThreads, 0, s, eng, ws.ctl, N,
+                 ws.u_tile_sum, ws.u);
+    launch_pdl(k_spec_spine, 1, kSpineThreads, s, ws.u_tile_sum,
+               ws.u_tile_excl, ws.ctl, N);
     const TermsNeg tn{ws.u, N};
-    k_exact_tiles<TermsNeg, false><<<exact_grid(nt), kThreads, 0, s>>>(
-        tn, N, ws.ctl, ws.u_tile_excl, ws.exu);
-    k_exact_spine<TermsNeg, false><<<1, kSpineThreads, 0, s>>>(
-        tn, N, ws.ctl, nt, ws.exu);
-    k_spec_uniforms<<<nt, kThreads, 0, s>>>(ws.ctl, N, ws.exu, ws.u,
-                                            ws.bins);
-    k_spec_commit<<<1, 1, 0, s>>>(ws.ctl);
+    launch_pdl(k_exact_tiles<TermsNeg, false>, exact_grid(nt), kThreads, s, tn,
+               N, ws.ctl, ws.u_tile_excl, ws.exu);
+    launch_pdl(k_exact_spine<TermsNeg, false>, 1, kSpineThreads, s, tn, N,
+               ws.ctl, nt, ws.exu);
+    launch_pdl(k_spec_uniforms, nt, kThreads, s, ws.ctl, N, ws.exu, ws.u,
+               ws.bins);
+    launch_pdl(k_spec_commit, 1, 1, s, ws.ctl);
 }
 
 } // namespace vsmc_b200

@@ -878,7 +878,8 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             // the residuals' sequential sum
             const double a0 = act ? rc_before(sm.sums, tile) : 0.0;
             if (act)
-                rc_classify(base, N, w, a0, pre, ExactMargin<W>::rel, th, g, g.scan[kRcB], a.rec, rw);
+                rc_classify(base, N, w, a0, pre, ExactMargin<W>::rel, th, g,
+                            g.scan[kRcB], a.rec, rw);
             cl.sync();
             if (U == kRcSorted) {
                 gather_usums(utiles());
@@ -1531,7 +1532,7 @@ inline int launch_finish(int scheme, const FinalizeArgs &fa, const W &w,
     const size_t smem = fa.ntiles <= kFinalSmemTiles
                             ? (size_t)fa.ntiles * sizeof(double)
                             : 0;
-    k_cv_finalize<<<1, kFinalThreads, smem, s>>>(fa);
+    launch_early(true, k_cv_finalize, 1, kFinalThreads, smem, s, fa);
     if (!resample)
         return 1;
     if (sorted_ready)

@@ -109,6 +109,14 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The start of a kernel that may be launched before its predecessor ends:
+// its successor may start too, then it waits.
+__device__ __forceinline__ void pdl_enter()
+{
+    pdl_launch();
+    pdl_wait();
+}
+
 // --------------------------------------------------------- reductions ------
 __device__ __forceinline__ double warp_sum(double v)
 {
