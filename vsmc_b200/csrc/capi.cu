@@ -2,7 +2,7 @@
 // RNG word streams, the device WeightSet update, the device resampler and
 // the particle gather.  The CV filter's entry points are in cv_filter.cu.
 #include "call_scratch.hpp"
-#include "resample_cluster.cuh"
+#include "resample_launch.cuh"
 #include "weights.cuh"
 
 #include <cstdio>
@@ -506,7 +506,7 @@ int vsmc_cuda_resample_mn(int scheme, uint64_t M, uint64_t N,
                         (long long)n_uniforms, rep, cf_scratch, s,
                         /*cfrp=*/false);
     if (copy_from != nullptr)
-        launch_expand(rep, (long long)M, (long long)N, ws, copy_from, s);
+        launch_resample_expand(rep, (long long)M, (long long)N, ws, copy_from, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_mn: launch");

@@ -13,8 +13,7 @@
 // monitor, resampling decision and the weight spine) + the resampling
 // kernels of resample.cuh, which return at once when the step does not
 // resample.  No host round trip happens inside a step.
-#include "cv_kernels.cuh"
-#include "resample_cluster.cuh"
+#include "resample_launch.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -110,7 +109,7 @@ void enqueue_sequence(vsmc_cuda_cv_filter *f)
 {
     cudaEventRecord(f->ev_pos, f->stream);
     cudaStreamWaitEvent(f->side, f->ev_pos, 0);
-    launch_spec_sorted((long long)f->cfg.N, f->eng, f->rws, f->side);
+    launch_sequence((long long)f->cfg.N, f->eng, f->rws, f->side);
     cudaEventRecord(f->ev_seq, f->side);
     f->seq_pending = true;
     f->launches += 6;
@@ -253,14 +252,13 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
     WeightsFromLog<Real> w;
     w.lw = static_cast<const Real *>(f->lw);
     w.stats = &f->ctl->lw_max;
-    const auto wait = [&] { cudaStreamWaitEvent(s, f->ev_seq, 0); };
     if (f->rep_cf != nullptr) {
         // comparing: the step's own resampling of its own weights goes into
         // the record row; the engine advances by the words it drew
         f->launches += launch_finish(
             c.scheme, fa, w, f->rws,
             compare ? f->rec_cf + (size_t)f->iter * c.N : f->copy_from,
-            compare, false, [] {}, s);
+            compare, nullptr, s);
         // replay: the recorded ancestry of this step (used only if the
         // recorded decision was to resample)
         cudaMemcpyAsync(f->copy_from, f->rep_cf + (size_t)f->iter * c.N,
@@ -268,7 +266,8 @@ void launch_step(vsmc_cuda_cv_filter *f, bool init)
     } else {
         // (a speculative sequence's launches are counted on the side)
         f->launches += launch_finish(c.scheme, fa, w, f->rws, f->copy_from,
-                                     true, speculate, wait, s);
+                                     true, speculate ? f->ev_seq : nullptr,
+                                     s);
         if (speculate)
             enqueue_sequence(f); // for the next resampling
     }
@@ -442,9 +441,6 @@ int vsmc_cuda_cv_create(const vsmc_cuda_cv_config *cfg, void *stream,
     f->seq_pending = false;
     // resample engine: Threefry4x64 seeded seed+2 (Seed::get twice)
     f->eng = cv_resample_engine(cfg->seed);
-    cudaFuncSetAttribute(k_cv_finalize,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kFinalSmemTiles * (int)sizeof(double));
     e = cudaMemsetAsync(f->mem, 0, f->bytes, f->stream);
     // (a filter that resamples in one cluster draws its sequence there)
     if (e == cudaSuccess && cfg->scheme == VSMC_CUDA_MULTINOMIAL &&

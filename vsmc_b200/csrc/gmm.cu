@@ -38,8 +38,7 @@
 // bound by the FP64 pipe, 60% on average, 70% on the SMs with 16 warps),
 // mixed 2.4 -> 1.73 (no bounds test in whole rounds; bound by the
 // special-function unit, 72%).
-#include "cv_kernels.cuh"
-#include "resample_cluster.cuh"
+#include "resample_launch.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1381,9 +1380,6 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
     }
     set_smem_attrs<true>(gmm_smem_bytes((int)n, true));
     set_smem_attrs<false>(gmm_smem_bytes((int)n, false));
-    cudaFuncSetAttribute(k_cv_finalize,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kFinalSmemTiles * (int)sizeof(double));
     *out = g;
     return VSMC_CUDA_OK;
 }
@@ -1502,7 +1498,7 @@ int vsmc_cuda_gmm_iterate(vsmc_cuda_gmm *g, uint64_t num)
         w.lw = g->lw;
         w.stats = &g->ctl->lw_max;
         g->launches += launch_finish(scheme, fa, w, g->rws, g->copy_from,
-                                     true, false, [] {}, s);
+                                     true, nullptr, s);
         cudaEvent_t *ev = nullptr;
         if (g->timing) {
             if (g->ev_used + 2 > g->ev.size())

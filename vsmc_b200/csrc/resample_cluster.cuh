@@ -25,15 +25,12 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 
-#include "cv_kernels.cuh"
+#include "resample_launch.cuh"
 
 namespace vsmc_b200 {
 
 namespace cg = cooperative_groups;
 
-constexpr int kRcMaxCtas = 16;  // CTAs of a cluster (above 8: non-portable)
-constexpr int kRcGroups = 2;    // groups (tiles) of a CTA, at most
-constexpr int kRcMaxTiles = kRcMaxCtas * kRcGroups;
 constexpr int kRcStage = 256;   // specials of a scan staged per CTA
 
 // How a resampling draws its U01 sequence.
@@ -1400,14 +1397,6 @@ inline cudaError_t rc_launch(K k, RcShape shape, int clusters, bool early,
     return cudaLaunchKernelEx(&c, k, args...);
 }
 
-// Whether a resampling of N weights to Nout children (0: N) runs in one
-// cluster: its weights and its uniforms must fit in kRcMaxTiles tiles.
-inline bool rc_fits(long long N, long long Nout)
-{
-    const long long n = Nout > N ? Nout : N;
-    return resample_ntiles(n) <= kRcMaxTiles;
-}
-
 // The scheme's instance: f(residual, sequence) with compile-time constants.
 template <typename F>
 inline void rc_scheme(int scheme, F f)
@@ -1458,17 +1447,12 @@ inline RcArgs rc_args(long long N, const EngineRef &eng,
     return a;
 }
 
-// A resampling of given weights: one cluster where it fits, the launch
-// sequence of resample.cuh otherwise (and for caller-supplied uniforms).
-// `h` holds the call's initial control block; `slot` is a call's pinned
-// memory, or nullptr.  Returns whether the result is in *slot (else in the
-// workspace's control block) once the stream gets there.
-inline bool launch_resample(int scheme, WeightsGiven w, long long N,
-                            const EngineRef &eng, ResampleWorkspace &ws,
-                            const ResampleCtl &h, ResampleCtl *slot,
-                            const double *u_given, long long n_given,
-                            int32_t *rep_out, int32_t *copy_from,
-                            cudaStream_t s, bool cfrp = true)
+bool launch_resample(int scheme, WeightsGiven w, long long N,
+                     const EngineRef &eng, ResampleWorkspace &ws,
+                     const ResampleCtl &h, ResampleCtl *slot,
+                     const double *u_given, long long n_given,
+                     int32_t *rep_out, int32_t *copy_from, cudaStream_t s,
+                     bool cfrp)
 {
     if (u_given != nullptr || !rc_fits(N, h.Nout)) {
         const ResampleCtl *src = &h;
@@ -1502,24 +1486,21 @@ inline bool launch_resample(int scheme, WeightsGiven w, long long N,
     return slot != nullptr;
 }
 
-// A filter step after its tile statistics: the finalisation (fa) and the
-// resampling of the weights w into copy_from.  One cluster where it fits;
-// else k_cv_finalize and the launch sequence (sorted_ready: the sorted
-// sequence is drawn elsewhere, `wait` orders the stream after it).
-// Returns the kernels launched (the caller's counter).
-template <typename W, typename Wait>
-inline int launch_finish(int scheme, const FinalizeArgs &fa, const W &w,
-                         ResampleWorkspace &ws, int32_t *copy_from,
-                         bool resample, bool sorted_ready, Wait wait,
-                         cudaStream_t s)
+// Dynamic shared memory that a kernel may have without asking for more.
+constexpr size_t kDefaultSmem = 48 << 10;
+
+template <typename W>
+inline int launch_finish_t(int scheme, const FinalizeArgs &fa, const W &w,
+                           ResampleWorkspace &ws, int32_t *copy_from,
+                           bool resample, cudaEvent_t seq, cudaStream_t s)
 {
     const long long N = fa.N;
     if (rc_fits(N, 0)) {
         const RcArgs a = rc_args(N, fa.eng, ws, nullptr, copy_from, true);
         const RcShape sh = rc_shape(fa.ntiles);
-        rc_scheme(scheme, [&](auto res, auto seq) {
+        rc_scheme(scheme, [&](auto res, auto u) {
             constexpr bool Re = decltype(res)::value;
-            constexpr int U = decltype(seq)::value;
+            constexpr int U = decltype(u)::value;
             if (sh.r == 8)
                 rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, true, s, fa, w,
                           a);
@@ -1532,17 +1513,21 @@ inline int launch_finish(int scheme, const FinalizeArgs &fa, const W &w,
     const size_t smem = fa.ntiles <= kFinalSmemTiles
                             ? (size_t)fa.ntiles * sizeof(double)
                             : 0;
+    if (smem > kDefaultSmem)
+        cudaFuncSetAttribute(k_cv_finalize,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kFinalSmemTiles * (int)sizeof(double));
     launch_early(true, k_cv_finalize, 1, kFinalThreads, smem, s, fa);
     if (!resample)
         return 1;
-    if (sorted_ready)
-        wait();
+    const bool ready = seq != nullptr;
+    if (ready)
+        cudaStreamWaitEvent(s, seq, 0);
     launch_resample_core(scheme, w, N, fa.eng, ws, nullptr, 0,
-                         /*spine_done=*/true, nullptr, copy_from, s,
-                         sorted_ready);
+                         /*spine_done=*/true, nullptr, copy_from, s, ready);
     return 1 +
            resample_launches(scheme, false, W::kExactNorm, W::kApprox) -
-           (sorted_ready ? 5 : 0);
+           (ready ? 5 : 0);
 }
 
 } // namespace vsmc_b200

@@ -17,7 +17,7 @@
 // so nothing stale is used, but two calls that overlap on the GPU (for
 // example on two streams) race on the same memory and must be serialised by
 // the caller.
-#include "resample_cluster.cuh"
+#include "resample_launch.cuh"
 
 #include <cstring>
 #include <mutex>

@@ -13,8 +13,7 @@
 // statistics (TileStats, one per kTile particles) and gather through
 // copy_from when the previous step resampled; vsmc_cuda_smc_finish_step then
 // runs the same finalize and resampling kernels as the built-in filter.
-#include "cv_kernels.cuh"
-#include "resample_cluster.cuh"
+#include "resample_launch.cuh"
 
 #include <cstring>
 #include <new>
@@ -170,9 +169,6 @@ int vsmc_cuda_smc_create(uint64_t N, uint64_t T_max, int scheme,
         s->eng.ctr.v[i] = 0;
     }
     s->eng.key.v[0] = resample_seed;
-    cudaFuncSetAttribute(k_cv_finalize,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kFinalSmemTiles * (int)sizeof(double));
     e = cudaMemsetAsync(s->mem, 0, s->bytes, s->stream);
     if (e == cudaSuccess) {
         k_smc_reset<<<1, 1, 0, s->stream>>>(s->ctl, s->rws.ctl);
@@ -271,7 +267,7 @@ int vsmc_cuda_smc_finish_step(vsmc_cuda_smc *s)
     w.lw = s->lw;
     w.stats = &s->ctl->lw_max;
     s->launches += launch_finish(sch, fa, w, s->rws, s->copy_from, true,
-                                 false, [] {}, s->stream);
+                                 nullptr, s->stream);
     ++s->iter;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VSMC_CUDA_OK
