@@ -122,6 +122,7 @@ template <typename Real, int MinBlocks>
 __global__ void __launch_bounds__(kMoveThreads, MinBlocks * 256 / kMoveThreads)
 kb_move(const BatchSlot *slots, const TileRef *map, CVParam p)
 {
+    pdl_enter();
     __shared__ double sh_w[7 * kMoveWarps];
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
@@ -140,6 +141,7 @@ constexpr int kBatchAgg = 2048; // tile shares staged in shared memory
 static __global__ void __launch_bounds__(kFinalThreads)
 kb_finalize(const BatchSlot *slots, const int32_t *work, BatchConst c)
 {
+    pdl_enter();
     __shared__ SmemFinal sm;
     __shared__ double agg[kBatchAgg];
     const BatchSlot &b = slots[work[blockIdx.x]];
@@ -173,6 +175,7 @@ template <typename Real, bool Residual>
 __global__ void __launch_bounds__(kThreads)
 kb_tile_sums(const BatchSlot *slots, const TileRef *map)
 {
+    pdl_enter();
     __shared__ SmemTileSums sm;
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
@@ -185,6 +188,7 @@ template <bool Residual, bool Sys>
 __global__ void __launch_bounds__(kSpineThreads)
 kb_spine_weights(const BatchSlot *slots, const int32_t *work)
 {
+    pdl_enter();
     __shared__ SmemSpine sm;
     const BatchSlot &b = slots[work[blockIdx.x]];
     k_spine_weights_body<Residual, Sys>(
@@ -199,6 +203,7 @@ kb_spine_weights(const BatchSlot *slots, const int32_t *work)
 static __global__ void __launch_bounds__(kThreads)
 kb_uniforms_stratified(const BatchSlot *slots, const TileRef *map)
 {
+    pdl_enter();
     __shared__ SmemNone sm;
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
@@ -214,6 +219,7 @@ kb_uniforms_stratified(const BatchSlot *slots, const TileRef *map)
 static __global__ void __launch_bounds__(kThreads)
 kb_sorted_tile_sums(const BatchSlot *slots, const TileRef *map)
 {
+    pdl_enter();
     __shared__ SmemSortedSums sm;
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
@@ -224,6 +230,7 @@ kb_sorted_tile_sums(const BatchSlot *slots, const TileRef *map)
 static __global__ void __launch_bounds__(kSpineThreads)
 kb_sorted_spine(const BatchSlot *slots, const int32_t *work)
 {
+    pdl_enter();
     __shared__ SmemSpine sm;
     const BatchSlot &b = slots[work[blockIdx.x]];
     k_sorted_spine_body(b.rws.u_tile_sum, b.rws.u_tile_excl, b.rws.ctl, 0,
@@ -233,6 +240,7 @@ kb_sorted_spine(const BatchSlot *slots, const int32_t *work)
 static __global__ void __launch_bounds__(kThreads)
 kb_sorted_uniforms(const BatchSlot *slots, const TileRef *map)
 {
+    pdl_enter();
     __shared__ SmemSortedUniforms sm;
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
@@ -245,6 +253,7 @@ kb_sorted_uniforms(const BatchSlot *slots, const TileRef *map)
 static __global__ void __launch_bounds__(kSpineThreads)
 kb_exact_terms_spine(const BatchSlot *slots, const int32_t *work)
 {
+    pdl_enter();
     __shared__ SmemExactSpine sm;
     const BatchSlot &b = slots[work[blockIdx.x]];
     k_exact_spine_body<TermsNeg, false>(TermsNeg{b.rws.u, 0}, b.N, b.rws.ctl,
@@ -255,6 +264,7 @@ template <typename Real, bool Residual, bool Sys>
 __global__ void __launch_bounds__(kThreads, VSMC_INVERT_MIN_BLOCKS)
 kb_invert(const BatchSlot *slots, const TileRef *map)
 {
+    pdl_enter();
     __shared__ SmemInvert<Residual> sm;
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
@@ -302,6 +312,7 @@ template <typename Src, bool Residual, bool Raw>
 __global__ void __launch_bounds__(kThreads, VSMC_EXACT_STAGE_MIN_BLOCKS)
 kb_exact_tiles_staged(const BatchSlot *slots, const TileRef *map, int nmap)
 {
+    pdl_enter();
     typedef typename Src::W W;
     typedef typename W::stage_t S;
     __shared__ SmemExactStage sm;
@@ -397,6 +408,7 @@ template <typename Real, bool Residual, bool Raw = false>
 __global__ void __launch_bounds__(kSpineThreads)
 kb_exact_spine(const BatchSlot *slots, const int32_t *work)
 {
+    pdl_enter();
     __shared__ SmemExactSpine sm;
     const BatchSlot &b = slots[work[blockIdx.x]];
     k_exact_spine_body<WeightsFromLog<Real>, Residual, Raw>(
@@ -404,38 +416,33 @@ kb_exact_spine(const BatchSlot *slots, const int32_t *work)
         b.rws.ex, sm);
 }
 
+// The zero-slot spine, then the resample engine position and the slot's step
+// count (the fill after it reads neither).
 static __global__ void __launch_bounds__(kSpineThreads)
-kb_zero_spine(const BatchSlot *slots, const int32_t *work)
+kb_zero_spine(BatchSlot *slots, const int32_t *work)
 {
     __shared__ SmemZeroSpine sm;
-    const BatchSlot &b = slots[work[blockIdx.x]];
+    pdl_enter();
+    BatchSlot &b = slots[work[blockIdx.x]];
     k_zero_spine_body(b.rws.tile_zeros, b.rws.tile_sinc_last, b.rws.zexcl,
                       b.rws.tfirst, b.rws.tlast, b.ntiles, b.rws.ctl, 0, sm);
+    if (threadIdx.x == 0) {
+        ResampleCtl *c = b.rws.ctl;
+        if (c->active)
+            c->offset += c->words;
+        b.t += 1;
+    }
 }
 
 static __global__ void __launch_bounds__(kThreads)
 kb_cfrp_fill(const BatchSlot *slots, const TileRef *map)
 {
+    pdl_enter();
     __shared__ SmemFill sm;
     const TileRef r = map[blockIdx.x];
     const BatchSlot &b = slots[r.slot];
     k_cfrp_fill_body(b.N, b.rws.ctl, b.rws.sinc, b.rws.zexcl, b.rws.tfirst,
                      b.rws.tlast, b.copy_from, r.tile, sm);
-}
-
-// End of a step: the resample engine position (k_resample_done) and the
-// slot's step count.
-static __global__ void kb_step_done(BatchSlot *slots, const int32_t *work,
-                                    int n)
-{
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= n)
-        return;
-    BatchSlot &b = slots[work[w]];
-    ResampleCtl *c = b.rws.ctl;
-    if (c->active)
-        c->offset += c->words;
-    b.t += 1;
 }
 
 // ---- block per filter ----------------------------------------------------
@@ -652,7 +659,7 @@ kb_block_run(BatchSlot *slots, const BlockItem *items, int n, int *queue,
                                  sm.ph.fill);
                 __syncthreads();
             }
-            // kb_step_done
+            // the engine position and the step count (kb_zero_spine)
             if (threadIdx.x == 0) {
                 ResampleCtl *rc = b.rws.ctl;
                 if (rc->active)
@@ -1022,8 +1029,9 @@ bool valid_slot(const vsmc_cuda_cv_batch *b, uint32_t s)
     return s < b->capacity && b->mem[s] != nullptr;
 }
 
-// Copies the work list into the device arrays: slots in the given order,
-// tile offsets as their exclusive prefix.  Returns the tile total.
+// Copies the work list into the device arrays: slots in the given order and,
+// unless `tiles` is null (a call whose kernels take a slot each), their tile
+// offsets and map; *tiles is the tile total.
 int stage_work(vsmc_cuda_cv_batch *b, const std::vector<uint32_t> &w,
                long long *tiles)
 {
@@ -1044,7 +1052,7 @@ int stage_work(vsmc_cuda_cv_batch *b, const std::vector<uint32_t> &w,
         set_last_error("vsmc_cuda_cv_batch: more than 2^31 tiles in a step");
         return VSMC_CUDA_EINVAL;
     }
-    if ((size_t)acc > b->map_cap) {
+    if (tiles != nullptr && (size_t)acc > b->map_cap) {
         if (b->d_map != nullptr)
             cudaFreeAsync(b->d_map, b->stream);
         b->d_map = nullptr;
@@ -1060,13 +1068,15 @@ int stage_work(vsmc_cuda_cv_batch *b, const std::vector<uint32_t> &w,
     }
     e = cudaMemcpyAsync(b->d_work, hw, (size_t)n * 4, cudaMemcpyHostToDevice,
                         b->stream);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && tiles != nullptr)
         e = cudaMemcpyAsync(b->d_tile0, ht, (size_t)(n + 1) * 4,
                             cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess)
         e = cudaEventRecord(b->staged, b->stream);
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_cv_batch: work list");
+    if (tiles == nullptr)
+        return VSMC_CUDA_OK;
     if (n > 0) {
         kb_expand<<<n, 256, 0, b->stream>>>(b->d_slots, b->d_work,
                                             b->d_tile0, n, b->d_map);
@@ -1077,110 +1087,110 @@ int stage_work(vsmc_cuda_cv_batch *b, const std::vector<uint32_t> &w,
 }
 
 // One step of the first n work items (whose tiles are the first `tiles`
-// map entries).
+// map entries).  `early`: each launch may start before the stream's previous
+// kernel has ended (launch_early).  Single steps do so: 48 resident filters
+// of 2^10 to 2^18 particles, mixed, took 220 us a step with ordinary launches
+// and take 198.  The steps of a run do not: as a graph they follow one another
+// closely already, and there it cost time (256 filters of 2^10 to 2^16:
+// 67.9 ms -> 69.9).
 template <typename Real>
 void launch_batch_step(vsmc_cuda_cv_batch *b, int n, long long tiles,
-                       cudaStream_t s)
+                       bool early, cudaStream_t s)
 {
     const int scheme = b->model.scheme;
     const bool residual = is_residual(scheme), sys = is_sys(scheme),
                strat = is_strat(scheme);
-    const unsigned nt = (unsigned)tiles;
-    const BatchSlot *sl = b->d_slots;
+    const unsigned nt = (unsigned)tiles, nf = (unsigned)n;
+    BatchSlot *sl = b->d_slots;
     const TileRef *map = b->d_map;
     const int32_t *work = b->d_work;
-    switch (b->tune_move) {
-    case 2:
-        kb_move<Real, 2><<<nt, kMoveThreads, 0, s>>>(
-            sl, map, b->bc.p);
-        break;
-    case 4:
-        kb_move<Real, 4><<<nt, kMoveThreads, 0, s>>>(
-            sl, map, b->bc.p);
-        break;
-    default:
-        kb_move<Real, 3><<<nt, kMoveThreads, 0, s>>>(
-            sl, map, b->bc.p);
-        break;
-    }
+    const unsigned et = exact_grid((int)nt);
     // a finalize CTA narrower than 1024 threads gives the same sums only
     // while every slot has at most 256 tiles
-    kb_finalize<<<n, b->max_ntiles <= 256 ? b->tune_final : kFinalThreads, 0,
-                  s>>>(sl, work, b->bc);
+    const int fin = b->max_ntiles <= 256 ? b->tune_final : kFinalThreads;
     // the per-filter spines on 256 threads while every slot has at most 256
     // tiles (each thread then holds at most one tile, so the sums are those
     // of 1024 threads): four times the spine CTAs fit on an SM
     const int spt = b->max_ntiles <= 256 ? 256 : kSpineThreads;
-    int launches = 2;
+    const auto tile_step = [&](auto k) {
+        launch_early(early, k, nt, kThreads, 0, s, sl, map);
+        ++b->launches;
+    };
+    const auto exact_step = [&](auto k) {
+        launch_early(early, k, et, kThreads, 0, s, sl, map, (int)nt);
+        ++b->launches;
+    };
+    const auto spine_step = [&](auto k, int threads) {
+        launch_early(early, k, nf, threads, 0, s, sl, work);
+        ++b->launches;
+    };
+    const auto move_step = [&](auto k) {
+        launch_early(early, k, nt, kMoveThreads, 0, s, sl, map, b->bc.p);
+        ++b->launches;
+    };
+    if (b->tune_move == 2)
+        move_step(kb_move<Real, 2>);
+    else if (b->tune_move == 4)
+        move_step(kb_move<Real, 4>);
+    else
+        move_step(kb_move<Real, 3>);
+    launch_early(early, kb_finalize, nf, fin, 0, s, sl, work, b->bc);
+    ++b->launches;
     if (WeightsFromLog<Real>::kExactNorm) {
         // the weights' sequential sum, whose reciprocal normalises them
-        kb_exact_tiles_staged<SlotWeights<Real, false>, false, true>
-            <<<exact_grid((int)nt), kThreads, 0, s>>>(sl, map, (int)nt);
-        kb_exact_spine<Real, false, true><<<n, spt, 0, s>>>(sl,
-                                                                     work);
-        launches += 2;
+        exact_step(
+            kb_exact_tiles_staged<SlotWeights<Real, false>, false, true>);
+        spine_step(kb_exact_spine<Real, false, true>, spt);
     }
     if (residual) {
-        kb_tile_sums<Real, true><<<nt, kThreads, 0, s>>>(sl, map);
+        tile_step(kb_tile_sums<Real, true>);
         if (sys)
-            kb_spine_weights<true, true><<<n, spt, 0, s>>>(sl,
-                                                                    work);
+            spine_step(kb_spine_weights<true, true>, spt);
         else
-            kb_spine_weights<true, false><<<n, spt, 0, s>>>(sl,
-                                                                     work);
-        launches += 2;
+            spine_step(kb_spine_weights<true, false>, spt);
     }
     if (strat) {
-        kb_uniforms_stratified<<<nt, kThreads, 0, s>>>(sl, map);
-        launches += 1;
+        tile_step(kb_uniforms_stratified);
     } else if (!sys) {
-        kb_sorted_tile_sums<<<nt, kThreads, 0, s>>>(sl, map);
-        kb_sorted_spine<<<n, spt, 0, s>>>(sl, work);
-        kb_exact_tiles_staged<SlotTerms, false, false>
-            <<<exact_grid((int)nt), kThreads, 0, s>>>(sl, map, (int)nt);
-        kb_exact_terms_spine<<<n, spt, 0, s>>>(sl, work);
-        kb_sorted_uniforms<<<nt, kThreads, 0, s>>>(sl, map);
-        launches += 5;
+        tile_step(kb_sorted_tile_sums);
+        spine_step(kb_sorted_spine, spt);
+        exact_step(kb_exact_tiles_staged<SlotTerms, false, false>);
+        spine_step(kb_exact_terms_spine, spt);
+        tile_step(kb_sorted_uniforms);
     }
     if (residual) {
         if (!WeightsFromLog<Real>::kApprox) { // the residuals' exact sum
-            kb_exact_tiles_staged<SlotWeights<Real, true>, true, true>
-                <<<exact_grid((int)nt), kThreads, 0, s>>>(sl, map, (int)nt);
-            kb_exact_spine<Real, true, true><<<n, spt, 0, s>>>(
-                sl, work);
-            launches += 2;
+            exact_step(
+                kb_exact_tiles_staged<SlotWeights<Real, true>, true, true>);
+            spine_step(kb_exact_spine<Real, true, true>, spt);
         }
-        kb_exact_tiles_staged<SlotWeights<Real, true>, true, false>
-            <<<exact_grid((int)nt), kThreads, 0, s>>>(sl, map, (int)nt);
-        kb_exact_spine<Real, true><<<n, spt, 0, s>>>(sl, work);
+        exact_step(
+            kb_exact_tiles_staged<SlotWeights<Real, true>, true, false>);
+        spine_step(kb_exact_spine<Real, true, false>, spt);
     } else {
-        kb_exact_tiles_staged<SlotWeights<Real, true>, false, false>
-            <<<exact_grid((int)nt), kThreads, 0, s>>>(sl, map, (int)nt);
-        kb_exact_spine<Real, false><<<n, spt, 0, s>>>(sl, work);
+        exact_step(
+            kb_exact_tiles_staged<SlotWeights<Real, true>, false, false>);
+        spine_step(kb_exact_spine<Real, false, false>, spt);
     }
-    launches += 2;
     if (residual && sys)
-        kb_invert<Real, true, true><<<nt, kThreads, 0, s>>>(sl, map);
+        tile_step(kb_invert<Real, true, true>);
     else if (residual)
-        kb_invert<Real, true, false><<<nt, kThreads, 0, s>>>(sl, map);
+        tile_step(kb_invert<Real, true, false>);
     else if (sys)
-        kb_invert<Real, false, true><<<nt, kThreads, 0, s>>>(sl, map);
+        tile_step(kb_invert<Real, false, true>);
     else
-        kb_invert<Real, false, false><<<nt, kThreads, 0, s>>>(sl, map);
-    kb_zero_spine<<<n, spt, 0, s>>>(sl, work);
-    kb_cfrp_fill<<<nt, kThreads, 0, s>>>(sl, map);
-    kb_step_done<<<(n + 255) / 256, 256, 0, s>>>(b->d_slots, b->d_work, n);
-    launches += 4;
-    b->launches += launches;
+        tile_step(kb_invert<Real, false, false>);
+    spine_step(kb_zero_spine, spt);
+    tile_step(kb_cfrp_fill);
 }
 
 void launch_step_any(vsmc_cuda_cv_batch *b, int n, long long tiles,
-                     cudaStream_t s)
+                     bool early, cudaStream_t s)
 {
     if (b->model.form == VSMC_CUDA_MIXED)
-        launch_batch_step<float>(b, n, tiles, s);
+        launch_batch_step<float>(b, n, tiles, early, s);
     else
-        launch_batch_step<double>(b, n, tiles, s);
+        launch_batch_step<double>(b, n, tiles, early, s);
 }
 
 void drop_run_graph(vsmc_cuda_cv_batch *b)
@@ -1198,7 +1208,7 @@ void launch_run_steps(vsmc_cuda_cv_batch *b, const std::vector<int> &active,
                       const std::vector<long long> &tile0, cudaStream_t s)
 {
     for (int a : active)
-        launch_step_any(b, a, tile0[a], s);
+        launch_step_any(b, a, tile0[a], /*early=*/false, s);
 }
 
 // The block-per-filter part of a run: `bs` forks from `s`, resets the work
@@ -1728,8 +1738,7 @@ int vsmc_cuda_cv_batch_initialize(vsmc_cuda_cv_batch *b, uint32_t n,
     if (n == 0)
         return VSMC_CUDA_OK;
     std::vector<uint32_t> w(slots, slots + n);
-    long long tiles = 0;
-    st = stage_work(b, w, &tiles);
+    st = stage_work(b, w, nullptr);
     if (st != VSMC_CUDA_OK)
         return st;
     kb_reset<<<(n + 255) / 256, 256, 0, b->stream>>>(b->d_slots, b->d_work,
@@ -1762,7 +1771,7 @@ int vsmc_cuda_cv_batch_step(vsmc_cuda_cv_batch *b, uint32_t n,
     st = stage_work(b, w, &tiles);
     if (st != VSMC_CUDA_OK)
         return st;
-    launch_step_any(b, (int)n, tiles, b->stream);
+    launch_step_any(b, (int)n, tiles, true, b->stream);
     for (uint32_t k = 0; k < n; ++k)
         ++b->t[slots[k]];
     cudaError_t e = cudaGetLastError();
@@ -1984,8 +1993,7 @@ int vsmc_cuda_cv_batch_read_last(vsmc_cuda_cv_batch *b, uint32_t n,
     if (n == 0)
         return VSMC_CUDA_OK;
     std::vector<uint32_t> w(slots, slots + n);
-    long long tiles = 0;
-    st = stage_work(b, w, &tiles);
+    st = stage_work(b, w, nullptr);
     if (st != VSMC_CUDA_OK)
         return st;
     kb_read_last<<<(n + 255) / 256, 256, 0, b->stream>>>(
@@ -2044,8 +2052,7 @@ int vsmc_cuda_cv_batch_history(vsmc_cuda_cv_batch *b, uint32_t slot,
     if (T == 0)
         return VSMC_CUDA_OK;
     std::vector<uint32_t> w(1, slot);
-    long long tiles = 0;
-    int st = stage_work(b, w, &tiles);
+    int st = stage_work(b, w, nullptr);
     if (st != VSMC_CUDA_OK)
         return st;
     if (b->model.form == VSMC_CUDA_MIXED)
