@@ -1447,87 +1447,21 @@ inline RcArgs rc_args(long long N, const EngineRef &eng,
     return a;
 }
 
-bool launch_resample(int scheme, WeightsGiven w, long long N,
-                     const EngineRef &eng, ResampleWorkspace &ws,
-                     const ResampleCtl &h, ResampleCtl *slot,
-                     const double *u_given, long long n_given,
-                     int32_t *rep_out, int32_t *copy_from, cudaStream_t s,
-                     bool cfrp)
-{
-    if (u_given != nullptr || !rc_fits(N, h.Nout)) {
-        const ResampleCtl *src = &h;
-        if (slot != nullptr) { // (pinned: copied without staging)
-            *slot = h;
-            src = slot;
-        }
-        // a failed copy leaves its error for the caller's check
-        if (cudaMemcpyAsync(ws.ctl, src, sizeof(h), cudaMemcpyHostToDevice,
-                            s) == cudaSuccess)
-            launch_resample_core(scheme, w, N, eng, ws, u_given, n_given,
-                                 false, rep_out, copy_from, s, false, cfrp,
-                                 h.Nout);
-        return false;
-    }
-    RcArgs a = rc_args(N, eng, ws, rep_out, copy_from, cfrp);
-    a.offset = h.offset;
-    a.Nout = h.Nout;
-    a.out = slot != nullptr ? slot : ws.ctl;
-    const RcShape sh = rc_shape(resample_ntiles(h.Nout > N ? h.Nout : N));
-    rc_scheme(scheme, [&](auto res, auto seq) {
-        constexpr bool Re = decltype(res)::value;
-        constexpr int U = decltype(seq)::value;
-        if (sh.r == 8)
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, false,
-                      s, w, a);
-        else
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, false,
-                      s, w, a);
-    });
-    return slot != nullptr;
-}
-
-// Dynamic shared memory that a kernel may have without asking for more.
-constexpr size_t kDefaultSmem = 48 << 10;
-
 template <typename W>
-inline int launch_finish_t(int scheme, const FinalizeArgs &fa, const W &w,
-                           ResampleWorkspace &ws, int32_t *copy_from,
-                           bool resample, cudaEvent_t seq, cudaStream_t s)
+void launch_cluster_finish(int scheme, const FinalizeArgs &fa, const W &w,
+                           const ResampleWorkspace &ws, int32_t *copy_from,
+                           cudaStream_t s)
 {
-    const long long N = fa.N;
-    if (rc_fits(N, 0)) {
-        const RcArgs a = rc_args(N, fa.eng, ws, nullptr, copy_from, true);
-        const RcShape sh = rc_shape(fa.ntiles);
-        rc_scheme(scheme, [&](auto res, auto u) {
-            constexpr bool Re = decltype(res)::value;
-            constexpr int U = decltype(u)::value;
-            if (sh.r == 8)
-                rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, true, s, fa, w,
-                          a);
-            else
-                rc_launch(k_finish_cluster<W, Re, U, 2>, sh, 1, true, s, fa, w,
-                          a);
-        });
-        return 1;
-    }
-    const size_t smem = fa.ntiles <= kFinalSmemTiles
-                            ? (size_t)fa.ntiles * sizeof(double)
-                            : 0;
-    if (smem > kDefaultSmem)
-        cudaFuncSetAttribute(k_cv_finalize,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kFinalSmemTiles * (int)sizeof(double));
-    launch_early(true, k_cv_finalize, 1, kFinalThreads, smem, s, fa);
-    if (!resample)
-        return 1;
-    const bool ready = seq != nullptr;
-    if (ready)
-        cudaStreamWaitEvent(s, seq, 0);
-    launch_resample_core(scheme, w, N, fa.eng, ws, nullptr, 0,
-                         /*spine_done=*/true, nullptr, copy_from, s, ready);
-    return 1 +
-           resample_launches(scheme, false, W::kExactNorm, W::kApprox) -
-           (ready ? 5 : 0);
+    const RcArgs a = rc_args(fa.N, fa.eng, ws, nullptr, copy_from, true);
+    const RcShape sh = rc_shape(fa.ntiles);
+    rc_scheme(scheme, [&](auto res, auto u) {
+        constexpr bool Re = decltype(res)::value;
+        constexpr int U = decltype(u)::value;
+        if (sh.r == 8)
+            rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, true, s, fa, w, a);
+        else
+            rc_launch(k_finish_cluster<W, Re, U, 2>, sh, 1, true, s, fa, w, a);
+    });
 }
 
 } // namespace vsmc_b200

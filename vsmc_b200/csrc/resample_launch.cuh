@@ -21,6 +21,18 @@ inline bool rc_fits(long long N, long long Nout)
     return resample_ntiles(n) <= kRcMaxTiles;
 }
 
+// The one-cluster forms (rc_fits): a resampling of given weights whose
+// control block goes to *out; a filter step's finalisation and resampling.
+void launch_cluster_resample(int scheme, WeightsGiven w, long long N,
+                             const EngineRef &eng, const ResampleWorkspace &ws,
+                             const ResampleCtl &h, ResampleCtl *out,
+                             int32_t *rep_out, int32_t *copy_from,
+                             cudaStream_t s, bool cfrp);
+template <typename W>
+void launch_cluster_finish(int scheme, const FinalizeArgs &fa, const W &w,
+                           const ResampleWorkspace &ws, int32_t *copy_from,
+                           cudaStream_t s);
+
 // A resampling of given weights: one cluster where it fits, the launch
 // sequence of resample.cuh otherwise (and for caller-supplied uniforms).
 // `h` holds the call's initial control block; `slot` is a call's pinned
