@@ -548,9 +548,9 @@ int vsmc_cuda_cv_batch_history(vsmc_cuda_cv_batch *b, uint32_t slot,
 
 int vsmc_cuda_cv_batch_synchronize(vsmc_cuda_cv_batch *b);
 
-/* vsmc_cuda_cv_batch_run records its steps in a CUDA graph and launches
- * the graph (on by default); a run with the same slots and step counts as
- * the previous one relaunches the same graph. */
+/* vsmc_cuda_cv_batch_run records its steps in a CUDA graph once a run of the
+ * same slots and step counts repeats, and relaunches it while they do (on by
+ * default; without it every run's kernels are launched one by one). */
 int vsmc_cuda_cv_batch_set_graphs(vsmc_cuda_cv_batch *b, int enable);
 
 /* The launch shape of later steps: the move compiled for `move_blocks`

@@ -930,7 +930,8 @@ struct vsmc_cuda_cv_batch {
     bool use_graphs;
     cudaStream_t cap_stream; // capture only; graphs launch on `stream`
     cudaGraphExec_t run_exec;
-    std::vector<uint64_t> run_key;
+    std::vector<uint64_t> run_key; // the last run's lists and step counts
+    int run_repeats;               // runs in a row that had them
     const TileRef *run_map;
     uint64_t run_launches;
     // launch shapes (vsmc_cuda_cv_batch_autotune); no result depends on them
@@ -949,6 +950,9 @@ struct vsmc_cuda_cv_batch {
     cudaStream_t block_stream;     // block-per-filter launches
     cudaStream_t block_cap_stream; // their capture twin
     cudaEvent_t ev_fork, ev_join;
+    cudaStream_t seq_stream;     // the sorted sequences of a run
+    cudaStream_t seq_cap_stream; // their capture twin
+    cudaEvent_t ev_seq_fork, ev_seq_join;
 };
 
 namespace {
@@ -1092,10 +1096,13 @@ int stage_work(vsmc_cuda_cv_batch *b, const std::vector<uint32_t> &w,
 // of 2^10 to 2^18 particles, mixed, took 220 us a step with ordinary launches
 // and take 198.  The steps of a run do not: as a graph they follow one another
 // closely already, and there it cost time (256 filters of 2^10 to 2^16:
-// 67.9 ms -> 69.9).
+// 67.9 ms -> 69.9).  `side` (a run; otherwise null): the sorted
+// sequence forks there, beside the weights' exact scans, neither of which
+// reads what the other writes; each chain's one-CTA-per-filter spines then
+// overlap the other's tiles.
 template <typename Real>
 void launch_batch_step(vsmc_cuda_cv_batch *b, int n, long long tiles,
-                       bool early, cudaStream_t s)
+                       bool early, cudaStream_t s, cudaStream_t side)
 {
     const int scheme = b->model.scheme;
     const bool residual = is_residual(scheme), sys = is_sys(scheme),
@@ -1112,21 +1119,40 @@ void launch_batch_step(vsmc_cuda_cv_batch *b, int n, long long tiles,
     // tiles (each thread then holds at most one tile, so the sums are those
     // of 1024 threads): four times the spine CTAs fit on an SM
     const int spt = b->max_ntiles <= 256 ? 256 : kSpineThreads;
-    const auto tile_step = [&](auto k) {
-        launch_early(early, k, nt, kThreads, 0, s, sl, map);
+    const auto tile_step = [&](auto k, cudaStream_t on) {
+        launch_early(early, k, nt, kThreads, 0, on, sl, map);
         ++b->launches;
     };
-    const auto exact_step = [&](auto k) {
-        launch_early(early, k, et, kThreads, 0, s, sl, map, (int)nt);
+    const auto exact_step = [&](auto k, cudaStream_t on) {
+        launch_early(early, k, et, kThreads, 0, on, sl, map, (int)nt);
         ++b->launches;
     };
-    const auto spine_step = [&](auto k, int threads) {
-        launch_early(early, k, nf, threads, 0, s, sl, work);
+    const auto spine_step = [&](auto k, cudaStream_t on) {
+        launch_early(early, k, nf, spt, 0, on, sl, work);
         ++b->launches;
     };
     const auto move_step = [&](auto k) {
         launch_early(early, k, nt, kMoveThreads, 0, s, sl, map, b->bc.p);
         ++b->launches;
+    };
+    // the U01 sequence of the step's resampling
+    const bool sorted = !strat && !sys;
+    if (!sorted)
+        side = nullptr;
+    const auto sequence = [&](cudaStream_t on) {
+        tile_step(kb_sorted_tile_sums, on);
+        spine_step(kb_sorted_spine, on);
+        exact_step(kb_exact_tiles_staged<SlotTerms, false, false>, on);
+        spine_step(kb_exact_terms_spine, on);
+        tile_step(kb_sorted_uniforms, on);
+    };
+    const auto fork = [&] { // its length is known here
+        if (side == nullptr)
+            return;
+        cudaEventRecord(b->ev_seq_fork, s);
+        cudaStreamWaitEvent(side, b->ev_seq_fork, 0);
+        sequence(side);
+        cudaEventRecord(b->ev_seq_join, side);
     };
     if (b->tune_move == 2)
         move_step(kb_move<Real, 2>);
@@ -1136,62 +1162,69 @@ void launch_batch_step(vsmc_cuda_cv_batch *b, int n, long long tiles,
         move_step(kb_move<Real, 3>);
     launch_early(early, kb_finalize, nf, fin, 0, s, sl, work, b->bc);
     ++b->launches;
+    if (!residual)
+        fork();
     if (WeightsFromLog<Real>::kExactNorm) {
         // the weights' sequential sum, whose reciprocal normalises them
         exact_step(
-            kb_exact_tiles_staged<SlotWeights<Real, false>, false, true>);
-        spine_step(kb_exact_spine<Real, false, true>, spt);
+            kb_exact_tiles_staged<SlotWeights<Real, false>, false, true>, s);
+        spine_step(kb_exact_spine<Real, false, true>, s);
     }
     if (residual) {
-        tile_step(kb_tile_sums<Real, true>);
+        tile_step(kb_tile_sums<Real, true>, s);
         if (sys)
-            spine_step(kb_spine_weights<true, true>, spt);
+            spine_step(kb_spine_weights<true, true>, s);
         else
-            spine_step(kb_spine_weights<true, false>, spt);
+            spine_step(kb_spine_weights<true, false>, s);
+        fork();
     }
-    if (strat) {
-        tile_step(kb_uniforms_stratified);
-    } else if (!sys) {
-        tile_step(kb_sorted_tile_sums);
-        spine_step(kb_sorted_spine, spt);
-        exact_step(kb_exact_tiles_staged<SlotTerms, false, false>);
-        spine_step(kb_exact_terms_spine, spt);
-        tile_step(kb_sorted_uniforms);
-    }
+    if (strat)
+        tile_step(kb_uniforms_stratified, s);
+    else if (sorted && side == nullptr)
+        sequence(s);
     if (residual) {
         if (!WeightsFromLog<Real>::kApprox) { // the residuals' exact sum
             exact_step(
-                kb_exact_tiles_staged<SlotWeights<Real, true>, true, true>);
-            spine_step(kb_exact_spine<Real, true, true>, spt);
+                kb_exact_tiles_staged<SlotWeights<Real, true>, true, true>, s);
+            spine_step(kb_exact_spine<Real, true, true>, s);
         }
         exact_step(
-            kb_exact_tiles_staged<SlotWeights<Real, true>, true, false>);
-        spine_step(kb_exact_spine<Real, true, false>, spt);
+            kb_exact_tiles_staged<SlotWeights<Real, true>, true, false>, s);
+        spine_step(kb_exact_spine<Real, true, false>, s);
     } else {
         exact_step(
-            kb_exact_tiles_staged<SlotWeights<Real, true>, false, false>);
-        spine_step(kb_exact_spine<Real, false, false>, spt);
+            kb_exact_tiles_staged<SlotWeights<Real, true>, false, false>, s);
+        spine_step(kb_exact_spine<Real, false, false>, s);
     }
+    if (side != nullptr)
+        cudaStreamWaitEvent(s, b->ev_seq_join, 0);
     if (residual && sys)
-        tile_step(kb_invert<Real, true, true>);
+        tile_step(kb_invert<Real, true, true>, s);
     else if (residual)
-        tile_step(kb_invert<Real, true, false>);
+        tile_step(kb_invert<Real, true, false>, s);
     else if (sys)
-        tile_step(kb_invert<Real, false, true>);
+        tile_step(kb_invert<Real, false, true>, s);
     else
-        tile_step(kb_invert<Real, false, false>);
-    spine_step(kb_zero_spine, spt);
-    tile_step(kb_cfrp_fill);
+        tile_step(kb_invert<Real, false, false>, s);
+    spine_step(kb_zero_spine, s);
+    tile_step(kb_cfrp_fill, s);
 }
 
 void launch_step_any(vsmc_cuda_cv_batch *b, int n, long long tiles,
-                     bool early, cudaStream_t s)
+                     bool early, cudaStream_t s, cudaStream_t side)
 {
     if (b->model.form == VSMC_CUDA_MIXED)
-        launch_batch_step<float>(b, n, tiles, early, s);
+        launch_batch_step<float>(b, n, tiles, early, s, side);
     else
-        launch_batch_step<double>(b, n, tiles, early, s);
+        launch_batch_step<double>(b, n, tiles, early, s, side);
 }
+
+// A run of the same lists is launched directly this many times, then recorded
+// as a graph: recording costs about four times what a relaunch saves (256
+// filters of 2^10 to 2^16 over 50 to 200 steps: 65.2 ms launched directly,
+// 17 ms to record, 60.6 ms relaunched; recorded at once, the first run took
+// 82 ms).
+constexpr int kRunsBeforeGraph = 2;
 
 void drop_run_graph(vsmc_cuda_cv_batch *b)
 {
@@ -1201,14 +1234,16 @@ void drop_run_graph(vsmc_cuda_cv_batch *b)
     }
     b->run_exec = nullptr;
     b->run_key.clear();
+    b->run_repeats = 0;
 }
 
 // The steps of a run: step k runs the first active(k) work items.
 void launch_run_steps(vsmc_cuda_cv_batch *b, const std::vector<int> &active,
-                      const std::vector<long long> &tile0, cudaStream_t s)
+                      const std::vector<long long> &tile0, cudaStream_t s,
+                      cudaStream_t side)
 {
     for (int a : active)
-        launch_step_any(b, a, tile0[a], /*early=*/false, s);
+        launch_step_any(b, a, tile0[a], /*early=*/false, s, side);
 }
 
 // The block-per-filter part of a run: `bs` forks from `s`, resets the work
@@ -1370,9 +1405,14 @@ int vsmc_cuda_cv_batch_create(const vsmc_cuda_cv_config *model,
     b->block_cap_stream = nullptr;
     b->ev_fork = nullptr;
     b->ev_join = nullptr;
+    b->seq_stream = nullptr;
+    b->seq_cap_stream = nullptr;
+    b->ev_seq_fork = nullptr;
+    b->ev_seq_join = nullptr;
     b->run_exec = nullptr;
     b->run_map = nullptr;
     b->run_launches = 0;
+    b->run_repeats = 0;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     cudaMemPoolProps props;
@@ -1438,6 +1478,15 @@ int vsmc_cuda_cv_batch_create(const vsmc_cuda_cv_config *model,
         e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&b->block_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = cudaEventCreateWithFlags(&b->ev_seq_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+        e = cudaEventCreateWithFlags(&b->ev_seq_join, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+        e = cudaStreamCreateWithFlags(&b->seq_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = cudaStreamCreateWithFlags(&b->seq_cap_stream,
+                                      cudaStreamNonBlocking);
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&b->block_cap_stream,
                                       cudaStreamNonBlocking);
@@ -1505,6 +1554,16 @@ int vsmc_cuda_cv_batch_destroy(vsmc_cuda_cv_batch *b)
     cudaFreeHost(b->h_items);
     if (b->items_staged != nullptr)
         cudaEventDestroy(b->items_staged);
+    if (b->seq_stream != nullptr) {
+        cudaStreamSynchronize(b->seq_stream);
+        cudaStreamDestroy(b->seq_stream);
+    }
+    if (b->seq_cap_stream != nullptr)
+        cudaStreamDestroy(b->seq_cap_stream);
+    if (b->ev_seq_fork != nullptr)
+        cudaEventDestroy(b->ev_seq_fork);
+    if (b->ev_seq_join != nullptr)
+        cudaEventDestroy(b->ev_seq_join);
     if (b->ev_fork != nullptr)
         cudaEventDestroy(b->ev_fork);
     if (b->ev_join != nullptr)
@@ -1771,7 +1830,7 @@ int vsmc_cuda_cv_batch_step(vsmc_cuda_cv_batch *b, uint32_t n,
     st = stage_work(b, w, &tiles);
     if (st != VSMC_CUDA_OK)
         return st;
-    launch_step_any(b, (int)n, tiles, true, b->stream);
+    launch_step_any(b, (int)n, tiles, /*early=*/true, b->stream, nullptr);
     for (uint32_t k = 0; k < n; ++k)
         ++b->t[slots[k]];
     cudaError_t e = cudaGetLastError();
@@ -1825,11 +1884,8 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
     }
     const int nsmall = (int)small.size();
     cudaError_t e = cudaSuccess;
-    if (b->use_graphs && (!active.empty() || nsmall > 0)) {
-        // the whole run as one CUDA graph, reused while the work lists and
-        // their step counts repeat (kernels read everything else from the
-        // slot records and the staged block items)
-        std::vector<uint64_t> key;
+    std::vector<uint64_t> key; // the run's work lists and step counts
+    if (b->use_graphs) {
         key.reserve(2 * n + 2);
         for (uint32_t k = 0; k < nw; ++k) {
             key.push_back(w[k]);
@@ -1840,9 +1896,22 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
             key.push_back(x);
             key.push_back(b->T_obs[x] - b->t[x]);
         }
-        if (b->run_exec == nullptr || key != b->run_key ||
-            b->run_map != b->d_map) {
+    }
+    if (key != b->run_key) {
+        drop_run_graph(b);
+        b->run_key = key;
+    }
+    const bool again = b->run_repeats >= kRunsBeforeGraph;
+    if (!again)
+        ++b->run_repeats;
+    if (b->use_graphs && again && (!active.empty() || nsmall > 0)) {
+        // the whole run as one CUDA graph, relaunched while the work lists
+        // and their step counts repeat (kernels read everything else from
+        // the slot records and the staged block items)
+        if (b->run_exec == nullptr || b->run_map != b->d_map) {
             drop_run_graph(b);
+            b->run_key = key;
+            b->run_repeats = kRunsBeforeGraph;
             cudaGraph_t g = nullptr;
             e = cudaStreamBeginCapture(b->cap_stream,
                                        cudaStreamCaptureModeThreadLocal);
@@ -1851,7 +1920,8 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
                 if (nsmall > 0)
                     launch_block_part(b, nsmall, b->cap_stream,
                                       b->block_cap_stream);
-                launch_run_steps(b, active, tile0, b->cap_stream);
+                launch_run_steps(b, active, tile0, b->cap_stream,
+                                 b->seq_cap_stream);
                 if (nsmall > 0)
                     join_block_part(b, b->cap_stream, b->block_cap_stream);
                 b->run_launches = b->launches - before;
@@ -1865,7 +1935,6 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
                 b->run_exec = nullptr;
                 return cuda_status(e, "vsmc_cuda_cv_batch_run: graph");
             }
-            b->run_key = key;
             b->run_map = b->d_map;
             b->launches -= b->run_launches; // counted when launched
         }
@@ -1874,7 +1943,7 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
     } else {
         if (nsmall > 0)
             launch_block_part(b, nsmall, b->stream, b->block_stream);
-        launch_run_steps(b, active, tile0, b->stream);
+        launch_run_steps(b, active, tile0, b->stream, b->seq_stream);
         if (nsmall > 0)
             join_block_part(b, b->stream, b->block_stream);
     }
