@@ -870,7 +870,7 @@ k_gmm_mcmc(GmmArgs a)
     cta_reduce_acc(acc, 3 * a.sweeps, a.tile_acc);
 }
 
-// Likelihood only (autotuning and precision checks): ll of every particle
+// Likelihood only (precision checks): ll of every particle
 // of `src` into out[i].
 template <int G, bool F32>
 __global__ void __launch_bounds__(kGmmThreads)

@@ -10,12 +10,16 @@
 //   (residual only) tile sums of r = modf(N w) and of floor(N w)
 //   spine      one CTA: deterministic exclusive prefix of the tile sums
 //   uniforms   U01 sequence u_0..u_{NN-1} (not for Systematic: closed form)
-//   invert     per tile: FP64 scan of the weights anchored on the spine,
-//              count of uniforms <= C_i, replication, zero-slot ranks by an
-//              integer decoupled look-back, copy_from for survivors and the
-//              inclusive surplus-children count
-//   fill       zero slots find their parent by a galloping search
-// Every FP64 sum is formed in a fixed order (no float atomics, no look-back
+//   exact      per tile, a spine, per tile again: the weights' sequential
+//              sums, bit for bit (exact_scan.cuh)
+//   invert     per tile: count of uniforms <= C_i, replication, zero-slot
+//              ranks, copy_from for survivors and the inclusive
+//              surplus-children count
+//   fill       zero slots find their parent: the running maximum of the
+//              ranks that the parents mark
+// Small filters run the same in one cluster (resample_cluster.cuh).  The
+// kernels launch before their stream's previous kernel has ended
+// (launch_early).  Every FP64 sum is formed in a fixed order (no float atomics, no look-back
 // on floats), so results are reproducible run to run.
 #pragma once
 

@@ -1350,7 +1350,16 @@ k_finish_cluster(FinalizeArgs fa, W wsrc, RcArgs a)
 }
 
 // The cluster of nt tiles: up to 16 a CTA of 1024 threads each (two
-// particles a thread), above two tiles a CTA of 512 threads (eight).
+// particles a thread), above two tiles a CTA of 512 threads (eight).  The
+// serial chain over a thread's particles is what a tile waits for, so few
+// particles a thread are better as long as an SM's threads suffice: two
+// tiles a CTA leave 1024 threads for 4096 particles, and there the fewer
+// registers of 1024-thread CTAs cost more than the shorter chain gives.
+// FP64 Multinomial filter, us a step at N = 1000 / 32768 / 65536 on one
+// B200: launch sequence 93.8 / 112.8 / 113; this cluster with 256 threads a
+// tile 62.7 / 83.0 / 89.9; as it is 48.0 / 65.1 / 82.6; with the
+// finalisation in the same kernel 37.5 / 46.0 / 63.8; launched early 31.7 /
+// - / 57.2.
 struct RcShape {
     int ctas, groups, r;
 };

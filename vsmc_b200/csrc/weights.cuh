@@ -15,9 +15,9 @@
 // normalisation; larger arrays take sums, join and normalisation kernels.
 // Bound: latency of launches and of the ordered joins below about 10^6
 // elements, HBM / L2 above.  Measured on one B200 (a program's whole step of
-// ESS, CESS, update, resampling and gather, most of it call_scratch.hpp's
-// allocations): 1000 particles 1620 -> 114 us, 3000001 particles 1950 ->
-// 382 us.
+// ESS, CESS, update, resampling and gather, most of the gain that of
+// call_scratch.hpp's allocations): 1000 particles 1620 -> 102 us, 3000001
+// particles 1950 -> 343 us.
 #pragma once
 
 #include <cooperative_groups.h>
