@@ -802,7 +802,7 @@ __device__ __forceinline__ void k_cv_finalize_body(const FinalizeArgs &a,
     for (int t = b; t < e; ++t)
         run += share[t] * coeff;
     double total;
-    double off = block_excl_scan(run, sh_spine, total);
+    double off = block_excl_sum(run, sh_spine, total);
     // in place in `share` (read before write per t); staged shares are then
     // copied out with coalesced stores
     for (int t = b; t < e; ++t) {

@@ -20,6 +20,10 @@
 //   sequential sum) + the error of G (a relative margin of the weight
 //   source); each thread uses one bound for its kItems elements,
 //   d = (8 i_last + 256) ulp(2 m) + margin * m, m >= every G and w there.
+//   The bound is relative to the thread's own prefixes, so no part of G may be
+//   formed by subtracting a later weight from a sum that holds it
+//   (block_excl_sum, block_prefix): beside a weight 2^53 times all before it
+//   the difference is 0 or off by a binade.
 // * A zero weight while the prefix is still 0 leaves S at 0: clean, k = 0.
 // * The other ("special") elements -- the first, binade crossings,
 //   uncertain binades, ties -- are few (about 40 at N = 2^24): the spine
@@ -189,7 +193,8 @@ exact_classify(long long i0, long long N, const double (&w)[R], double a,
                     // S_{-1} = 0: the first addition is the hardware's
                 } else if (gp == 0.0 && w[j] == 0.0) {
                     // a leading zero: every weight before it is 0 (sums of
-                    // non-negative weights vanish only so)
+                    // non-negative weights, formed without subtractions,
+                    // vanish only so)
                     sp = false;
                 } else if (ec != kNoBinade && ec == ep) {
                     // k = w / 2^(e-52) rounded to nearest: adding 2^52 rounds

@@ -548,7 +548,7 @@ __device__ __forceinline__ void spine_scan_f64(const double *in, double *excl,
         for (int k = 0; k < 8; ++k)
             if (b + k < e)
                 run += x[k];
-        run = block_excl_scan(run, sh, total);
+        run = block_excl_sum(run, sh, total);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
             if (b + k < e) {
@@ -558,7 +558,7 @@ __device__ __forceinline__ void spine_scan_f64(const double *in, double *excl,
     } else {
         for (int t = b; t < e; ++t)
             run += __dmul_rn(in[t], scale);
-        const double off = block_excl_scan(run, sh, total);
+        const double off = block_excl_sum(run, sh, total);
         run = off;
         for (int t = b; t < e; ++t) {
             excl[t] = run;
@@ -1204,7 +1204,7 @@ __device__ __forceinline__ double block_prefix(double v, double *sh,
         all += x;
     }
     total = all;
-    return before + inc - v;
+    return before + warp_excl_of(inc);
 }
 
 // Where a tile's scan puts its specials and last binade in global memory.

@@ -130,7 +130,7 @@ struct RcArgs {
 };
 
 // Exclusive scan over a group (any association: FP64 sums here feed only
-// the exact scan's classification, or are integers).
+// the exact scan's classification, or are integers), without a subtraction.
 template <typename T, int R>
 __device__ __forceinline__ T rc_excl_scan(T v, T *sh, const RcThread<R> &th,
                                           T &total)
@@ -140,12 +140,11 @@ __device__ __forceinline__ T rc_excl_scan(T v, T *sh, const RcThread<R> &th,
     if (th.lane == 31)
         sh[th.wid] = inc;
     th.sync();
-    const T x = th.lane < NW ? sh[th.lane] : T(0);
-    const T xi = warp_incl_scan(x);
+    const T xi = warp_incl_scan(th.lane < NW ? sh[th.lane] : T(0));
     total = __shfl_sync(0xffffffffu, xi, 31);
-    const T before = __shfl_sync(0xffffffffu, xi - x, th.wid);
+    const T before = __shfl_sync(0xffffffffu, warp_excl_of(xi), th.wid);
     th.sync();
-    return before + inc - v;
+    return before + warp_excl_of(inc);
 }
 
 // The plain scan's prefixes of a tile in the launch sequence's association:
@@ -1296,7 +1295,7 @@ __device__ __forceinline__ void rc_finalize(const FinalizeArgs &a,
     const int res = a.replay_flags != nullptr ? rflag != 0 : own;
     // the spine of the normalised shares, for the classification
     const double sh = share * __ddiv_rn(1.0, S1);
-    const double excl = warp_incl_scan(sh) - sh;
+    const double excl = warp_excl_of(warp_incl_scan(sh));
     sm.excl[lane] = excl;
     if (lane != 0)
         return;

@@ -180,4 +180,37 @@ __device__ __forceinline__ T block_excl_scan(T v, T *sh, T &total)
     return wexcl + inc - v;
 }
 
+// The lane's exclusive prefix from its inclusive one: the lane before's, not
+// inc - v, which for doubles loses a sum more than 2^53 times smaller than v.
+template <typename T>
+__device__ __forceinline__ T warp_excl_of(T inc)
+{
+    const T before = __shfl_up_sync(0xffffffffu, inc, 1);
+    return (threadIdx.x & 31) > 0 ? before : T(0);
+}
+
+// block_excl_scan without its subtraction: a prefix of non-negative values is
+// then within a few ulps of itself, and 0 only when every value before it is.
+__device__ __forceinline__ double block_excl_sum(double v, double *sh,
+                                                 double &total)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nw = blockDim.x >> 5;
+    const double inc = warp_incl_scan(v);
+    if (lane == 31)
+        sh[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        double s = lane < nw ? sh[lane] : 0.0;
+        s = warp_incl_scan(s);
+        if (lane < nw)
+            sh[lane] = s;
+    }
+    __syncthreads();
+    const double wexcl = wid > 0 ? sh[wid - 1] : 0.0;
+    total = sh[nw - 1];
+    __syncthreads();
+    return wexcl + warp_excl_of(inc);
+}
+
 } // namespace vsmc_b200
