@@ -549,8 +549,9 @@ int vsmc_cuda_cv_batch_history(vsmc_cuda_cv_batch *b, uint32_t slot,
 int vsmc_cuda_cv_batch_synchronize(vsmc_cuda_cv_batch *b);
 
 /* vsmc_cuda_cv_batch_run records its steps in a CUDA graph once a run of the
- * same slots and step counts repeats, and relaunches it while they do (on by
- * default; without it every run's kernels are launched one by one). */
+ * same slots, particle tiles and step counts repeats, and relaunches it while
+ * they do (on by default; without it every run's kernels are launched one by
+ * one). */
 int vsmc_cuda_cv_batch_set_graphs(vsmc_cuda_cv_batch *b, int enable);
 
 /* The launch shape of later steps: the move compiled for `move_blocks`

@@ -930,7 +930,7 @@ struct vsmc_cuda_cv_batch {
     bool use_graphs;
     cudaStream_t cap_stream; // capture only; graphs launch on `stream`
     cudaGraphExec_t run_exec;
-    std::vector<uint64_t> run_key; // the last run's lists and step counts
+    std::vector<uint64_t> run_key; // the last run's lists, tiles, step counts
     int run_repeats;               // runs in a row that had them
     const TileRef *run_map;
     uint64_t run_launches;
@@ -1884,18 +1884,20 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
     }
     const int nsmall = (int)small.size();
     cudaError_t e = cudaSuccess;
-    std::vector<uint64_t> key; // the run's work lists and step counts
+    // all that a recorded run depends on: its work lists, their filters' tiles
+    // (the grids; a slot's filter may have been replaced) and step counts
+    std::vector<uint64_t> key;
     if (b->use_graphs) {
-        key.reserve(2 * n + 2);
-        for (uint32_t k = 0; k < nw; ++k) {
-            key.push_back(w[k]);
-            key.push_back(b->T_obs[w[k]] - b->t[w[k]]);
-        }
-        key.push_back(~0ull);
-        for (uint32_t x : small) {
-            key.push_back(x);
+        key.reserve(2 * n + 1);
+        const auto add = [&](uint32_t x) {
+            key.push_back(x | (uint64_t)b->slots[x].ntiles << 32);
             key.push_back(b->T_obs[x] - b->t[x]);
-        }
+        };
+        for (uint32_t x : w)
+            add(x);
+        key.push_back(~0ull);
+        for (uint32_t x : small)
+            add(x);
     }
     if (key != b->run_key) {
         drop_run_graph(b);
@@ -1905,9 +1907,9 @@ int vsmc_cuda_cv_batch_run(vsmc_cuda_cv_batch *b, uint32_t n,
     if (!again)
         ++b->run_repeats;
     if (b->use_graphs && again && (!active.empty() || nsmall > 0)) {
-        // the whole run as one CUDA graph, relaunched while the work lists
-        // and their step counts repeat (kernels read everything else from
-        // the slot records and the staged block items)
+        // the whole run as one CUDA graph, relaunched while the key repeats
+        // (kernels read everything else from the slot records and the staged
+        // block items)
         if (b->run_exec == nullptr || b->run_map != b->d_map) {
             drop_run_graph(b);
             b->run_key = key;
