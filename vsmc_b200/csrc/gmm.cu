@@ -427,8 +427,9 @@ ll_product(const LlPoint &q, const double *x, int n, int g, unsigned mask,
 
 // The values of one likelihood; false when a component lies outside what
 // ll_density is made for (t below -2^22, where its integer would wrap, or
-// a W that could overflow a class's product): then the reference's own
-// operations evaluate it.
+// a W that could overflow a class's product) or anything is NaN, the data's
+// range included (ll_product's renorm would make a finite number of a NaN
+// product): then the reference's own operations evaluate it.
 __device__ __forceinline__ bool ll_prepare(const GmmState &s, double xmin,
                                            double xmax, LlPoint &q)
 {
@@ -1352,8 +1353,12 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
             xmin = data[i];
     }
     const double kappa = 1 / ((xmax - xmin) * (xmax - xmin));
-    g->xmin = xmin;
-    g->xmax = xmax;
+    // (ll_prepare's range: a NaN point, which the comparisons pass over, must
+    // not reach the product form)
+    const bool nan =
+        std::any_of(data, data + n, [](double x) { return x != x; });
+    g->xmin = nan ? NAN : xmin;
+    g->xmax = nan ? NAN : xmax;
     g->mu0 = 0.5 * (xmin + xmax);
     g->sd0 = 1 / std::sqrt(kappa);
     g->shape0 = 2;
