@@ -49,22 +49,25 @@ void *context()
 
 // The entry of the current device and context, or -1.  Called with the
 // mutex held.  A stream that is being captured gets none (creating it would
-// end the capture).
+// end the capture, and its work runs when the call is over).
 int find_entry(cudaStream_t s)
 {
     int dev = 0;
     void *ctx = context();
     if (ctx == nullptr || cudaGetDevice(&dev) != cudaSuccess)
         return -1;
-    for (int k = 0; k < g_n; ++k)
-        if (g_entries[k].dev == dev && g_entries[k].ctx == ctx)
-            return k;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (g_n == kEntries || cudaStreamIsCapturing(s, &st) != cudaSuccess ||
-        st != cudaStreamCaptureStatusNone) {
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
         cudaGetLastError();
         return -1;
     }
+    if (st != cudaStreamCaptureStatusNone)
+        return -1;
+    for (int k = 0; k < g_n; ++k)
+        if (g_entries[k].dev == dev && g_entries[k].ctx == ctx)
+            return k;
+    if (g_n == kEntries)
+        return -1;
     Entry e;
     std::memset(&e, 0, sizeof(e));
     e.dev = dev;
@@ -97,7 +100,8 @@ int find_entry(cudaStream_t s)
 } // namespace
 
 CallScratch::CallScratch(cudaStream_t s)
-    : s_(s), entry_(-1), index_(-1), slot_(nullptr), mem_(nullptr)
+    : s_(s), entry_(-1), index_(-1), waited_(false), slot_(nullptr),
+      mem_(nullptr)
 {
     std::lock_guard<std::mutex> lock(g_mutex);
     entry_ = find_entry(s);
@@ -118,6 +122,10 @@ CallScratch::~CallScratch()
     if (mem_ != nullptr)
         cudaFreeAsync(mem_, s_);
     if (index_ >= 0) {
+        // (a call that failed after its launches; a stream that cannot be
+        // waited for keeps the slot)
+        if (!waited_ && cudaStreamSynchronize(s_) != cudaSuccess)
+            return;
         std::lock_guard<std::mutex> lock(g_mutex);
         g_entries[entry_].used &= ~(uint64_t(1) << index_);
     }

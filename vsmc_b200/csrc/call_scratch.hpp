@@ -18,7 +18,9 @@ namespace vsmc_b200 {
 constexpr size_t kSlotBytes = 256;
 constexpr size_t kPoolKeep = 32u << 20;
 
-// A call's resources; released by the destructor (the scratch on `s`).
+// A call's resources; released by the destructor (the scratch on `s`).  The
+// slot goes to another call then, so the destructor first waits for what the
+// stream may still write there, unless the call has waited itself.
 class CallScratch {
   public:
     explicit CallScratch(cudaStream_t s);
@@ -27,8 +29,11 @@ class CallScratch {
     CallScratch &operator=(const CallScratch &) = delete;
 
     // Pinned host memory of kSlotBytes that device code can write, or
-    // nullptr (none free): then results go through device memory.
+    // nullptr (none free, or `s` is being captured): then results go through
+    // device memory.
     void *slot() const { return slot_; }
+    // The stream has been waited for since the slot's last use.
+    void waited() { waited_ = true; }
     // `bytes` of device memory (once per call).
     cudaError_t alloc(size_t bytes, void **p);
 
@@ -36,6 +41,7 @@ class CallScratch {
     cudaStream_t s_;
     int entry_;
     int index_;
+    bool waited_;
     void *slot_;
     void *mem_;
 };

@@ -200,7 +200,10 @@ cudaError_t weight_call(uint64_t N, double *lw, double *w, const double *inc,
         e = cudaMemcpyAsync(&h, out, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && cs.slot() != nullptr)
+    if (e != cudaSuccess)
+        return e;
+    cs.waited();
+    if (cs.slot() != nullptr)
         std::memcpy(&h, cs.slot(), sizeof(h));
     return e;
 }
@@ -235,16 +238,20 @@ int prospective(uint64_t N, const double *lw, const double *w,
 // A resampling call's result once its stream is done: in the slot already
 // (`done`), or copied from the workspace's control block.
 static_assert(sizeof(ResampleCtl) <= kSlotBytes, "result fits a slot");
-cudaError_t resample_result(const ResampleWorkspace &ws, ResampleCtl *slot,
+cudaError_t resample_result(const ResampleWorkspace &ws, CallScratch &cs,
                             bool done, cudaStream_t s, ResampleCtl &h)
 {
+    ResampleCtl *slot = static_cast<ResampleCtl *>(cs.slot());
     cudaError_t e = cudaSuccess;
     if (!done)
         e = cudaMemcpyAsync(slot != nullptr ? slot : &h, ws.ctl, sizeof(h),
                             cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && slot != nullptr) {
+    if (e != cudaSuccess)
+        return e;
+    cs.waited();
+    if (slot != nullptr) {
         h.error = slot->error;
         h.offset = slot->offset;
     }
@@ -423,7 +430,7 @@ int vsmc_cuda_resample(int scheme, uint64_t N, const double *weight,
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample: launch");
-    e = resample_result(ws, slot, done, s, h);
+    e = resample_result(ws, cs, done, s, h);
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample");
     if (h.error != 0) {
@@ -510,7 +517,7 @@ int vsmc_cuda_resample_mn(int scheme, uint64_t M, uint64_t N,
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_mn: launch");
-    e = resample_result(ws, slot, done, s, h);
+    e = resample_result(ws, cs, done, s, h);
     if (e != cudaSuccess)
         return cuda_status(e, "vsmc_cuda_resample_mn");
     if (h.error != 0) {
