@@ -14,7 +14,7 @@ constexpr int kSlots = 64;   // calls in flight per pair
 
 struct Entry {
     int dev;
-    void *ctx;
+    unsigned long long id; // its context
     char *host;
     uint64_t used;
     cudaMemPool_t pool;
@@ -25,36 +25,25 @@ std::mutex g_mutex;
 Entry g_entries[kEntries];
 int g_n = 0;
 
-typedef int (*CtxGetCurrentFn)(void **);
-
-// The current context (cuCtxGetCurrent through the runtime's driver entry
-// point): what the entries belong to.  cudaDeviceReset ends a context and
-// its memory; the next one is another entry.
-void *context()
+template <typename F>
+F driver_function(const char *name)
 {
-    static CtxGetCurrentFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault,
-                                    &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<CtxGetCurrentFn>(p);
-    }();
-    void *ctx = nullptr;
-    if (fn == nullptr || fn(&ctx) != 0)
-        return nullptr;
-    return ctx;
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) !=
+            cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+        p = nullptr;
+    return reinterpret_cast<F>(p);
 }
 
 // The entry of the current device and context, or -1.  Called with the
 // mutex held.  A stream that is being captured gets none (creating it would
 // end the capture, and its work runs when the call is over).
-int find_entry(cudaStream_t s)
+int find_entry(cudaStream_t s, unsigned long long id)
 {
     int dev = 0;
-    void *ctx = context();
-    if (ctx == nullptr || cudaGetDevice(&dev) != cudaSuccess)
+    if (id == 0 || cudaGetDevice(&dev) != cudaSuccess)
         return -1;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
@@ -64,14 +53,14 @@ int find_entry(cudaStream_t s)
     if (st != cudaStreamCaptureStatusNone)
         return -1;
     for (int k = 0; k < g_n; ++k)
-        if (g_entries[k].dev == dev && g_entries[k].ctx == ctx)
+        if (g_entries[k].dev == dev && g_entries[k].id == id)
             return k;
     if (g_n == kEntries)
         return -1;
     Entry e;
     std::memset(&e, 0, sizeof(e));
     e.dev = dev;
-    e.ctx = ctx;
+    e.id = id;
     void *h = nullptr;
     if (cudaHostAlloc(&h, kSlots * kSlotBytes,
                       cudaHostAllocPortable | cudaHostAllocMapped) !=
@@ -99,12 +88,27 @@ int find_entry(cudaStream_t s)
 
 } // namespace
 
+unsigned long long context_id()
+{
+    typedef int (*GetCurrent)(void **);
+    typedef int (*GetId)(void *, unsigned long long *);
+    static const GetCurrent current =
+        driver_function<GetCurrent>("cuCtxGetCurrent");
+    static const GetId id_of = driver_function<GetId>("cuCtxGetId");
+    void *ctx = nullptr;
+    unsigned long long id = 0;
+    if (current == nullptr || id_of == nullptr || current(&ctx) != 0 ||
+        ctx == nullptr || id_of(ctx, &id) != 0)
+        return 0;
+    return id;
+}
+
 CallScratch::CallScratch(cudaStream_t s)
     : s_(s), entry_(-1), index_(-1), waited_(false), slot_(nullptr),
       mem_(nullptr)
 {
     std::lock_guard<std::mutex> lock(g_mutex);
-    entry_ = find_entry(s);
+    entry_ = find_entry(s, context_id());
     if (entry_ < 0)
         return;
     Entry &e = g_entries[entry_];

@@ -15,6 +15,11 @@
 
 namespace vsmc_b200 {
 
+// The current context's id, which no other context of the process ever has
+// (a handle may come back: cudaDeviceReset ends a context and its memory, and
+// the device's next one can stand at the same address); 0: none is current.
+unsigned long long context_id();
+
 constexpr size_t kSlotBytes = 256;
 constexpr size_t kPoolKeep = 32u << 20;
 

@@ -17,6 +17,7 @@
 // so nothing stale is used, but two calls that overlap on the GPU (for
 // example on two streams) race on the same memory and must be serialised by
 // the caller.
+#include "call_scratch.hpp"
 #include "resample_launch.cuh"
 
 #include <cstring>
@@ -49,30 +50,9 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mutex;
 void *g_noalloc_ptr[kMaxDevices] = {};
-void *g_noalloc_ctx[kMaxDevices] = {}; // the context the address belongs to
-
-// cuCtxGetCurrent through the runtime's driver entry point (no link against
-// libcuda): the current context identifies the module instance the cached
-// address belongs to.  After cudaDeviceReset the device's primary context is
-// a new one, the module is loaded again and the symbol may move.
-typedef int (*CtxGetCurrentFn)(void **);
-
-void *current_context()
-{
-    static CtxGetCurrentFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault,
-                                    &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<CtxGetCurrentFn>(p);
-    }();
-    void *ctx = nullptr;
-    if (fn == nullptr || fn(&ctx) != 0)
-        return nullptr;
-    return ctx;
-}
+// the context the address belongs to: after cudaDeviceReset the module is
+// loaded again and the symbol may move
+unsigned long long g_noalloc_ctx[kMaxDevices] = {};
 
 // Device address of the scratch array on the current device, looked up
 // once per device and context (with that device current) and cached.
@@ -89,9 +69,9 @@ int noalloc_scratch(void **out)
     // (no context is current before the process's first runtime call that
     // needs one; the lookup below creates it, and the next call then finds
     // the context and looks the address up once more)
-    void *ctx = current_context();
+    const unsigned long long ctx = context_id();
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-    if (g_noalloc_ptr[dev] == nullptr || ctx == nullptr ||
+    if (g_noalloc_ptr[dev] == nullptr || ctx == 0 ||
         ctx != g_noalloc_ctx[dev]) {
         void *p = nullptr;
         e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
@@ -100,7 +80,7 @@ int noalloc_scratch(void **out)
                                "vsmc_cuda_resample_noalloc: "
                                "cudaGetSymbolAddress");
         g_noalloc_ptr[dev] = p;
-        g_noalloc_ctx[dev] = ctx != nullptr ? ctx : current_context();
+        g_noalloc_ctx[dev] = ctx != 0 ? ctx : context_id();
     }
     *out = g_noalloc_ptr[dev];
     return VSMC_CUDA_OK;
