@@ -138,7 +138,28 @@ cudaError_t weight_call(uint64_t N, double *lw, double *w, const double *inc,
     WeightCtl *out = static_cast<WeightCtl *>(cs.slot());
     WeightCtl *ctl = nullptr;
     WAcc *tiles = nullptr;
-    const bool cluster = nt <= kWcTiles;
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at[1];
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    bool cluster = false;
+    if (nt <= kWcTiles) {
+        int ctas = 1;
+        while (ctas < nt && ctas < kWcCtas)
+            ctas *= 2;
+        if (ctas > 8)
+            cudaFuncSetAttribute(
+                k_weight_cluster<Kind>,
+                cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        c.gridDim = dim3((unsigned)ctas);
+        c.blockDim = dim3(kThreads);
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)ctas;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cluster = cluster_room(k_weight_cluster<Kind>, c);
+    }
     cudaError_t e;
     if (out == nullptr || !cluster) {
         void *p = nullptr;
@@ -155,25 +176,7 @@ cudaError_t weight_call(uint64_t N, double *lw, double *w, const double *inc,
             reinterpret_cast<WAcc *>(q + 2 * align256(sizeof(WeightCtl)));
     }
     what = "";
-    cudaLaunchConfig_t c = {};
-    cudaLaunchAttribute at[1];
-    c.stream = s;
-    c.attrs = at;
-    c.numAttrs = 1;
     if (cluster) {
-        int ctas = 1;
-        while (ctas < nt && ctas < kWcCtas)
-            ctas *= 2;
-        if (ctas > 8)
-            cudaFuncSetAttribute(
-                k_weight_cluster<Kind>,
-                cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        c.gridDim = dim3((unsigned)ctas);
-        c.blockDim = dim3(kThreads);
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)ctas;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
         e = cudaLaunchKernelEx(&c, k_weight_cluster<Kind>, (long long)N, lw,
                                w, inc, out);
     } else {

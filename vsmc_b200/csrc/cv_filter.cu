@@ -126,8 +126,9 @@ void join_sequence(vsmc_cuda_cv_filter *f)
         cudaStreamWaitEvent(f->stream, f->ev_seq, 0);
 }
 
+// (false: no room for the cluster, nothing launched)
 template <typename Real, bool Init, int S>
-void launch_move_split(const MoveArgs<Real> &a, cudaStream_t s)
+bool launch_move_split(const MoveArgs<Real> &a, cudaStream_t s)
 {
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((unsigned)(a.ntiles * S));
@@ -142,7 +143,10 @@ void launch_move_split(const MoveArgs<Real> &a, cudaStream_t s)
     at[1].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
     c.numAttrs = 2;
+    if (!cluster_room(k_cv_move_split<Real, Init, S>, c))
+        return false;
     cudaLaunchKernelEx(&c, k_cv_move_split<Real, Init, S>, a);
+    return true;
 }
 
 // The largest split of a tile whose CTAs are at most two per SM, else one
@@ -157,17 +161,14 @@ template <typename Real, bool Init>
 void launch_move(const MoveArgs<Real> &a, bool alone, cudaStream_t s)
 {
     const int room = alone ? 2 * device_sms() / a.ntiles : 0;
-    if (room >= 8)
-        launch_move_split<Real, Init, 8>(a, s);
-    else if (room >= 4)
-        launch_move_split<Real, Init, 4>(a, s);
-    else if (room >= 2)
-        launch_move_split<Real, Init, 2>(a, s);
-    else
-        // the block scheduler hands tiles to SMs as they free, which
-        // balances the rejection loops' uneven cost better than a
-        // persistent grid striding over tiles (measured 5% faster at 2^24)
-        launch_pdl(k_cv_move<Real, Init>, a.ntiles, kMoveThreads, s, a);
+    if ((room >= 8 && launch_move_split<Real, Init, 8>(a, s)) ||
+        (room >= 4 && launch_move_split<Real, Init, 4>(a, s)) ||
+        (room >= 2 && launch_move_split<Real, Init, 2>(a, s)))
+        return;
+    // the block scheduler hands tiles to SMs as they free, which balances the
+    // rejection loops' uneven cost better than a persistent grid striding over
+    // tiles (measured 5% faster at 2^24)
+    launch_pdl(k_cv_move<Real, Init>, a.ntiles, kMoveThreads, s, a);
 }
 
 template <typename Real>

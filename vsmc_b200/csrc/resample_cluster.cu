@@ -6,7 +6,7 @@
 
 namespace vsmc_b200 {
 
-void launch_cluster_resample(int scheme, WeightsGiven w, long long N,
+bool launch_cluster_resample(int scheme, WeightsGiven w, long long N,
                              const EngineRef &eng, const ResampleWorkspace &ws,
                              const ResampleCtl &h, ResampleCtl *out,
                              int32_t *rep_out, int32_t *copy_from,
@@ -16,17 +16,19 @@ void launch_cluster_resample(int scheme, WeightsGiven w, long long N,
     a.offset = h.offset;
     a.Nout = h.Nout;
     a.out = out;
+    bool done = false;
     const RcShape sh = rc_shape(resample_ntiles(h.Nout > N ? h.Nout : N));
     rc_scheme(scheme, [&](auto res, auto seq) {
         constexpr bool Re = decltype(res)::value;
         constexpr int U = decltype(seq)::value;
         if (sh.r == 8)
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh, 1, false,
-                      s, w, a);
+            done = rc_launch(k_resample_cluster<WeightsGiven, Re, U, 8>, sh,
+                             false, s, w, a);
         else
-            rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh, 1, false,
-                      s, w, a);
+            done = rc_launch(k_resample_cluster<WeightsGiven, Re, U, 2>, sh,
+                             false, s, w, a);
     });
+    return done;
 }
 
 } // namespace vsmc_b200

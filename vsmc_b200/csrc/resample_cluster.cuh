@@ -1374,22 +1374,21 @@ inline RcShape rc_shape(int nt)
     return s;
 }
 
-// Launches `k` with one cluster of `shape` per `clusters`; `early`: before
-// the stream's previous kernel has ended (k waits itself).
+// Launches `k` as one cluster of `shape`; `early`: before the stream's
+// previous kernel has ended (k waits itself).  False: no room for the
+// cluster, nothing launched.
 template <typename K, typename... A>
-inline cudaError_t rc_launch(K k, RcShape shape, int clusters, bool early,
-                             cudaStream_t s, const A &...args)
+inline bool rc_launch(K k, RcShape shape, bool early, cudaStream_t s,
+                      const A &...args)
 {
     const size_t smem = rc_smem_bytes(shape.groups);
-    cudaError_t e = cudaFuncSetAttribute(
-        k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && shape.ctas > 8)
-        e = cudaFuncSetAttribute(
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
+    if (shape.ctas > 8)
+        cudaFuncSetAttribute(
             k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess)
-        return e;
     cudaLaunchConfig_t c = {};
-    c.gridDim = dim3((unsigned)(shape.ctas * clusters));
+    c.gridDim = dim3((unsigned)shape.ctas);
     c.blockDim = dim3((unsigned)(kTile / shape.r * shape.groups));
     c.dynamicSmemBytes = smem;
     c.stream = s;
@@ -1402,7 +1401,10 @@ inline cudaError_t rc_launch(K k, RcShape shape, int clusters, bool early,
     at[1].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
     c.numAttrs = early ? 2 : 1;
-    return cudaLaunchKernelEx(&c, k, args...);
+    if (!cluster_room(k, c))
+        return false;
+    cudaLaunchKernelEx(&c, k, args...);
+    return true;
 }
 
 // The scheme's instance: f(residual, sequence) with compile-time constants.
@@ -1456,20 +1458,24 @@ inline RcArgs rc_args(long long N, const EngineRef &eng,
 }
 
 template <typename W>
-void launch_cluster_finish(int scheme, const FinalizeArgs &fa, const W &w,
+bool launch_cluster_finish(int scheme, const FinalizeArgs &fa, const W &w,
                            const ResampleWorkspace &ws, int32_t *copy_from,
                            cudaStream_t s)
 {
+    bool done = false;
     const RcArgs a = rc_args(fa.N, fa.eng, ws, nullptr, copy_from, true);
     const RcShape sh = rc_shape(fa.ntiles);
     rc_scheme(scheme, [&](auto res, auto u) {
         constexpr bool Re = decltype(res)::value;
         constexpr int U = decltype(u)::value;
         if (sh.r == 8)
-            rc_launch(k_finish_cluster<W, Re, U, 8>, sh, 1, true, s, fa, w, a);
+            done = rc_launch(k_finish_cluster<W, Re, U, 8>, sh, true, s, fa, w,
+                             a);
         else
-            rc_launch(k_finish_cluster<W, Re, U, 2>, sh, 1, true, s, fa, w, a);
+            done = rc_launch(k_finish_cluster<W, Re, U, 2>, sh, true, s, fa, w,
+                             a);
     });
+    return done;
 }
 
 } // namespace vsmc_b200

@@ -4,7 +4,7 @@
 
 namespace vsmc_b200 {
 
-template void launch_cluster_finish<WeightsFromLog<float>>(
+template bool launch_cluster_finish<WeightsFromLog<float>>(
     int, const FinalizeArgs &, const WeightsFromLog<float> &,
     const ResampleWorkspace &, int32_t *, cudaStream_t);
 

@@ -4,7 +4,7 @@
 
 namespace vsmc_b200 {
 
-template void launch_cluster_finish<WeightsFromLog<double>>(
+template bool launch_cluster_finish<WeightsFromLog<double>>(
     int, const FinalizeArgs &, const WeightsFromLog<double> &,
     const ResampleWorkspace &, int32_t *, cudaStream_t);
 

@@ -11,7 +11,10 @@ bool launch_resample(int scheme, WeightsGiven w, long long N,
                      int32_t *rep_out, int32_t *copy_from, cudaStream_t s,
                      bool cfrp)
 {
-    if (u_given != nullptr || !rc_fits(N, h.Nout)) {
+    if (u_given != nullptr || !rc_fits(N, h.Nout) ||
+        !launch_cluster_resample(scheme, w, N, eng, ws, h,
+                                 slot != nullptr ? slot : ws.ctl, rep_out,
+                                 copy_from, s, cfrp)) {
         const ResampleCtl *src = &h;
         if (slot != nullptr) { // (pinned: copied without staging)
             *slot = h;
@@ -25,9 +28,6 @@ bool launch_resample(int scheme, WeightsGiven w, long long N,
                                  h.Nout);
         return false;
     }
-    launch_cluster_resample(scheme, w, N, eng, ws, h,
-                            slot != nullptr ? slot : ws.ctl, rep_out,
-                            copy_from, s, cfrp);
     return slot != nullptr;
 }
 
@@ -43,10 +43,9 @@ int launch_finish_t(int scheme, const FinalizeArgs &fa, const W &w,
                     cudaEvent_t seq, cudaStream_t s)
 {
     const long long N = fa.N;
-    if (rc_fits(N, 0)) {
-        launch_cluster_finish(scheme, fa, w, ws, copy_from, s);
+    if (rc_fits(N, 0) &&
+        launch_cluster_finish(scheme, fa, w, ws, copy_from, s))
         return 1;
-    }
     const size_t smem = fa.ntiles <= kFinalSmemTiles
                             ? (size_t)fa.ntiles * sizeof(double)
                             : 0;

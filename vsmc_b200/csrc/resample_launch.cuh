@@ -23,13 +23,14 @@ inline bool rc_fits(long long N, long long Nout)
 
 // The one-cluster forms (rc_fits): a resampling of given weights whose
 // control block goes to *out; a filter step's finalisation and resampling.
-void launch_cluster_resample(int scheme, WeightsGiven w, long long N,
+// False: the device has no room for the cluster, nothing is launched.
+bool launch_cluster_resample(int scheme, WeightsGiven w, long long N,
                              const EngineRef &eng, const ResampleWorkspace &ws,
                              const ResampleCtl &h, ResampleCtl *out,
                              int32_t *rep_out, int32_t *copy_from,
                              cudaStream_t s, bool cfrp);
 template <typename W>
-void launch_cluster_finish(int scheme, const FinalizeArgs &fa, const W &w,
+bool launch_cluster_finish(int scheme, const FinalizeArgs &fa, const W &w,
                            const ResampleWorkspace &ws, int32_t *copy_from,
                            cudaStream_t s);
 

@@ -117,6 +117,21 @@ __device__ __forceinline__ void pdl_enter()
     pdl_wait();
 }
 
+// Whether the device, as far as this process and stream see it, can hold one
+// cluster of a launch: its SMs must be free in one GPC, and a partition of a
+// GPU may have fewer there than the cluster has CTAs.  Asked at every launch
+// (0.15 to 0.3 us, a launch takes 3 to 5): the answer belongs to the context
+// and the stream.  Each caller has a way without clusters.
+template <typename K>
+inline bool cluster_room(K k, const cudaLaunchConfig_t &c)
+{
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &c) == cudaSuccess)
+        return n > 0;
+    cudaGetLastError();
+    return false;
+}
+
 // --------------------------------------------------------- reductions ------
 __device__ __forceinline__ double warp_sum(double v)
 {
