@@ -359,6 +359,16 @@ __device__ __forceinline__ double residual_split(double w, double Nd,
     return modf(__dmul_rn(Nd, w), &k);
 }
 
+// More residual children than children: the integer parts are negative in
+// sum, as only negative weights make them.  Such a call is degenerate and
+// draws no sequence: the arrays (and a cluster's tiles) hold as many uniforms
+// as there are children.
+__device__ __forceinline__ bool residual_excess(long long NN,
+                                                long long children)
+{
+    return NN > children;
+}
+
 // A tile's values in shared memory are padded by one slot per 8, so that a
 // thread reading its kItems consecutive values meets no bank conflict.
 constexpr int kTilePad = kTile + kTile / 8;
@@ -626,6 +636,10 @@ k_spine_weights_body(const double *tile_sum, const long long *tile_k,
     }
     spine_scan_f64(tile_sum, tile_excl, ntiles, coeff, shd);
     if (threadIdx.x == 0) {
+        if (residual_excess(NN, resample_children(ctl, N))) {
+            ctl->error = VSMC_CUDA_EDEGENERATE;
+            NN = 0;
+        }
         ctl->NN = NN;
         ctl->coeff_r = coeff;
         ctl->coeff_r_apx = coeff;

@@ -851,7 +851,12 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
             x = warp_incl_scan(x);
             if (lane == 31) {
                 sm.total = x;
-                const long long NN = Nout - ki;
+                long long NN = Nout - ki;
+                if (residual_excess(NN, Nout)) {
+                    if (rank == 0)
+                        a.ctl->error = VSMC_CUDA_EDEGENERATE;
+                    NN = 0;
+                }
                 sm.NN = NN;
                 sm.delta = __ddiv_rn(1.0, (double)NN);
                 sm.kbits = bin_kbits(NN);
@@ -1116,7 +1121,7 @@ __device__ __forceinline__ void rc_resample(W wsrc, const RcArgs &a,
         a.ctl->offset = off;
         if (Given) {
             a.out->offset = off;
-            a.out->error = 0;
+            a.out->error = *(volatile int *)&a.ctl->error;
         }
     }
     if (!a.cfrp)
