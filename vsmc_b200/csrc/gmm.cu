@@ -1198,30 +1198,59 @@ double alpha_at(uint64_t t, uint64_t iters, int power)
     return a;
 }
 
+// CTAs of k_gmm_mcmc that fit on an SM (registers: two; FP64 data of about
+// 10000 points and more, beside the table: one).
+template <bool F32>
+int resident_ctas(int G, int n)
+{
+    int c = 0;
+#define VSMC_CALL(K)                                                          \
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(                            \
+        &c, k_gmm_mcmc<K, F32>, kGmmThreads, gmm_smem_bytes(n, F32))
+    VSMC_GMM_SWITCH(G, VSMC_CALL)
+#undef VSMC_CALL
+    return c < 1 ? 1 : c;
+}
+
 // The lanes per particle G (a choice of speed alone: no result depends on
-// it).  A thread's time is that of n / G points plus `over` points' worth of
-// proposal and acceptance work, which every lane repeats; a CTA alone on its
-// SM runs at latency, two take `two` times as long, and more follow at
-// `rate` per CTA and SM.  The constants are fitted to measured sweeps (both
-// forms, n = 250 and 1000, N = 1000 to 300000, one B200): the pick is 1% (FP64)
-// and 2% (mixed) slower than the fastest G on average, 16% at most.  Timing
-// every G at each initialize, as before, cost 15 sweeps (12% of a run of 20
-// steps) and two waits of the host.
+// it).  A thread's time is that of n / G points, each `point` times as long as
+// with one lane (fewer classes of points side by side), plus `over` points'
+// worth of proposal and acceptance work, which every lane repeats.  A CTA
+// alone on its SM runs at latency; two together take `two` times as long, the
+// less the more lanes share a particle.  The CTAs go in waves of as many as
+// fit at once: whole waves where that is one to an SM, else the last one
+// costs `tail` of what it lacks.
+// The constants are fitted to measured sweeps (both forms, 86 sizes, n = 100 to
+// 16384, N = 300 to 200000, one B200): the pick is 0.5% (FP64) and 0.2%
+// (mixed) slower than the fastest G on average and 9% at most; at 30 other
+// sizes a form 1.8% and 0.6%, 10% at most.  Timing every G at each initialize,
+// as before, cost 15 sweeps (12% of a run of 20 steps) and two waits of the
+// host.
+struct GroupCost {
+    double point[5], two[5]; // G = 1, 2, 4, 8, 16
+    double over, tail;
+};
+constexpr GroupCost kGroupCost[2] = {
+    {{1.0, 1.15, 1.2, 1.35, 1.55}, {1.6, 1.55, 1.45, 1.35, 1.25}, 50.0, 0.45},
+    {{1.0, 1.25, 1.25, 1.15, 1.45}, {1.8, 1.7, 1.55, 1.4, 1.3}, 115.0, 0.4}};
+
 int pick_group(const vsmc_cuda_gmm *g)
 {
     const bool f32 = gmm_f32(g);
-    const double over = f32 ? 160.0 : 30.0;
-    const double two = f32 ? 1.5 : 1.3, rate = f32 ? 0.9 : 0.8;
+    const GroupCost &m = kGroupCost[f32 ? 1 : 0];
     const int sms = device_sms();
     int best = 1;
     double least = 0.0;
-    for (int G = 1; G <= kLlClasses; G *= 2) {
+    for (int G = 1, k = 0; G <= kLlClasses; G *= 2, ++k) {
         const int c = gmm_ntiles_mcmc((long long)g->cfg.N, G);
-        const double per = (double)c / sms;
-        const double load =
-            c <= sms ? 1.0
-                     : (c <= 2 * sms ? two : rate * std::max(per, 2.0));
-        const double cost = ((double)g->n / G + over) * load;
+        const int r = f32 ? resident_ctas<true>(G, g->n)
+                          : resident_ctas<false>(G, g->n);
+        const double waves = (double)c / ((double)sms * r);
+        double load = std::ceil(waves);
+        if (r > 1 && c > sms)
+            load = m.two[k] *
+                   (waves <= 1.0 ? 1.0 : waves + m.tail * (load - waves));
+        const double cost = (m.point[k] * g->n / G + m.over) * load;
         if (G == 1 || cost < least) {
             least = cost;
             best = G;
@@ -1343,7 +1372,6 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
     g->timing = false;
     g->ev_used = 0;
     g->launches = 0;
-    g->group = cfg->group == 0 ? pick_group(g) : cfg->group;
     // gmm_state::read_data (gmm_state.hpp:118-157)
     double xmax = data[0], xmin = data[0];
     for (uint64_t i = 0; i != n; ++i) {
@@ -1385,6 +1413,7 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
     }
     set_smem_attrs<true>(gmm_smem_bytes((int)n, true));
     set_smem_attrs<false>(gmm_smem_bytes((int)n, false));
+    g->group = cfg->group == 0 ? pick_group(g) : cfg->group;
     *out = g;
     return VSMC_CUDA_OK;
 }
