@@ -1155,10 +1155,12 @@ void launch_loglik_t(vsmc_cuda_gmm *g, const GmmArgs &a, int G, double *out)
 #undef VSMC_CALL
 }
 
+// The kernels' limit of dynamic shared memory: that of the most data, since it
+// holds for every sampler of the process.
 template <bool F32>
-void set_smem_attrs(size_t smem)
+void set_smem_attrs()
 {
-    const int b = (int)smem;
+    const int b = (int)gmm_smem_bytes(kGmmMaxData, F32);
 #define VSMC_GMM_ATTR(G)                                                      \
     cudaFuncSetAttribute(k_gmm_init<G, F32>,                                  \
                          cudaFuncAttributeMaxDynamicSharedMemorySize, b);     \
@@ -1411,8 +1413,8 @@ int vsmc_cuda_gmm_create(const vsmc_cuda_gmm_config *cfg, const double *data,
         delete g;
         return cuda_status(e, "vsmc_cuda_gmm_create");
     }
-    set_smem_attrs<true>(gmm_smem_bytes((int)n, true));
-    set_smem_attrs<false>(gmm_smem_bytes((int)n, false));
+    set_smem_attrs<true>();
+    set_smem_attrs<false>();
     g->group = cfg->group == 0 ? pick_group(g) : cfg->group;
     *out = g;
     return VSMC_CUDA_OK;
