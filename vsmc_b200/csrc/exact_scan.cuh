@@ -47,7 +47,8 @@ namespace vsmc_b200 {
 
 constexpr int kExactCap = 64;         // specials kept per tile
 constexpr int kNoBinade = -100000;    // binade of a special element
-constexpr int kExactStage = 1280;     // additions the spine stages
+constexpr int kExactStage = 1540;     // additions the spine stages: 1024
+                                      // specials in 256 tiles (and padding)
 
 struct ExactTile {
     unsigned long long k_total; // sum of the clean elements' k

@@ -1597,11 +1597,32 @@ struct SmemExactSpine {
     double sout[kExactDirtyStage];
     // the walk's additions, when they fit: tile q's from st_off[q], first
     // the clean tiles before it, then its specials (each after the clean
-    // run before it), then its clean tail; S after each
+    // run before it), then its clean tail; the walk leaves the exact S after
+    // each in its place (seg)
     ExactStep st[kExactStage];
-    double S[kExactStage];
     int st_off[kExactDirtyStage];
 };
+
+// A tile with more specials than kept: the reference's loop itself, from S.
+// Returns S after the tile.
+template <typename W, bool Residual, bool Raw>
+__device__ __forceinline__ double exact_sum_tile(const W &wsrc, long long N,
+                                                 const ResampleCtl *ctl,
+                                                 int tile, double S,
+                                                 const ExactScan &ex)
+{
+    const double Nd = (double)resample_children(ctl, N);
+    const double coeff_r = Residual && !Raw ? ctl->coeff_r : 1.0;
+    const long long b0 = (long long)tile * kTile;
+    const long long b1 = min(b0 + (long long)kTile, N);
+    for (long long i = b0; i < b1; ++i) {
+        S = __dadd_rn(S, scan_weight<W, Residual, Raw>(wsrc, i, Nd, coeff_r,
+                                                       nullptr));
+        if (!Raw)
+            ex.rec[i] = S;
+    }
+    return S;
+}
 
 // Phase B (one CTA): the exact S before every tile and at every special.
 // Each warp owns a contiguous range of tiles and reads it 32 tiles at a
@@ -1714,39 +1735,47 @@ k_exact_spine_body(W wsrc, long long N, ResampleCtl *ctl, int nt,
     }
     __syncthreads();
     const bool staged_all = ndt <= kExactDirtyStage;
-    // 2. stage the walk's additions when they all fit (a tile with more
-    // specials than kept is summed element by element)
-    int nsq = 0;
+    // 2. stage the walk's additions when they all fit.  A tile with more
+    // specials than kept is summed element by element, between its first
+    // addition and its last (2^20 weights with one such tile and 229 of three
+    // specials: 237 us a resampling, 430 when it sent every tile's walk to
+    // global memory)
+    const auto kept = [](const ExactTile &et) {
+        return et.nspec <= kExactCap ? et.nspec : 0;
+    };
+    int nsq = 0, over = 0;
     if ((int)threadIdx.x < min(ndt, kExactDirtyStage)) {
         const ExactTile et = sm.tq[threadIdx.x];
-        nsq = et.nspec <= kExactCap ? et.nspec + 2 : kExactStage;
+        nsq = kept(et) + 2;
+        over = et.nspec > kExactCap;
     }
     int nst;
     const int soff = block_excl_scan(nsq, sm.shi, nst); // ends with a barrier
     const bool fits = staged_all && nst <= kExactStage - 4;
     if (fits && (int)threadIdx.x < ndt)
         sm.st_off[threadIdx.x] = soff;
-    __syncthreads();
+    over = __syncthreads_or(over);
     if (fits) { // a warp per tile with specials
         for (int q = wq; q < ndt; q += nw) {
             const ExactTile et = sm.tq[q];
+            const int ns = kept(et);
             const ExactSpecial *sp = ex.spec + (size_t)sm.dq[q] * kExactCap;
             ExactStep *st = sm.st + sm.st_off[q];
-            for (int r = lane; r < et.nspec + 2; r += 32) {
+            for (int r = lane; r < ns + 2; r += 32) {
                 ExactStep x;
-                x.w = 0.0;
+                x.seg = x.w = 0.0;
                 if (r == 0) {
-                    x.seg = q == 0 ? 0.0
-                                   : exact_clean(sm.pkq[q] - sm.pkq[q - 1],
-                                                 sm.eaft[q - 1]);
+                    if (q > 0)
+                        x.seg = exact_clean(sm.pkq[q] - sm.pkq[q - 1],
+                                            sm.eaft[q - 1]);
                 } else {
                     const unsigned long long kb =
                         r > 1 ? sp[r - 2].k_before : 0ull;
-                    if (r <= et.nspec) {
+                    if (r <= ns) {
                         x.seg = exact_clean(sp[r - 1].k_before - kb,
                                             sp[r - 1].e_seg);
                         x.w = sp[r - 1].w;
-                    } else {
+                    } else if (et.nspec == ns) {
                         x.seg = exact_clean(et.k_total - kb, et.e_last);
                     }
                 }
@@ -1759,33 +1788,44 @@ k_exact_spine_body(W wsrc, long long N, ResampleCtl *ctl, int nt,
     if (fits) {
         if (threadIdx.x == 0) {
             double S = 0.0;
-            for (int i = 0; i < nst; i += 4) { // (the array is padded by 4)
-                ExactStep q[4];
+            const auto chain = [&](int i, int e) {
+                for (; i < e; i += 4) { // (the array is padded by 4)
+                    ExactStep q[4];
 #pragma unroll
-                for (int m = 0; m < 4; ++m)
-                    q[m] = sm.st[i + m];
+                    for (int m = 0; m < 4; ++m)
+                        q[m] = sm.st[i + m];
 #pragma unroll
-                for (int m = 0; m < 4; ++m)
-                    if (i + m < nst) {
-                        S = __dadd_rn(__dadd_rn(S, q[m].seg), q[m].w);
-                        sm.S[i + m] = S;
+                    for (int m = 0; m < 4; ++m)
+                        if (i + m < e) {
+                            S = __dadd_rn(__dadd_rn(S, q[m].seg), q[m].w);
+                            sm.st[i + m].seg = S;
+                        }
+                }
+            };
+            int i = 0;
+            if (over)
+                for (int q = 0; q < ndt; ++q)
+                    if (sm.tq[q].nspec > kExactCap) {
+                        chain(i, sm.st_off[q] + 1);
+                        S = exact_sum_tile<W, Residual, Raw>(wsrc, N, ctl,
+                                                             sm.dq[q], S, ex);
+                        sm.st[sm.st_off[q] + 1].seg = S;
+                        i = sm.st_off[q] + 2;
                     }
-            }
+            chain(i, nst);
         }
         __syncthreads();
         for (int q = wq; q < ndt; q += nw) {
-            const int d = sm.dq[q], ns = sm.tq[q].nspec;
-            const double *Sq = sm.S + sm.st_off[q];
+            const int d = sm.dq[q], ns = kept(sm.tq[q]);
+            const ExactStep *Sq = sm.st + sm.st_off[q];
             for (int r = lane; r < ns; r += 32)
-                ex.s_spec[(size_t)d * kExactCap + r] = Sq[r + 1];
+                ex.s_spec[(size_t)d * kExactCap + r] = Sq[r + 1].seg;
             if (lane == 0) {
-                ex.start[d] = Sq[0];
-                sm.sout[q] = Sq[ns + 1];
+                ex.start[d] = Sq[0].seg;
+                sm.sout[q] = Sq[ns + 1].seg;
             }
         }
     } else if (threadIdx.x == 0) {
-        const double Nd = (double)resample_children(ctl, N);
-        const double coeff_r = Residual && !Raw ? ctl->coeff_r : 1.0;
         double S = 0.0;
         unsigned long long pk_prev = 0;
         int ea_prev = kNoBinade;
@@ -1816,15 +1856,7 @@ k_exact_spine_body(W wsrc, long long N, ResampleCtl *ctl, int nt,
                     S = __dadd_rn(S, __dmul_rn((double)tail,
                                                exact_pow2(et.e_last - 52)));
             } else {
-                // more specials than kept: the reference's loop itself
-                const long long b0 = (long long)d * kTile;
-                const long long b1 = min(b0 + (long long)kTile, N);
-                for (long long i = b0; i < b1; ++i) {
-                    S = __dadd_rn(S, scan_weight<W, Residual, Raw>(
-                                         wsrc, i, Nd, coeff_r, nullptr));
-                    if (!Raw)
-                        ex.rec[i] = S;
-                }
+                S = exact_sum_tile<W, Residual, Raw>(wsrc, N, ctl, d, S, ex);
             }
             if (sq)
                 sm.sout[q] = S;
