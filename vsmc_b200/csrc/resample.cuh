@@ -1209,6 +1209,7 @@ __device__ __forceinline__ double block_prefix(double v, double *sh,
     const double inc = warp_incl_scan(v);
     if (lane == 31)
         sh[wid] = inc;
+    const double mine = warp_excl_of(inc);
     __syncthreads();
     double before = 0.0, all = 0.0;
 #pragma unroll
@@ -1218,7 +1219,7 @@ __device__ __forceinline__ double block_prefix(double v, double *sh,
         all += x;
     }
     total = all;
-    return before + warp_excl_of(inc);
+    return before + mine;
 }
 
 // Where a tile's scan puts its specials and last binade in global memory.
@@ -1907,8 +1908,10 @@ k_exact_spine_body(W wsrc, long long N, ResampleCtl *ctl, int nt,
     }
 }
 
+// (one CTA: without the 1 the compiler keeps to 32 registers, for two on an SM,
+// and spills)
 template <typename W, bool Residual, bool Raw = false>
-__global__ void __launch_bounds__(kSpineThreads)
+__global__ void __launch_bounds__(kSpineThreads, 1)
 k_exact_spine(W wsrc, long long N, ResampleCtl *ctl, int nt, ExactScan ex)
 {
     pdl_enter();

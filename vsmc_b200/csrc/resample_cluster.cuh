@@ -139,12 +139,13 @@ __device__ __forceinline__ T rc_excl_scan(T v, T *sh, const RcThread<R> &th,
     const T inc = warp_incl_scan(v);
     if (th.lane == 31)
         sh[th.wid] = inc;
+    const T mine = warp_excl_of(inc);
     th.sync();
     const T xi = warp_incl_scan(th.lane < NW ? sh[th.lane] : T(0));
     total = __shfl_sync(0xffffffffu, xi, 31);
-    const T before = __shfl_sync(0xffffffffu, warp_excl_of(xi), th.wid);
+    const T upto = __shfl_sync(0xffffffffu, xi, th.wid > 0 ? th.wid - 1 : 0);
     th.sync();
-    return before + warp_excl_of(inc);
+    return (th.wid > 0 ? upto : T(0)) + mine;
 }
 
 // The plain scan's prefixes of a tile in the launch sequence's association:

@@ -214,6 +214,7 @@ __device__ __forceinline__ double block_excl_sum(double v, double *sh,
     const double inc = warp_incl_scan(v);
     if (lane == 31)
         sh[wid] = inc;
+    const double mine = warp_excl_of(inc);
     __syncthreads();
     if (wid == 0) {
         double s = lane < nw ? sh[lane] : 0.0;
@@ -225,7 +226,7 @@ __device__ __forceinline__ double block_excl_sum(double v, double *sh,
     const double wexcl = wid > 0 ? sh[wid - 1] : 0.0;
     total = sh[nw - 1];
     __syncthreads();
-    return wexcl + warp_excl_of(inc);
+    return wexcl + mine;
 }
 
 } // namespace vsmc_b200
