@@ -21,7 +21,7 @@
 //   source); each thread uses one bound for its kItems elements,
 //   d = (8 i_last + 256) ulp(2 m) + margin * m, m >= every G and w there.
 //   The bound is relative to the thread's own prefixes, so no part of G may be
-//   formed by subtracting a later weight from a sum that holds it
+//   formed by subtracting a later thread's weight from a sum that holds it
 //   (block_excl_sum, block_prefix): beside a weight 2^53 times all before it
 //   the difference is 0 or off by a binade.
 // * A zero weight while the prefix is still 0 leaves S at 0: clean, k = 0.
@@ -108,7 +108,8 @@ __device__ __forceinline__ int exact_window(double g, double d)
 
 // The classification of a thread's R consecutive elements of a tile
 // (global index i0 + j): approximate tile start `a`, the thread's exclusive
-// prefix `pre` of the tile's weights, the weights `w`.  Elements at or past
+// prefix `pre` of the tile's weights, the weights `w`; first: pre is 0 only
+// when every weight of the tile before the thread's is.  Elements at or past
 // N count as clean with k = 0 and the previous element's binade.
 template <int R>
 struct ExactLocal {
@@ -121,7 +122,8 @@ struct ExactLocal {
 template <int R>
 __device__ __forceinline__ void
 exact_classify(long long i0, long long N, const double (&w)[R], double a,
-               double pre, double run, double rel, ExactLocal<R> &x)
+               double pre, double run, double rel, bool first,
+               ExactLocal<R> &x)
 {
     // one error bound for the thread's elements (run: their sum).  A
     // negative weight (the sign bits) or one that is not finite (m) leaves
@@ -192,10 +194,9 @@ exact_classify(long long i0, long long N, const double (&w)[R], double a,
                 int e = kNoBinade;
                 if (i == 0) {
                     // S_{-1} = 0: the first addition is the hardware's
-                } else if (gp == 0.0 && w[j] == 0.0) {
+                } else if (first && gp == 0.0 && w[j] == 0.0) {
                     // a leading zero: every weight before it is 0 (sums of
-                    // non-negative weights, formed without subtractions,
-                    // vanish only so)
+                    // non-negative weights vanish only so)
                     sp = false;
                 } else if (ec != kNoBinade && ec == ep) {
                     // k = w / 2^(e-52) rounded to nearest: adding 2^52 rounds
@@ -258,12 +259,12 @@ template <int R, int NW, typename Sync, typename Out>
 __device__ __forceinline__ void
 exact_scan_tile(long long base, long long i0, long long N,
                 const double (&w)[R], double a, double pre, double run,
-                double rel, int lane, int wid, SmemExactScan<NW> &sm,
-                Sync sync, Out out, ExactRec<R> &r)
+                double rel, bool first, int lane, int wid,
+                SmemExactScan<NW> &sm, Sync sync, Out out, ExactRec<R> &r)
 {
     constexpr unsigned kAll = 0xffffffffu;
     ExactLocal<R> x;
-    exact_classify(i0, N, w, a, pre, run, rel, x);
+    exact_classify(i0, N, w, a, pre, run, rel, first, x);
     const unsigned long long kr = x.kloc[R - 1];
     const unsigned long long ki = warp_incl_scan(kr);
     const unsigned long long ke = ki - kr;

@@ -1199,17 +1199,20 @@ struct SmemExactCore {
     SmemExactScan<kThreads / 32> et;
 };
 
-// Block-wide exclusive prefix of one double per thread of 256 and the
-// block's total, where the association does not matter (two barriers).
+// Block-wide exclusive prefix of one non-negative double per thread of 256 and
+// the block's total, for the exact scan's classification (two barriers).  The
+// one subtraction, of the thread's own value from its warp's prefix, is off by
+// roundings of sums that its bound m holds; first: whether the warp's earlier
+// threads are all 0 (and the prefix exactly that of the earlier warps).
 __device__ __forceinline__ double block_prefix(double v, double *sh,
-                                               double &total)
+                                               double &total, bool &first)
 {
     constexpr int NW = kThreads / 32;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double inc = warp_incl_scan(v);
     if (lane == 31)
         sh[wid] = inc;
-    const double mine = warp_excl_of(inc);
+    first = (__ballot_sync(0xffffffffu, v != 0.0) & ((1u << lane) - 1u)) == 0;
     __syncthreads();
     double before = 0.0, all = 0.0;
 #pragma unroll
@@ -1219,7 +1222,7 @@ __device__ __forceinline__ double block_prefix(double v, double *sh,
         all += x;
     }
     total = all;
-    return before + mine;
+    return before + (inc - v);
 }
 
 // Where a tile's scan puts its specials and last binade in global memory.
@@ -1357,7 +1360,8 @@ exact_tile_compute(const W &wsrc, long long N, const ResampleCtl *ctl,
             approx_tile_record<Residual>(w, kk, pre, total, N, i0, tile, ex);
         return;
     }
-    const double pre = block_prefix(run, sm.shd, total);
+    bool first;
+    const double pre = block_prefix(run, sm.shd, total, first);
     double a_apx;
     if (Residual)
         a_apx = Raw ? __ddiv_rn(tile_excl[tile], ctl->coeff_r_apx)
@@ -1368,6 +1372,7 @@ exact_tile_compute(const W &wsrc, long long N, const ResampleCtl *ctl,
                     : __dmul_rn(tile_excl[tile], wsrc.spine_ratio());
     ExactRec<kItems> x;
     exact_scan_tile(base, i0, N, w, a_apx, pre, run, ExactMargin<W>::rel,
+                    first,
                     (int)(threadIdx.x & 31), (int)(threadIdx.x >> 5), sm.et,
                     [] { __syncthreads(); }, ExactOut{ex, tile}, x);
     if (threadIdx.x == 0) {

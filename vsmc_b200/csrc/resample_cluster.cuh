@@ -237,7 +237,7 @@ rc_classify(long long base, long long N, const double (&w)[R], double a,
 #pragma unroll
     for (int j = 0; j < R; ++j)
         run += w[j];
-    exact_scan_tile(base, i0, N, w, a, pre, run, rel, th.lane, th.wid,
+    exact_scan_tile(base, i0, N, w, a, pre, run, rel, true, th.lane, th.wid,
                     reinterpret_cast<SmemExactScan<RcThread<R>::NW> &>(g.scn),
                     [&] { th.sync(); }, RcOut{out}, r);
     if (th.tid == 0) {
