@@ -1220,9 +1220,10 @@ void launch_step_any(vsmc_cuda_cv_batch *b, int n, long long tiles,
 }
 
 // A run of the same lists is launched directly this many times, then recorded
-// as a graph: recording costs about seven times what a relaunch saves (256
-// filters of 2^10 to 2^16 over 50 to 200 steps: 65.2 ms launched directly, 91 to
-// 97 the run that records, in a few processes 140 to 470, 60.6 relaunched).
+// as a graph: recording costs three to seven times what a relaunch saves (256
+// filters of 2^10 to 2^16 over 50 to 200 steps: 65.3 ms launched directly, 75 to
+// 80 the run that records on an idle host and 91 and more, once 470, on a busy
+// one, 60.6 to 61 relaunched).
 constexpr int kRunsBeforeGraph = 2;
 
 void drop_run_graph(vsmc_cuda_cv_batch *b)
